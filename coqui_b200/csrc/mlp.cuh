@@ -22,7 +22,8 @@ struct Mlp {
   int64_t adam_t = 0;
   // activations of the last forward pass (batch capacity cap)
   int64_t cap = 0;
-  DevBuf<float> x, h1, h2, y, t, dy, dh2, dh1, part;
+  DevBuf<float> x, h1, h2, y, t, dy, dh2, dh1;
+  DevBuf<float> part, lpart;    // partial sums of the split reductions and of the loss
   DevBuf<int64_t> idx;
   DevBuf<float> xall, tall;     // training set (device)
   int64_t nall = 0;

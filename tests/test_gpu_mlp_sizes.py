@@ -1,0 +1,34 @@
+"""Loss, gradient and forward pass of the network's kernels at batch sizes around their tile and
+slice edges and at layer sizes outside the fused output / input kernels, against the FP64 oracle.
+
+Tolerance: every product is an FP32 sum of at most max(width, batch) terms; with sums of length n
+cut into blocks the error is below sqrt(n) rounding units of 6e-8 relative to the sum of
+magnitudes, 2e-5 of the largest gradient element for the sizes here."""
+import numpy as np
+import pytest
+
+from coqui_b200 import capi
+from oracle import mlp_oracle as M
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(4, 256, 2, 1), (4, 256, 2, 15), (4, 256, 2, 257), (4, 256, 2, 5001), (4, 256, 2, 20000),
+         (3, 100, 1, 700), (8, 33, 4, 513), (9, 256, 2, 300), (4, 300, 2, 300), (5, 64, 5, 1030)]
+
+
+@pytest.mark.parametrize("din,width,dout,batch", SIZES)
+def test_loss_gradient_and_forward(din, width, dout, batch):
+    net = capi.Mlp(din, width, dout, seed=11)
+    rng = np.random.default_rng(batch)
+    p = (net.params() + 0.05 * rng.standard_normal(net.nparam)).astype(np.float32)
+    net.set_params(p)  # nonzero biases
+    X = rng.standard_normal((batch, din)).astype(np.float32)
+    T = rng.standard_normal((batch, dout)).astype(np.float32)
+    loss_ref, g_ref = M.loss_and_grad(p, X, T, din, width, dout)
+    Y_ref, _ = M.forward(p, X, din, width, dout)
+    for _ in range(2):  # the second call runs on kept workspaces
+        loss, g = net.gradient(X, T)
+        assert abs(loss - loss_ref) < 1e-5 * loss_ref
+        assert np.abs(g - g_ref).max() < 2e-5 * np.abs(g_ref).max()
+        assert np.abs(net.forward(X) - Y_ref).max() < 1e-5 * max(1.0, np.abs(Y_ref).max())
+    net.close()
