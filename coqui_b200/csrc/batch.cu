@@ -168,9 +168,14 @@ void batch_gw(Batch* b) {
   cq::tc_cgemm_grouped(g2, b->gtab, s);
   // ---- Pi(t) over all columns (nk = 1: no k <-> R transform) ----
   const cq::KGrid g0{1, 1, 1};
-  for (int64_t it = 0; it < nth; ++it)
-    cq::launch_pi_fused<float>(b->cache.p + it * cols, b->cache.p + (nt - 1 - it) * cols,
-                               b->PW.p + it * cols, cols, g0, -2.0, s);
+  cq::TauSlices ts;
+  ts.n = nth;
+  ts.n_minus = nt / 2;
+  ts.sp = cols;
+  ts.sn = -cols;
+  ts.sw = cols;
+  cq::launch_pi_fused<float>(b->cache.p, b->cache.p + (nt - 1) * cols, b->PW.p, cols, g0, -2.0, s,
+                             ts);
   cq::launch_ir_transform_real<float>(b->PW.p, cols, (int)nth, (int)nwh, b->dTwtR.p, s);
   // ---- Dyson per (m, iW): M = L^H Pi L, I - M = C C^H, W = L (D + D^H + D^H D) L^H ----
   std::vector<cq::TcGroup> p1, p2;
@@ -330,12 +335,8 @@ void batch_gw(Batch* b) {
     cq::launch_mirror_upper(b->PW.p + b->offPQ[m], b->Np[m], nwh, s, cols);
   cq::launch_ir_transform_real<float>(b->PW.p, cols, (int)nwh, (int)nth, b->dTtwR.p, s);
   // ---- Sigma_PQ(t) = -G_PQ(t) o W(t) in place in the cache (both halves), then X^H S X ----
-  for (int64_t it = 0; it < nth; ++it) {
-    const bool minus = it < nt / 2;
-    float2* gp = b->cache.p + it * cols;
-    float2* gn = minus ? b->cache.p + (nt - 1 - it) * cols : nullptr;
-    cq::launch_sigma_fused<float>(gp, gn, b->PW.p + it * cols, gp, gn, cols, g0, s);
-  }
+  float2* gn = b->cache.p + (nt - 1) * cols;
+  cq::launch_sigma_fused<float>(b->cache.p, gn, b->PW.p, b->cache.p, gn, cols, g0, s, ts);
   std::vector<cq::TcGroup> a1, a2;
   for (int64_t m = 0; m < b->nmol; ++m) {
     const int64_t nb = b->nb[m], Np = b->Np[m];

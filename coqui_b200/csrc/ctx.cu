@@ -339,32 +339,89 @@ void require_ready(Ctx* c, bool thc, bool ir, bool k) {
 
 // ntau consecutive G slices (ntau, nk, nb, nb) complex128 on the device -> out (ntau, nk,
 // Np, Np) in storage precision.  The tensor-core form batches all ntau * nk problems.
+// FP64: the tau slices go in batches of at least 256 (tau, k) problems (one 384 x 48 x 48
+// product of 27 k-points has 162 CTAs, one per SM), X addressed periodically in k.
+int64_t fp64_tau_batch(Ctx* c, int64_t ntau) {
+  return std::min<int64_t>(ntau, (256 + c->nk - 1) / c->nk);
+}
 void p2a_fp64(Ctx* c, const double2* Gk, double2* out, int64_t ntau) {
-  const int64_t nk = c->nk, nb = c->nb, Np = c->Np;
-  c->Tproj.ensure((size_t)nk * Np * nb);
-  for (int64_t t = 0; t < ntau; ++t) {
-    const double2* G = Gk + t * nk * nb * nb;
-    double2* O = out + t * nk * Np * Np;
+  const int64_t nk = c->nk, nb = c->nb, Np = c->Np, step = fp64_tau_batch(c, ntau);
+  c->Tproj.ensure((size_t)step * nk * Np * nb);
+  for (int64_t t = 0; t < ntau; t += step) {
+    const int64_t n = std::min(step, ntau - t) * nk;
     // T = X G  (Np x nb)
-    zgemm_rm(c, 'N', 'N', Np, nb, nb, make_double2(1, 0), c->X.p, nb, Np * nb, G, nb, nb * nb,
-             make_double2(0, 0), c->Tproj.p, nb, Np * nb, nk);
+    cq::ZgemmArgs a;
+    a.M = Np;
+    a.N = a.K = nb;
+    a.A = c->X.p;
+    a.lda = nb;
+    a.sA = Np * nb;
+    a.a_mod = nk;
+    a.B = Gk + t * nk * nb * nb;
+    a.ldb = nb;
+    a.sB = nb * nb;
+    a.C = c->Tproj.p;
+    a.ldc = nb;
+    a.sC = Np * nb;
+    a.batch = n;
+    cq::zgemm(a, c->st);
     // O = T X^H  (Np x Np)
-    zgemm_rm(c, 'N', 'C', Np, Np, nb, make_double2(1, 0), c->Tproj.p, nb, Np * nb, c->X.p, nb,
-             Np * nb, make_double2(0, 0), O, Np, Np * Np, nk);
+    cq::ZgemmArgs o;
+    o.opB = 'C';
+    o.M = o.N = Np;
+    o.K = nb;
+    o.A = c->Tproj.p;
+    o.lda = nb;
+    o.sA = Np * nb;
+    o.B = c->X.p;
+    o.ldb = nb;
+    o.sB = Np * nb;
+    o.b_mod = nk;
+    o.C = out + t * nk * Np * Np;
+    o.ldc = Np;
+    o.sC = Np * Np;
+    o.batch = n;
+    cq::zgemm(o, c->st);
   }
 }
 void a2p_fp64(Ctx* c, const double2* Sk, double2* out, int64_t ntau) {
-  const int64_t nk = c->nk, nb = c->nb, Np = c->Np;
-  c->Tproj.ensure((size_t)nk * Np * nb);
-  for (int64_t t = 0; t < ntau; ++t) {
-    const double2* S = Sk + t * nk * Np * Np;
-    double2* O = out + t * nk * nb * nb;
+  const int64_t nk = c->nk, nb = c->nb, Np = c->Np, step = fp64_tau_batch(c, ntau);
+  c->Tproj.ensure((size_t)step * nk * Np * nb);
+  for (int64_t t = 0; t < ntau; t += step) {
+    const int64_t n = std::min(step, ntau - t) * nk;
     // T = X^H S  (nb x Np)
-    zgemm_rm(c, 'C', 'N', nb, Np, Np, make_double2(1, 0), c->X.p, nb, Np * nb, S, Np, Np * Np,
-             make_double2(0, 0), c->Tproj.p, Np, Np * nb, nk);
+    cq::ZgemmArgs a;
+    a.opA = 'C';
+    a.M = nb;
+    a.N = a.K = Np;
+    a.A = c->X.p;
+    a.lda = nb;
+    a.sA = Np * nb;
+    a.a_mod = nk;
+    a.B = Sk + t * nk * Np * Np;
+    a.ldb = Np;
+    a.sB = Np * Np;
+    a.C = c->Tproj.p;
+    a.ldc = Np;
+    a.sC = Np * nb;
+    a.batch = n;
+    cq::zgemm(a, c->st);
     // O = T X  (nb x nb)
-    zgemm_rm(c, 'N', 'N', nb, nb, Np, make_double2(1, 0), c->Tproj.p, Np, Np * nb, c->X.p, nb,
-             Np * nb, make_double2(0, 0), O, nb, nb * nb, nk);
+    cq::ZgemmArgs o;
+    o.M = o.N = nb;
+    o.K = Np;
+    o.A = c->Tproj.p;
+    o.lda = Np;
+    o.sA = Np * nb;
+    o.B = c->X.p;
+    o.ldb = nb;
+    o.sB = Np * nb;
+    o.b_mod = nk;
+    o.C = out + t * nk * nb * nb;
+    o.ldc = nb;
+    o.sC = nb * nb;
+    o.batch = n;
+    cq::zgemm(o, c->st);
   }
 }
 
@@ -495,7 +552,15 @@ void eval_pi_device(Ctx* c) {
       project_p2a(c, c->G.p + a * gsz, gslab(c, a), b - a);
       project_p2a(c, c->G.p + (nt - b) * gsz, gslab(c, nt - b), b - a);
     }
-    for (int64_t it = a; it < b; ++it) {
+    // a cached chunk in one launch, else one tau at a time through the slabs Gp, Gn
+    cq::TauSlices ts;
+    if (cached) {
+      ts.n = b - a;
+      ts.sp = nk * ncol;
+      ts.sn = -ts.sp;
+      ts.sw = c->nq * ncol;
+    }
+    for (int64_t it = a; it < b; it += ts.n) {
       const unsigned char* gp = c->Gp.p;
       const unsigned char* gn = c->Gn.p;
       if (cached) {
@@ -509,10 +574,10 @@ void eval_pi_device(Ctx* c) {
       cq::Prof::Scope sc(&c->prof, "pi_fused");
       if (c->mode == COQUI_B200_FP64)
         cq::launch_pi_fused<double>((const double2*)gp, (const double2*)gn, (double2*)dst, ncol,
-                                    c->g, sp, c->st);
+                                    c->g, sp, c->st, ts);
       else
         cq::launch_pi_fused<float>((const float2*)gp, (const float2*)gn, (float2*)dst, ncol, c->g,
-                                   sp, c->st);
+                                   sp, c->st, ts);
     }
   }
   c->gcache_valid = (cache != nullptr);
@@ -1453,8 +1518,16 @@ void sigma_device(Ctx* c, double* host_out) {
     tau_chunk_range(c, i, &a, &b);
     const bool cached = cache && gchunk_cached(c, b);
     if (!cached) wait_G_chunk(c, i);
-    for (int64_t it = a; it < b; ++it) {
+    cq::TauSlices ts;
+    if (cached) {
+      ts.n = b - a;
+      ts.sp = nk * ncol;
+      ts.sn = -ts.sp;
+      ts.sw = c->nq * ncol;
+    }
+    for (int64_t it = a; it < b; it += ts.n) {
       const bool minus = it < nt / 2;  // thc_gw.icc:59-61 writes Sigma(nt-1-it) for it < nt/2
+      ts.n_minus = std::min(ts.n, std::max<int64_t>(nt / 2 - it, 0));
       unsigned char* gp = c->Gp.p;
       unsigned char* gn = minus ? c->Gn.p : nullptr;
       if (cached) {
@@ -1469,10 +1542,10 @@ void sigma_device(Ctx* c, double* host_out) {
         cq::Prof::Scope sc(&c->prof, "sigma_fused");
         if (c->mode == COQUI_B200_FP64)
           cq::launch_sigma_fused<double>((double2*)gp, (double2*)gn, (double2*)WR, (double2*)gp,
-                                         (double2*)gn, ncol, c->g, c->st);
+                                         (double2*)gn, ncol, c->g, c->st, ts);
         else
           cq::launch_sigma_fused<float>((float2*)gp, (float2*)gn, (float2*)WR, (float2*)gp,
-                                        (float2*)gn, ncol, c->g, c->st);
+                                        (float2*)gn, ncol, c->g, c->st, ts);
       }
       if (!cached) {
         project_a2p(c, gp, c->Sig.p + it * gsz);

@@ -465,7 +465,7 @@ template <typename R, int TILE, int NC>
 __global__ void __launch_bounds__(2 * NC * TILE) k_pi_plane(const cplx_t<R>* __restrict__ Gp,
                                                            const cplx_t<R>* __restrict__ Gn,
                                                            cplx_t<R>* __restrict__ Pi,
-                                                           int64_t ncol, R scale) {
+                                                           int64_t ncol, R scale, TauSlices ts) {
   using C = cplx_t<R>;
   constexpr int P = NC * NC, NK = NC * P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -474,9 +474,10 @@ __global__ void __launch_bounds__(2 * NC * TILE) k_pi_plane(const cplx_t<R>* __r
   const int h = threadIdx.x / (NC * TILE), r = threadIdx.x % (NC * TILE);
   const int i0 = r / TILE, c = r % TILE;
   const int64_t ntiles = (ncol + TILE - 1) / TILE;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t col0 = t * TILE;
-    plane_load_dft<C, TILE, NC>(h ? B : A, h ? Gn : Gp, i0, c, ncol, col0, -1);
+  for (int64_t t = blockIdx.x; t < ntiles * ts.n; t += gridDim.x) {
+    const int64_t b = t / ntiles, col0 = (t - b * ntiles) * TILE;
+    plane_load_dft<C, TILE, NC>(h ? B : A, h ? Gn + b * ts.sn : Gp + b * ts.sp, i0, c, ncol, col0,
+                                -1);
     __syncthreads();
     outer_pointwise<C, TILE, NC>(A, B, false, P, [](C (&)[NC], int, int) {},
                                  [&](C (&a)[NC], C (&b)[NC], C (&)[NC]) {
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(2 * NC * TILE) k_pi_plane(const cplx_t<R>* __r
       for (int m = 0; m < NC; ++m) a[m] = cscale(cmulc(a[m], b[m]), scale);
     });
     __syncthreads();
-    if (h == 0) plane_dft_store<C, TILE, NC>(A, Pi, i0, c, ncol, col0, +1);
+    if (h == 0) plane_dft_store<C, TILE, NC>(A, Pi + b * ts.sw, i0, c, ncol, col0, +1);
     __syncthreads();
   }
 }
@@ -521,22 +522,29 @@ __global__ void __launch_bounds__(2 * NC * TILE) k_sigma_plane(const cplx_t<R>* 
                                                               const cplx_t<R>* Gm,
                                                               const cplx_t<R>* __restrict__ WR,
                                                               cplx_t<R>* Sp, cplx_t<R>* Sm,
-                                                              int64_t ncol, R scale) {
+                                                              int64_t ncol, R scale,
+                                                              TauSlices ts) {
   using C = cplx_t<R>;
   constexpr int P = NC * NC, NK = NC * P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* A = reinterpret_cast<C*>(smem_raw);
   C* B = A + NK * TILE;
   C* Wt = B + NK * TILE;
-  const bool has_m = (Gm != nullptr);
   const int h = threadIdx.x / (NC * TILE), r = threadIdx.x % (NC * TILE);
   const int i0 = r / TILE, c = r % TILE;
-  const bool owns = (h == 0) || has_m;
   const int64_t ntiles = (ncol + TILE - 1) / TILE;
-  if (blockIdx.x < ntiles) w_tile_async<C, TILE, NK>(Wt, WR, ncol, (int64_t)blockIdx.x * TILE);
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t col0 = t * TILE;
-    if (owns) plane_load_dft<C, TILE, NC>(h ? B : A, h ? Gm : Gp, i0, c, ncol, col0, -1);
+  const int64_t total = ntiles * ts.n;
+  auto w_async = [&](int64_t t) {
+    const int64_t b = t / ntiles;
+    w_tile_async<C, TILE, NK>(Wt, WR + b * ts.sw, ncol, (t - b * ntiles) * TILE);
+  };
+  if (blockIdx.x < total) w_async(blockIdx.x);
+  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const int64_t b = t / ntiles, col0 = (t - b * ntiles) * TILE;
+    const bool has_m = b < ts.n_minus, owns = (h == 0) || has_m;
+    if (owns)
+      plane_load_dft<C, TILE, NC>(h ? B : A, h ? Gm + b * ts.sn : Gp + b * ts.sp, i0, c, ncol,
+                                  col0, -1);
     cp_async_wait_all();
     __syncthreads();
     outer_pointwise<C, TILE, NC>(A, has_m ? B : nullptr, true, P,
@@ -552,9 +560,10 @@ __global__ void __launch_bounds__(2 * NC * TILE) k_sigma_plane(const cplx_t<R>* 
       }
     });
     __syncthreads();
-    const int64_t tn = t + gridDim.x;
-    if (tn < ntiles) w_tile_async<C, TILE, NK>(Wt, WR, ncol, tn * TILE);
-    if (owns) plane_dft_store<C, TILE, NC>(h ? B : A, h ? Sm : Sp, i0, c, ncol, col0, +1);
+    if (t + gridDim.x < total) w_async(t + gridDim.x);
+    if (owns)
+      plane_dft_store<C, TILE, NC>(h ? B : A, h ? Sm + b * ts.sn : Sp + b * ts.sp, i0, c, ncol,
+                                   col0, +1);
     __syncthreads();
   }
 }
@@ -600,7 +609,8 @@ template <typename R, int TILE, int NC>
 __global__ void __launch_bounds__(256) k_pi_fused(const cplx_t<R>* __restrict__ Gp,
                                                   const cplx_t<R>* __restrict__ Gn,
                                                   cplx_t<R>* __restrict__ Pi, int64_t ncol,
-                                                  int rn0, int rn1, int rn2, R scale) {
+                                                  int rn0, int rn1, int rn2, R scale,
+                                                  TauSlices ts) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n0 = NC ? NC : rn0, n1 = NC ? NC : rn1, n2 = NC ? NC : rn2;
@@ -608,10 +618,11 @@ __global__ void __launch_bounds__(256) k_pi_fused(const cplx_t<R>* __restrict__ 
   C* A = reinterpret_cast<C*>(smem_raw);
   C* B = A + nk * TILE;
   const int64_t ntiles = (ncol + TILE - 1) / TILE;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t col0 = t * TILE;
+  for (int64_t t = blockIdx.x; t < ntiles * ts.n; t += gridDim.x) {
+    const int64_t bt = t / ntiles, col0 = (t - bt * ntiles) * TILE;
     with_n(n2, [&](auto N2) {
-      load_dft_inner2<C, TILE, decltype(N2)::value>(A, Gp, B, Gn, nk, ncol, col0, -1);
+      load_dft_inner2<C, TILE, decltype(N2)::value>(A, Gp + bt * ts.sp, B, Gn + bt * ts.sn, nk,
+                                                    ncol, col0, -1);
     });
     __syncthreads();
     mid_pass<C, TILE, NC>(A, n1, n2, nk, -1);
@@ -629,7 +640,7 @@ __global__ void __launch_bounds__(256) k_pi_fused(const cplx_t<R>* __restrict__ 
     mid_pass<C, TILE, NC>(A, n1, n2, nk, +1);
     __syncthreads();
     with_n(n2, [&](auto N2) {
-      dft_inner_store<C, TILE, decltype(N2)::value>(A, Pi, nk, ncol, col0, +1);
+      dft_inner_store<C, TILE, decltype(N2)::value>(A, Pi + bt * ts.sw, nk, ncol, col0, +1);
     });
     __syncthreads();
   }
@@ -641,19 +652,22 @@ template <typename R, int TILE, int NC>
 __global__ void __launch_bounds__(256) k_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm,
                                                      const cplx_t<R>* __restrict__ WR,
                                                      cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol,
-                                                     int rn0, int rn1, int rn2, R scale) {
+                                                     int rn0, int rn1, int rn2, R scale,
+                                                     TauSlices ts) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n0 = NC ? NC : rn0, n1 = NC ? NC : rn1, n2 = NC ? NC : rn2;
   const int nk = n0 * n1 * n2;
   C* A = reinterpret_cast<C*>(smem_raw);
   C* B = A + nk * TILE;
-  const bool has_m = (Gm != nullptr);
   const int64_t ntiles = (ncol + TILE - 1) / TILE;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t col0 = t * TILE;
+  for (int64_t t = blockIdx.x; t < ntiles * ts.n; t += gridDim.x) {
+    const int64_t bt = t / ntiles, col0 = (t - bt * ntiles) * TILE;
+    const bool has_m = bt < ts.n_minus;
+    const C* W = WR + bt * ts.sw;
     with_n(n2, [&](auto N2) {
-      load_dft_inner2<C, TILE, decltype(N2)::value>(A, Gp, B, has_m ? Gm : nullptr, nk, ncol,
+      load_dft_inner2<C, TILE, decltype(N2)::value>(A, Gp + bt * ts.sp, B,
+                                                    has_m ? Gm + bt * ts.sn : nullptr, nk, ncol,
                                                     col0, -1);
     });
     __syncthreads();
@@ -670,7 +684,7 @@ __global__ void __launch_bounds__(256) k_sigma_fused(const cplx_t<R>* Gp, const 
         for (int m = 0; m < N; ++m) {
           w[m].x = 0;
           w[m].y = 0;
-          if (col < ncol) w[m] = WR[(int64_t)(inner + m * stride) * ncol + col];
+          if (col < ncol) w[m] = W[(int64_t)(inner + m * stride) * ncol + col];
         }
       }, [&](C (&a)[N], C (&b)[N], C (&w)[N]) {
 #pragma unroll
@@ -686,8 +700,9 @@ __global__ void __launch_bounds__(256) k_sigma_fused(const cplx_t<R>* Gp, const 
     if (has_m) mid_pass<C, TILE, NC>(B, n1, n2, nk, +1);
     __syncthreads();
     with_n(n2, [&](auto N2) {
-      dft_inner_store<C, TILE, decltype(N2)::value>(A, Sp, nk, ncol, col0, +1);
-      if (has_m) dft_inner_store<C, TILE, decltype(N2)::value>(B, Sm, nk, ncol, col0, +1);
+      dft_inner_store<C, TILE, decltype(N2)::value>(A, Sp + bt * ts.sp, nk, ncol, col0, +1);
+      if (has_m)
+        dft_inner_store<C, TILE, decltype(N2)::value>(B, Sm + bt * ts.sn, nk, ncol, col0, +1);
     });
     __syncthreads();
   }
@@ -762,7 +777,11 @@ static int cubic_edge(KGrid g) {
 template <typename R>
 __global__ void __launch_bounds__(256) k_pi_gamma(const cplx_t<R>* __restrict__ Gp,
                                                   const cplx_t<R>* __restrict__ Gn,
-                                                  cplx_t<R>* __restrict__ Pi, int64_t n, R scale) {
+                                                  cplx_t<R>* __restrict__ Pi, int64_t n, R scale,
+                                                  TauSlices ts) {
+  Gp += blockIdx.y * ts.sp;
+  Gn += blockIdx.y * ts.sn;
+  Pi += blockIdx.y * ts.sw;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     Pi[i] = cscale(cmulc(Gp[i], Gn[i]), scale);
@@ -771,12 +790,20 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_sigma_gamma(const cplx_t<R>* Gp, const cplx_t<R>* Gm,
                                                      const cplx_t<R>* __restrict__ WR,
                                                      cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t n,
-                                                     R scale) {
+                                                     R scale, TauSlices ts) {
+  const bool has_m = blockIdx.y < ts.n_minus;
+  Gp += blockIdx.y * ts.sp;
+  Sp += blockIdx.y * ts.sp;
+  WR += blockIdx.y * ts.sw;
+  if (has_m) {
+    Gm += blockIdx.y * ts.sn;
+    Sm += blockIdx.y * ts.sn;
+  }
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const cplx_t<R> w = cscale(WR[i], scale);
     Sp[i] = cmul(Gp[i], w);
-    if (Gm) Sm[i] = cmul(Gm[i], w);
+    if (has_m) Sm[i] = cmul(Gm[i], w);
   }
 }
 template <typename R>
@@ -792,26 +819,29 @@ __global__ void __launch_bounds__(256) k_scale_batch(cplx_t<R>* buf, int64_t nco
 
 template <typename R>
 void launch_pi_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gn, cplx_t<R>* Pi, int64_t ncol,
-                     KGrid g, double sp, cudaStream_t s) {
+                     KGrid g, double sp, cudaStream_t s, const TauSlices& ts) {
   check_grid(g);
+  CQ_REQUIRE(ts.n >= 1 && ts.n <= 65535, COQUI_B200_EINVAL, "bad number of tau slices");
   const int nk = g.nk();
   const R scale = (R)(sp / ((double)nk * (double)nk));
   if (nk == 1) {
-    k_pi_gamma<R><<<grid_for(ncol, 256), 256, 0, s>>>(Gp, Gn, Pi, ncol, scale);
+    k_pi_gamma<R><<<dim3(grid_for(ncol, 256), (unsigned)ts.n), 256, 0, s>>>(Gp, Gn, Pi, ncol,
+                                                                            scale, ts);
     CQ_LAUNCHED();
     return;
   }
   const int tile = pick_tile<R>(nk);
   const size_t smem = (size_t)2 * nk * tile * sizeof(cplx_t<R>);
   const int64_t ntiles = (ncol + tile - 1) / tile;
-  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, 148 * 16);
+  const unsigned grid = (unsigned)std::min<int64_t>(ntiles * ts.n, 148 * 16);
 #define CQ_PI_LAUNCH(T)                                                                    \
   CQ_DISPATCH_NC(g, if constexpr (use_plane<R, NCV>()) {                                     \
     set_smem((const void*)k_pi_plane<R, T, NCV>, smem);                                      \
-    k_pi_plane<R, T, NCV><<<grid, 2 * NCV * T, smem, s>>>(Gp, Gn, Pi, ncol, scale);          \
+    k_pi_plane<R, T, NCV><<<grid, 2 * NCV * T, smem, s>>>(Gp, Gn, Pi, ncol, scale, ts);      \
   } else {                                                                                   \
     set_smem((const void*)k_pi_fused<R, T, NCV>, smem);                                      \
-    k_pi_fused<R, T, NCV><<<grid, 256, smem, s>>>(Gp, Gn, Pi, ncol, g.n0, g.n1, g.n2, scale); \
+    k_pi_fused<R, T, NCV><<<grid, 256, smem, s>>>(Gp, Gn, Pi, ncol, g.n0, g.n1, g.n2, scale,  \
+                                                  ts);                                       \
   })
   if (tile == 32) {
     CQ_PI_LAUNCH(32)
@@ -824,29 +854,35 @@ void launch_pi_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gn, cplx_t<R>* Pi, in
 
 template <typename R>
 void launch_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm, const cplx_t<R>* WR,
-                        cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol, KGrid g, cudaStream_t s) {
+                        cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol, KGrid g, cudaStream_t s,
+                        const TauSlices& slices) {
   check_grid(g);
+  CQ_REQUIRE(slices.n >= 1 && slices.n <= 65535, COQUI_B200_EINVAL, "bad number of tau slices");
+  TauSlices ts = slices;
+  if (!Gm) ts.n_minus = 0;
   const int nk = g.nk();
   // Sigma = f_kR [ -(f_Rk G) * W_R ]; f_Rk carries 1/nk
   const R scale = (R)(-1.0 / (double)nk);
   if (nk == 1) {
-    k_sigma_gamma<R><<<grid_for(ncol, 256), 256, 0, s>>>(Gp, Gm, WR, Sp, Sm, ncol, scale);
+    k_sigma_gamma<R><<<dim3(grid_for(ncol, 256), (unsigned)ts.n), 256, 0, s>>>(
+        Gp, Gm, WR, Sp, Sm, ncol, scale, ts);
     CQ_LAUNCHED();
     return;
   }
   const int tile = pick_tile<R>(nk);
   const size_t smem = (size_t)2 * nk * tile * sizeof(cplx_t<R>);
   const int64_t ntiles = (ncol + tile - 1) / tile;
-  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, 148 * 16);
+  const unsigned grid = (unsigned)std::min<int64_t>(ntiles * ts.n, 148 * 16);
 #define CQ_SIGMA_LAUNCH(T)                                                                  \
   CQ_DISPATCH_NC(g, if constexpr (use_plane<R, NCV>()) {                                      \
     const size_t smem3 = smem / 2 * 3; /* G+, G- and W tiles */                               \
     set_smem((const void*)k_sigma_plane<R, T, NCV>, smem3);                                   \
-    k_sigma_plane<R, T, NCV><<<grid, 2 * NCV * T, smem3, s>>>(Gp, Gm, WR, Sp, Sm, ncol, scale); \
+    k_sigma_plane<R, T, NCV><<<grid, 2 * NCV * T, smem3, s>>>(Gp, Gm, WR, Sp, Sm, ncol, scale, \
+                                                              ts);                            \
   } else {                                                                                    \
     set_smem((const void*)k_sigma_fused<R, T, NCV>, smem);                                    \
     k_sigma_fused<R, T, NCV><<<grid, 256, smem, s>>>(Gp, Gm, WR, Sp, Sm, ncol, g.n0, g.n1,    \
-                                                     g.n2, scale);                            \
+                                                     g.n2, scale, ts);                        \
   })
   if (tile == 32) {
     CQ_SIGMA_LAUNCH(32)
@@ -1399,9 +1435,10 @@ void launch_gemm_simt(const GemmDesc& d, const TA* A, const TB* B, TC* C, cudaSt
 // ---------------------------------------------------------------------------------------
 #define CQ_INST(R)                                                                                \
   template void launch_pi_fused<R>(const cplx_t<R>*, const cplx_t<R>*, cplx_t<R>*, int64_t,     \
-                                   KGrid, double, cudaStream_t);                                \
+                                   KGrid, double, cudaStream_t, const TauSlices&);          \
   template void launch_sigma_fused<R>(const cplx_t<R>*, const cplx_t<R>*, const cplx_t<R>*,    \
-                                      cplx_t<R>*, cplx_t<R>*, int64_t, KGrid, cudaStream_t);    \
+                                      cplx_t<R>*, cplx_t<R>*, int64_t, KGrid, cudaStream_t, \
+                                      const TauSlices&);                                        \
   template void launch_dft_plain<R>(cplx_t<R>*, int64_t, KGrid, int, double, int64_t, int64_t,  \
                                     cudaStream_t);                                              \
   template void launch_ir_transform<R>(cplx_t<R>*, int64_t, int, int, const double2*,           \

@@ -13,18 +13,28 @@ struct KGrid {
 
 void upload_twiddles();
 
+// tau slices of one Pi / Sigma launch, in elements: slice b works on G(tau) at Gp + b sp (Sigma
+// is written beside it with the same stride), G(beta - tau) at Gn + b sn and Pi / W at + b sw;
+// Sigma(beta - tau) is formed for the first n_minus slices.  One launch over a whole tau chunk:
+// the slices of a small system (8 k-points, N_mu 128) fill a fraction of the GPU each.
+struct TauSlices {
+  int64_t n = 1, n_minus = 1;
+  int64_t sp = 0, sn = 0, sw = 0;
+};
+
 // Pi(tau) columns: Pi[q, c] = sp * IDFT_R->q( DFT_k->R(Gp)[R, c] * conj(DFT_k->R(Gn)[R, c]) )
 // with the reference's normalisation (f_Rk = e^{-ikR}/nk, f_qR = e^{+iqR}).
 // Arrays are (nk, ncol) row-major in storage precision R.
 template <typename R>
 void launch_pi_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gn, cplx_t<R>* Pi, int64_t ncol,
-                     KGrid g, double sp, cudaStream_t s);
+                     KGrid g, double sp, cudaStream_t s, const TauSlices& ts = {});
 
 // Sigma(tau) and Sigma(beta - tau) columns from G(tau), G(beta - tau) and W_R(tau):
 // S = IDFT_R->k( -DFT_k->R(G) * W_R ).  Sm/Gm may be null (skipped).
 template <typename R>
 void launch_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm, const cplx_t<R>* WR,
-                        cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol, KGrid g, cudaStream_t s);
+                        cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol, KGrid g, cudaStream_t s,
+                        const TauSlices& ts = {});
 
 // In-place 3D DFT over the leading k index of nbatch blocks of (nk, ncol):
 // sign = -1 with scale 1/nk is f_Rk; sign = +1 with scale 1 is f_kR.
