@@ -18,6 +18,7 @@
 
 #include "chol.cuh"
 #include "dyson.cuh"
+#include "hostcopy.cuh"
 #include "kernels.cuh"
 #include "mlp.cuh"
 #include "scgw.cuh"
@@ -77,6 +78,7 @@ struct coqui_b200_ctx {
   int mode = COQUI_B200_MIXED;
   int dev = 0;
   std::string err;
+  cq::StageUser staging;  // keeps the pageable copies' staging buffers while a context lives
   cudaStream_t st = nullptr;
   int64_t launch_base = 0;
   bool have_ir = false, have_k = false, have_thc = false, w_valid = false, w_in_R = false;
@@ -321,10 +323,10 @@ void zgemm_rm_ptrs(Ctx* c, char opA, char opB, int64_t M, int64_t N, int64_t K, 
 }
 
 void upload(Ctx* c, void* dst, const void* src, size_t bytes) {
-  CQ_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->st));
+  cq::copy_to_device(dst, src, bytes, c->st);
 }
 void download(Ctx* c, void* dst, const void* src, size_t bytes) {
-  CQ_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->st));
+  cq::copy_from_device(dst, src, bytes, c->st);
 }
 
 void require_ready(Ctx* c, bool thc, bool ir, bool k) {
@@ -460,15 +462,6 @@ int64_t n_tau_chunks(Ctx* c) { return (c->nth + tau_chunk(c) - 1) / tau_chunk(c)
 void tau_chunk_range(Ctx* c, int64_t i, int64_t* a, int64_t* b) {
   *a = i * tau_chunk(c);
   *b = std::min<int64_t>(c->nth, *a + tau_chunk(c));
-}
-
-bool is_pinned(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeHost;
 }
 
 // make the compute stream wait for the G slices of chunk i (pipelined upload only)
@@ -613,7 +606,7 @@ void upload_G(Ctx* c, const double* G_tskij) {
   c->G.ensure(n);
   c->gcache_valid = false;
   c->g_resident = true;
-  if (!is_pinned(G_tskij)) {
+  if (!cq::host_is_pinned(G_tskij)) {
     c->g_pipelined = false;
     upload(c, c->G.p, G_tskij, n * sizeof(double2));
     return;
@@ -1512,7 +1505,7 @@ void sigma_device(Ctx* c, double* host_out) {
   unsigned char* cache = c->gcache_valid ? c->Gcache.p : nullptr;
   c->gcache_valid = false;
   // with the q -> 0 correction, Sigma leaves once it is complete
-  const bool pipe_out = host_out && is_pinned(host_out) && !corr;
+  const bool pipe_out = host_out && cq::host_is_pinned(host_out) && !corr;
   for (int64_t i = 0; i < n_tau_chunks(c); ++i) {
     int64_t a, b;
     tau_chunk_range(c, i, &a, &b);
@@ -1870,7 +1863,7 @@ int coqui_b200_gw_iteration(coqui_b200_ctx* c, const double* G_tskij, double* Si
     // buffers and replayed by the following ones
     // page-locked host buffers: the copies join the graph
     if (!eps_inv_head && c->mode == COQUI_B200_MIXED && !c->prof.on && !div_active(c) &&
-        (G_tskij ? is_pinned(G_tskij) : c->g_resident) && (!Sigma_tskij || is_pinned(Sigma_tskij))) {
+        (G_tskij ? cq::host_is_pinned(G_tskij) : c->g_resident) && (!Sigma_tskij || cq::host_is_pinned(Sigma_tskij))) {
       gw_iteration_graph(c, G_tskij, Sigma_tskij);
       return;
     }
@@ -1972,7 +1965,7 @@ int coqui_b200_rpa_energy(coqui_b200_ctx* c, const double* G_tskij, double* e_rp
     // resident G or a page-locked host G: one CUDA graph, captured on the first of a run of
     // such calls and replayed by the following ones
     if (c->mode == COQUI_B200_MIXED && !c->prof.on &&
-        (G_tskij ? is_pinned(G_tskij) : c->g_resident)) {
+        (G_tskij ? cq::host_is_pinned(G_tskij) : c->g_resident)) {
       rpa_energy_graph(c, G_tskij, e_rpa);
       return;
     }
