@@ -52,6 +52,10 @@ struct SymState {
   DevBuf<int> qsrc;               // (nq_ibz) lexicographic position of -q
   DevBuf<int4> terms;             // (w slab, G slab, conj flags) per (isym, ik, term)
   DevBuf<int2> rows;              // (nsym * nk_ibz): (first term, term count)
+  // the same sums as convolutions (k_sigma_sym): G, W and output row maps, (nk) + 2 (nsym, nk)
+  bool conv = false;
+  DevBuf<int> maps;
+  bool d_identity = false;        // every rotation is the identity
   DevBuf<double2> D;
   // built from the THC data on first use (set_thc clears thc_ready)
   bool thc_ready = false;

@@ -15,9 +15,10 @@
 //
 // The polarizability takes the R-space route because the fused DFT kernels make it one pass
 // over G per tau, where the reference's k-space double loop costs nq_ibz * nk element products;
-// both give the same sums.  The self-energy keeps the reference's term lists: per tau slice one
-// pass stages each column tile of every G(k) and W(q_ibz) in shared memory and forms the rows
-// of all (isym, k_ibz) from there, so G and W cross HBM once however many terms read them.
+// both give the same sums.  The self-energy's rows of one operation are a convolution over the
+// k-grid, formed with DFTs (k_sigma_sym) when there are enough rows, or else summed term by term
+// (k_sigma_ksum); either way each column tile of every G(k) and W(q_ibz) is staged in shared
+// memory, so G and W cross HBM once however many terms read them.
 // defined further down in ctx.cu, inside its extern "C" block (shared with the full-BZ route)
 extern "C" {
 namespace {
@@ -166,14 +167,52 @@ void sym_update_w(Ctx* c) {
   c->w_valid = false;
 }
 
-// Sigma_ab = X^H S X for nkx problems with the given X (FP64 form)
-void a2p_with(Ctx* c, const double2* X, int64_t nkx, const double2* Sk, double2* out) {
+// Whether the convolution form of the self-energy rows (DFTs per operation) is faster than
+// summing the rows' terms (nk_ibz terms per q-point): measured per tau loop at N_mu 256 (ms,
+// terms against convolutions), 4x4x1 with 10 irreducible k-points 0.84 / 1.05, 6x6x1 with 21 and
+// two operations 2.17 / 2.63, 5x4x3 with 31 4.5 / 1.9, 6x6x2 with 42 and two operations 7.7 / 3.4;
+// the cubic grids run DFTs of compile-time shape: 2x2x2 with 8 0.49 / 0.19, 3x3x3 with 14
+// 1.28 / 0.40, 4x4x4 with 36 5.7 / 0.80.
+bool sym_conv_pays(KGrid g, int64_t nk_ibz, int64_t nsym) {
+  const bool cubic = g.n0 == g.n1 && g.n1 == g.n2;
+  return (cubic ? 8 : 12) * nsym <= nk_ibz;
+}
+
+// Sigma_ab = X^H S X for n problems, problem i with X[i % nkx] (FP64 form)
+void a2p_with(Ctx* c, const double2* X, int64_t nkx, int64_t n, const double2* Sk, double2* out) {
   const int64_t nb = c->nb, Np = c->Np;
-  c->Tproj.ensure((size_t)nkx * Np * nb);
-  zgemm_rm(c, 'C', 'N', nb, Np, Np, make_double2(1, 0), X, nb, Np * nb, Sk, Np, Np * Np,
-           make_double2(0, 0), c->Tproj.p, Np, Np * nb, nkx);
-  zgemm_rm(c, 'N', 'N', nb, nb, Np, make_double2(1, 0), c->Tproj.p, Np, Np * nb, X, nb,
-           Np * nb, make_double2(0, 0), out, nb, nb * nb, nkx);
+  c->Tproj.ensure((size_t)n * Np * nb);
+  cq::ZgemmArgs a;
+  a.opA = 'C';
+  a.M = nb;
+  a.N = a.K = Np;
+  a.A = X;
+  a.lda = nb;
+  a.sA = Np * nb;
+  a.a_mod = nkx;
+  a.B = Sk;
+  a.ldb = Np;
+  a.sB = Np * Np;
+  a.C = c->Tproj.p;
+  a.ldc = Np;
+  a.sC = Np * nb;
+  a.batch = n;
+  cq::zgemm(a, c->st);
+  cq::ZgemmArgs o;
+  o.M = o.N = nb;
+  o.K = Np;
+  o.A = c->Tproj.p;
+  o.lda = Np;
+  o.sA = Np * nb;
+  o.B = X;
+  o.ldb = nb;
+  o.sB = Np * nb;
+  o.b_mod = nkx;
+  o.C = out;
+  o.ldc = nb;
+  o.sC = nb * nb;
+  o.batch = n;
+  cq::zgemm(o, c->st);
 }
 
 bool sym_div_active(const Ctx* c) { return c->div != 0 && c->sym->nq_ibz > 1; }
@@ -221,9 +260,9 @@ void sym_eps_head(Ctx* c, double* out) {
     }
 }
 
-// eval_Sigma_all_kspace for t and beta - t into c->Sig (nt, nk_ibz, nb, nb).  Per tau slice:
-// one gather pass forms the Sigma_PQ rows of every (isym, ik), one batched projection takes
-// them to the orbitals at ks_to_k, D^H Sigma_ab D per row, and the rows of each ik are summed.
+// eval_Sigma_all_kspace for t and beta - t into c->Sig (nt, nk_ibz, nb, nb).  A group of tau
+// slices at a time: the Sigma_PQ rows of every (isym, ik), one batched projection of all of them
+// to the orbitals at ks_to_k, D^H Sigma_ab D per row, and the rows of each ik summed.
 void sym_sigma(Ctx* c, double* host_out) {
   SymState& S = *c->sym;
   CQ_REQUIRE(S.w_valid, COQUI_B200_EINVAL, "no screened interaction: call update_w or set_w");
@@ -232,11 +271,16 @@ void sym_sigma(Ctx* c, double* host_out) {
   const int64_t nki = S.nk_ibz, nqi = S.nq_ibz, pp = Np * Np, bb = nb * nb;
   const int64_t nrow = S.nsym * nki;
   const size_t es = c->elem(), slab = (size_t)nk * pp * es;
+  // slices per group: 256 projections fill the GPU (36 of N_mu 384 leave most of it idle), in at
+  // most 512 MB of Sigma_PQ rows
+  const int64_t group = std::max<int64_t>(
+      1, std::min<int64_t>({(256 + nrow - 1) / nrow, nth,
+                            (int64_t)(((size_t)512 << 20) / ((size_t)nrow * pp * es))}));
   c->Gp.ensure(slab);
-  S.Sq.ensure((size_t)nrow * pp * es);
-  S.Sab.ensure((size_t)nrow * bb);
-  S.Tab.ensure((size_t)nrow * bb);
-  S.Rab.ensure((size_t)nrow * bb);
+  S.Sq.ensure((size_t)group * nrow * pp * es);
+  S.Sab.ensure((size_t)group * nrow * bb);
+  S.Tab.ensure((size_t)group * nrow * bb);
+  S.Rab.ensure((size_t)group * nrow * bb);
   c->Sig.ensure((size_t)nt * nki * bb);
   CQ_CHECK_CUDA(cudaMemsetAsync(c->Sig.p, 0, (size_t)nt * nki * bb * sizeof(double2), c->st));
   // G_PQ of every tau is still in the cache when the polarizability of this G just ran
@@ -244,39 +288,85 @@ void sym_sigma(Ctx* c, double* host_out) {
   c->gcache_valid = false;
   const double factor = -1.0 / (double)nk;
   const bool fp64 = (c->mode == COQUI_B200_FP64);
-  for (int64_t it = 0; it < nth; ++it) {
-    for (int minus = 0; minus < 2; ++minus) {
-      const int64_t itg = minus ? nt - it - 1 : it;
-      if (minus && itg == nth - 1) continue;  // odd nt: the middle slice once (thc_gw.icc:297)
-      const unsigned char* g = c->Gp.p;
-      if (cache && gcached(c, itg))
-        g = gslab(c, itg);
-      else
-        project_p2a(c, c->G.p + itg * nk * bb, c->Gp.p);
-      const unsigned char* W = S.PWi.p + (size_t)it * nqi * pp * es;
-      {
+  cq::SymMaps mp;
+  mp.g = S.maps.p;
+  mp.w = S.maps.p + nk;
+  mp.row = S.maps.p + nk + S.nsym * nk;
+  mp.nsym = (int)S.nsym;
+  mp.nki = (int)nki;
+  for (int minus = 0; minus < 2; ++minus) {
+    // odd nt: the middle slice once (thc_gw.icc:297)
+    const int64_t ntau = minus ? nt / 2 : nth;
+    for (int64_t i0 = 0; i0 < ntau; i0 += group) {
+      const int64_t n = std::min(group, ntau - i0);
+      auto slice = [&](int64_t j) { return minus ? nt - (i0 + j) - 1 : i0 + j; };
+      bool all = cache != nullptr;
+      for (int64_t j = 0; j < n; ++j) all = all && gcached(c, slice(j));
+      // the rows of all cached slices of the group in one launch (convolutions only)
+      const int64_t step = all && S.conv ? n : 1;
+      for (int64_t j = 0; j < n; j += step) {
+        const int64_t itg = slice(j);
+        const unsigned char* g = c->Gp.p;
+        if (cache && gcached(c, itg))
+          g = gslab(c, itg);
+        else
+          project_p2a(c, c->G.p + itg * nk * bb, c->Gp.p);
+        const unsigned char* W = S.PWi.p + (size_t)(i0 + j) * nqi * pp * es;
+        unsigned char* Sq = S.Sq.p + (size_t)j * nrow * pp * es;
         cq::Prof::Scope sc(&c->prof, "sigma_ksum");
-        if (fp64)
+        if (S.conv) {
+          cq::TauSlices ts;
+          ts.n = step;
+          ts.sp = (minus ? -1 : 1) * nk * pp;
+          ts.sw = nqi * pp;
+          ts.sn = nrow * pp;
+          if (fp64)
+            cq::launch_sigma_sym<double>((const double2*)g, (const double2*)W, (double2*)Sq, mp, pp,
+                                         c->g, c->st, ts);
+          else
+            cq::launch_sigma_sym<float>((const float2*)g, (const float2*)W, (float2*)Sq, mp, pp,
+                                        c->g, c->st, ts);
+        } else if (fp64) {
           cq::launch_sigma_ksum<double>((const double2*)g, (const double2*)W, S.terms.p, S.rows.p,
-                                        nrow, nk, nqi, pp, factor, (double2*)S.Sq.p, c->st);
-        else
+                                        nrow, nk, nqi, pp, factor, (double2*)Sq, c->st);
+        } else {
           cq::launch_sigma_ksum<float>((const float2*)g, (const float2*)W, S.terms.p, S.rows.p,
-                                       nrow, nk, nqi, pp, factor, (float2*)S.Sq.p, c->st);
+                                       nrow, nk, nqi, pp, factor, (float2*)Sq, c->st);
+        }
       }
       {
-        cq::Prof::Scope sc(&c->prof, "proj_a2p", nrow);
+        cq::Prof::Scope sc(&c->prof, "proj_a2p", n * nrow);
         if (fp64)
-          a2p_with(c, S.Xs.p, nrow, (const double2*)S.Sq.p, S.Sab.p);
+          a2p_with(c, S.Xs.p, nrow, n * nrow, (const double2*)S.Sq.p, S.Sab.p);
         else
-          cq::tc_project_a2p(S.Xtc, (const float2*)S.Sq.p, S.Sab.p, nrow, Np, nb, nrow, c->st);
+          cq::tc_project_a2p(S.Xtc, (const float2*)S.Sq.p, S.Sab.p, nrow, Np, nb, n * nrow, c->st);
       }
-      // D^H Sigma_ab D per (isym, ik) (the identity operation's D is the identity), then the
-      // rows of each ik summed into Sigma(itg, ik)
-      zgemm_rm(c, 'C', 'N', nb, nb, nb, make_double2(1, 0), S.D.p, nb, bb, S.Sab.p, nb, bb,
-               make_double2(0, 0), S.Tab.p, nb, bb, nrow);
-      zgemm_rm(c, 'N', 'N', nb, nb, nb, make_double2(1, 0), S.Tab.p, nb, bb, S.D.p, nb, bb,
-               make_double2(0, 0), S.Rab.p, nb, bb, nrow);
-      cq::launch_add_blocks(S.Rab.p, c->Sig.p + itg * nki * bb, S.nsym, nki * bb, c->st);
+      // D^H Sigma_ab D per (isym, ik), then the rows of each ik summed into Sigma(itg, ik)
+      const double2* rows = S.Sab.p;
+      if (!S.d_identity) {
+        cq::ZgemmArgs a;
+        a.opA = 'C';
+        a.M = a.N = a.K = nb;
+        a.A = S.D.p;
+        a.a_mod = nrow;
+        a.B = S.Sab.p;
+        a.C = S.Tab.p;
+        a.lda = a.ldb = a.ldc = nb;
+        a.sA = a.sB = a.sC = bb;
+        a.batch = n * nrow;
+        cq::zgemm(a, c->st);
+        cq::ZgemmArgs o = a;
+        o.opA = 'N';
+        o.A = S.Tab.p;
+        o.a_mod = 0;
+        o.B = S.D.p;
+        o.b_mod = nrow;
+        o.C = S.Rab.p;
+        cq::zgemm(o, c->st);
+        rows = S.Rab.p;
+      }
+      cq::launch_add_blocks(rows, c->Sig.p + slice(0) * nki * bb, S.nsym, nki * bb, n,
+                            (minus ? -1 : 1) * nki * bb, c->st);
     }
   }
   // Sigma_div_correction on the IBZ k-points (thc_gw.icc:31-33, 446-526)
@@ -464,6 +554,32 @@ extern "C" int coqui_b200_set_symmetry(coqui_b200_ctx* c, const coqui_b200_symme
     }
     for (int64_t q = 0; q < nq; ++q)
       CQ_REQUIRE(seen[q], COQUI_B200_EINVAL, "Qs must list every q-point exactly once");
+    // The sums as convolutions: G~(k) as the terms read it, W~_s(q) at q = qs, or the conjugate
+    // at -qs for a time-reversal q-point, and the k-point of each row.  They hold when no two
+    // q-points of an operation fall on one q and no two rows on one k (any mean field's maps).
+    std::vector<int> maps(nk + 2 * m.nsym * nk, -1);
+    bool conv = true;
+    for (int64_t p = 0; p < nk; ++p) {
+      const int64_t i = inv[p];
+      const bool tr = m.kp_trev[i] != 0;
+      maps[p] = (int)(tr ? S->lex[m.kp_trev_pair[i]] : p) | (tr ? 1 << 30 : 0);
+    }
+    for (int64_t s = 0; s < m.nsym; ++s) {
+      for (int64_t j = 0; j < m.nq_per_s[s]; ++j) {
+        const int64_t qp = m.Qs[s * m.ld_Qs + j], qs = m.qp_to_ibz[qp];
+        const bool tr = m.qp_trev[qp] != 0;
+        const int64_t at = tr ? lex_combine(c, 0, S->lex[qs], -1) : S->lex[qs];
+        int& w = maps[nk + s * nk + at];
+        conv = conv && w < 0;
+        w = (int)qs | (tr ? 1 << 30 : 0);
+      }
+      for (int64_t ik = 0; ik < m.nk_ibz; ++ik) {
+        int& r = maps[nk + m.nsym * nk + s * nk + S->ks_lex[s * m.nk_ibz + ik]];
+        conv = conv && r < 0;
+        r = (int)ik;
+      }
+    }
+    S->conv = conv && sym_conv_pays(c->g, m.nk_ibz, m.nsym);
     // rotations d[isym, k]: identity for the identity operation or when not given
     const int64_t bb = nb * nb;
     S->D_h.assign((size_t)m.nsym * m.nk_ibz * bb, make_double2(0, 0));
@@ -495,6 +611,9 @@ extern "C" int coqui_b200_set_symmetry(coqui_b200_ctx* c, const coqui_b200_symme
     if (!terms.empty()) upload(c, S->terms.p, terms.data(), terms.size() * sizeof(int4));
     S->rows.ensure(rows.size());
     upload(c, S->rows.p, rows.data(), rows.size() * sizeof(int2));
+    S->maps.ensure(maps.size());
+    upload(c, S->maps.p, maps.data(), maps.size() * sizeof(int));
+    S->d_identity = m.nsym == 1 || !m.D;
     S->D.ensure(S->D_h.size());
     upload(c, S->D.p, S->D_h.data(), S->D_h.size() * sizeof(double2));
     CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));

@@ -708,6 +708,113 @@ __global__ void __launch_bounds__(256) k_sigma_fused(const cplx_t<R>* Gp, const 
   }
 }
 
+// load_dft_inner with the row of each k looked up: map[k] is the source row, its complex
+// conjugate with bit 30 set, zero when negative.
+template <typename C, int TILE, int N>
+__device__ __forceinline__ void load_dft_inner_map(C* A, const C* __restrict__ src,
+                                                   const int* __restrict__ map, int nk,
+                                                   int64_t ncol, int64_t col0, int sign) {
+  const int lines = nk / N;
+  for (int i = threadIdx.x; i < lines * TILE; i += blockDim.x) {
+    const int c = i % TILE, line = i / TILE;
+    const int64_t col = col0 + c;
+    C x[N];
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+      const int code = __ldg(map + line * N + m);
+      x[m].x = 0;
+      x[m].y = 0;
+      if (col < ncol && code >= 0) {
+        x[m] = src[(int64_t)(code & 0x3fffffff) * ncol + col];
+        if (code >> 30) x[m].y = -x[m].y;
+      }
+    }
+    dft_line<C, N>(x, sign);
+#pragma unroll
+    for (int m = 0; m < N; ++m) A[(line * N + m) * TILE + c] = x[m];
+  }
+}
+
+// IBZ self-energy rows as convolutions on the whole k-grid (SymMaps in kernels.cuh): per column
+// tile the forward DFT of G once, then per symmetry operation the forward DFT of its W (zero on
+// the q-points of the other operations), the product with G(R) and the inverse in the
+// outermost-dimension sweep, and the rows its k-points need.
+//
+// Summing each row's terms instead (k_sigma_ksum) reads two shared-memory words per term,
+// nk_ibz nq of them per column: 340 us a tau slice at 64 k (36 irreducible), N_mu 384, where this
+// form takes 51 us.  Bound by the shared-memory sweeps (about 15 word accesses per k-point and
+// operation); memory alone would allow 25 us.
+template <typename R, int TILE, int NC>
+__global__ void __launch_bounds__(256) k_sigma_sym(const cplx_t<R>* __restrict__ G,
+                                                   const cplx_t<R>* __restrict__ W,
+                                                   cplx_t<R>* __restrict__ S, SymMaps mp,
+                                                   int64_t ncol, int rn0, int rn1, int rn2, R scale,
+                                                   TauSlices ts) {
+  using C = cplx_t<R>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n0 = NC ? NC : rn0, n1 = NC ? NC : rn1, n2 = NC ? NC : rn2;
+  const int nk = n0 * n1 * n2, stride = n1 * n2;
+  C* A = reinterpret_cast<C*>(smem_raw);
+  C* B = A + nk * TILE;
+  const int64_t ntiles = (ncol + TILE - 1) / TILE;
+  for (int64_t t = blockIdx.x; t < ntiles * ts.n; t += gridDim.x) {
+    const int64_t bt = t / ntiles, col0 = (t - bt * ntiles) * TILE;
+    const C* Wt = W + bt * ts.sw;
+    with_n(n2, [&](auto N2) {
+      constexpr int N = decltype(N2)::value;
+      load_dft_inner_map<C, TILE, N>(A, G + bt * ts.sp, mp.g, nk, ncol, col0, -1);
+      load_dft_inner_map<C, TILE, N>(B, Wt, mp.w, nk, ncol, col0, -1);
+    });
+    __syncthreads();
+    mid_pass<C, TILE, NC>(A, n1, n2, nk, -1);
+    mid_pass<C, TILE, NC>(B, n1, n2, nk, -1);
+    __syncthreads();
+    with_n(n0, [&](auto N0) { dft_dim_n<C, TILE, decltype(N0)::value>(A, stride, nk, -1); });
+    for (int s = 0; s < mp.nsym; ++s) {
+      if (s > 0) {
+        with_n(n2, [&](auto N2) {
+          load_dft_inner_map<C, TILE, decltype(N2)::value>(B, Wt, mp.w + s * nk, nk, ncol, col0, -1);
+        });
+        __syncthreads();
+        mid_pass<C, TILE, NC>(B, n1, n2, nk, -1);
+      }
+      __syncthreads();
+      with_n(n0, [&](auto N0) {
+        constexpr int N = decltype(N0)::value;
+        outer_pointwise<C, TILE, N>(B, (C*)nullptr, false, stride,
+                                    [&](C (&w)[N], int inner, int c) {
+#pragma unroll
+          for (int m = 0; m < N; ++m) w[m] = A[(inner + m * stride) * TILE + c];
+        }, [&](C (&a)[N], C (&)[N], C (&w)[N]) {
+#pragma unroll
+          for (int m = 0; m < N; ++m) a[m] = cscale(cmul(a[m], w[m]), scale);
+        });
+      });
+      __syncthreads();
+      mid_pass<C, TILE, NC>(B, n1, n2, nk, +1);
+      __syncthreads();
+      C* out = S + bt * ts.sn + (int64_t)s * mp.nki * ncol;
+      with_n(n2, [&](auto N2) {
+        constexpr int N = decltype(N2)::value;
+        for (int i = threadIdx.x; i < nk / N * TILE; i += blockDim.x) {
+          const int c = i % TILE, line = i / TILE;
+          const int64_t col = col0 + c;
+          C x[N];
+#pragma unroll
+          for (int m = 0; m < N; ++m) x[m] = B[(line * N + m) * TILE + c];
+          dft_line<C, N>(x, +1);
+#pragma unroll
+          for (int m = 0; m < N; ++m) {
+            const int row = __ldg(mp.row + s * nk + line * N + m);
+            if (row >= 0 && col < ncol) out[(int64_t)row * ncol + col] = x[m];
+          }
+        }
+      });
+      __syncthreads();
+    }
+  }
+}
+
 template <typename R, int TILE, int NC>
 __global__ void __launch_bounds__(256) k_dft_plain(cplx_t<R>* __restrict__ buf, int64_t ncol,
                                                    int rn0, int rn1, int rn2, int sign, R scale,
@@ -890,6 +997,30 @@ void launch_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm, const cplx_t<R
     CQ_SIGMA_LAUNCH(16)
   }
 #undef CQ_SIGMA_LAUNCH
+  CQ_LAUNCHED();
+}
+
+template <typename R>
+void launch_sigma_sym(const cplx_t<R>* G, const cplx_t<R>* W, cplx_t<R>* S, const SymMaps& mp,
+                      int64_t ncol, KGrid g, cudaStream_t s, const TauSlices& ts) {
+  check_grid(g);
+  const int nk = g.nk();
+  // -1/nk of the reference's sum and 1/nk of the inverse DFT
+  const R scale = (R)(-1.0 / ((double)nk * (double)nk));
+  const int tile = pick_tile<R>(nk);
+  const size_t smem = (size_t)2 * nk * tile * sizeof(cplx_t<R>);
+  const int64_t ntiles = (ncol + tile - 1) / tile;
+  const unsigned grid = (unsigned)std::min<int64_t>(ntiles * ts.n, 148 * 16);
+#define CQ_SYM_LAUNCH(T)                                                                    \
+  CQ_DISPATCH_NC(g, set_smem((const void*)k_sigma_sym<R, T, NCV>, smem);                      \
+                 k_sigma_sym<R, T, NCV><<<grid, 256, smem, s>>>(G, W, S, mp, ncol, g.n0, g.n1, \
+                                                                g.n2, scale, ts))
+  if (tile == 32) {
+    CQ_SYM_LAUNCH(32)
+  } else {
+    CQ_SYM_LAUNCH(16)
+  }
+#undef CQ_SYM_LAUNCH
   CQ_LAUNCHED();
 }
 
@@ -1439,6 +1570,9 @@ void launch_gemm_simt(const GemmDesc& d, const TA* A, const TB* B, TC* C, cudaSt
   template void launch_sigma_fused<R>(const cplx_t<R>*, const cplx_t<R>*, const cplx_t<R>*,    \
                                       cplx_t<R>*, cplx_t<R>*, int64_t, KGrid, cudaStream_t, \
                                       const TauSlices&);                                        \
+  template void launch_sigma_sym<R>(const cplx_t<R>*, const cplx_t<R>*, cplx_t<R>*,             \
+                                    const SymMaps&, int64_t, KGrid, cudaStream_t,               \
+                                    const TauSlices&);                                          \
   template void launch_dft_plain<R>(cplx_t<R>*, int64_t, KGrid, int, double, int64_t, int64_t,  \
                                     cudaStream_t);                                              \
   template void launch_ir_transform<R>(cplx_t<R>*, int64_t, int, int, const double2*,           \

@@ -36,6 +36,22 @@ void launch_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm, const cplx_t<R
                         cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol, KGrid g, cudaStream_t s,
                         const TauSlices& ts = {});
 
+// Row maps of the IBZ self-energy as convolutions: operation s contributes
+//   S[s, ik] = -1/nk sum_q G~(k - q) W~_s(q),  row[s, k] = ik,
+// with G~(k) the row g[k] of G and W~_s(q) the row w[s, q] of W (the complex conjugate with bit
+// 30 set, zero when negative); row[s, k] is -1 where no irreducible k-point needs S.
+struct SymMaps {
+  const int* g = nullptr;    // (nk)
+  const int* w = nullptr;    // (nsym, nk)
+  const int* row = nullptr;  // (nsym, nk)
+  int nsym = 1, nki = 1;
+};
+// G (nk, ncol), W (nq_ibz, ncol) and S (nsym, nki, ncol) of ts.n tau slices, ts.sp, ts.sw and
+// ts.sn elements apart.
+template <typename R>
+void launch_sigma_sym(const cplx_t<R>* G, const cplx_t<R>* W, cplx_t<R>* S, const SymMaps& mp,
+                      int64_t ncol, KGrid g, cudaStream_t s, const TauSlices& ts);
+
 // In-place 3D DFT over the leading k index of nbatch blocks of (nk, ncol):
 // sign = -1 with scale 1/nk is f_Rk; sign = +1 with scale 1 is f_kR.
 template <typename R>

@@ -171,9 +171,11 @@ void launch_sigma_ksum(const cplx_t<R>* G, const cplx_t<R>* W, const int4* terms
   CQ_CHECK_CUDA(cudaGetLastError());
 }
 
-// out[i] += sum_s R[s * n + i]
+// slice y: out[y ostep + i] += sum over b of Rb[(y nblk + b) n + i]
 __global__ void k_add_blocks(const double2* __restrict__ Rb, double2* __restrict__ out,
-                             int64_t nblk, int64_t n) {
+                             int64_t nblk, int64_t n, int64_t ostep) {
+  Rb += blockIdx.y * nblk * n;
+  out += blockIdx.y * ostep;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     double2 a = out[i];
@@ -186,8 +188,10 @@ __global__ void k_add_blocks(const double2* __restrict__ Rb, double2* __restrict
   }
 }
 
-void launch_add_blocks(const double2* Rb, double2* out, int64_t nblk, int64_t n, cudaStream_t s) {
-  k_add_blocks<<<grid_for(n, 256), 256, 0, s>>>(Rb, out, nblk, n);
+void launch_add_blocks(const double2* Rb, double2* out, int64_t nblk, int64_t n, int64_t nslice,
+                       int64_t ostep, cudaStream_t s) {
+  CQ_REQUIRE(nslice >= 1 && nslice <= 65535, COQUI_B200_EINVAL, "add_blocks: bad slice count");
+  k_add_blocks<<<dim3(grid_for(n, 256), (unsigned)nslice), 256, 0, s>>>(Rb, out, nblk, n, ostep);
   count_launch(1);
   CQ_CHECK_CUDA(cudaGetLastError());
 }

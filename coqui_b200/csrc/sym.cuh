@@ -33,7 +33,9 @@ void launch_sigma_ksum(const cplx_t<R>* G, const cplx_t<R>* W, const int4* terms
                        const int2* rows, int64_t nrow, int64_t nk, int64_t nqi, int64_t ncol,
                        double factor, cplx_t<R>* S, cudaStream_t s);
 
-// out[i] += sum over b < nblk of Rb[b * n + i] (complex128)
-void launch_add_blocks(const double2* Rb, double2* out, int64_t nblk, int64_t n, cudaStream_t s);
+// out[y ostep + i] += sum over b < nblk of Rb[(y nblk + b) n + i] for the slices y < nslice
+// (complex128)
+void launch_add_blocks(const double2* Rb, double2* out, int64_t nblk, int64_t n, int64_t nslice,
+                       int64_t ostep, cudaStream_t s);
 
 }  // namespace cq

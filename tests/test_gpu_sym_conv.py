@@ -1,0 +1,37 @@
+"""The IBZ self-energy on grids where its rows are formed as convolutions (enough irreducible
+k-points per operation; cubic and non-cubic grids, odd edges, one and two operations, whole and
+partial groups of tau slices) against the k-space oracle, with an odd number of tau points too.
+Tolerances as the other IBZ parity tests."""
+import numpy as np
+import pytest
+
+from coqui_b200 import capi
+from coqui_b200.iaft import IAFT as ProductIAFT
+from coqui_b200.symmetry import symmetric_system
+from oracle import sym_oracle as SO
+from oracle import thc_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind,grid,lam", [("trev", (2, 2, 2), 1e4), ("trev", (3, 3, 3), 1e5),
+                                           ("trev", (5, 2, 3), 1e4), ("swap", (5, 5, 2), 1e4)])
+@pytest.mark.parametrize("mode,tol", [(capi.FP64, 1e-10), (capi.MIXED, 1e-6)], ids=["fp64", "mixed"])
+def test_convolution_rows_match_the_term_sums(kind, grid, lam, mode, tol):
+    ft, pft = O.IAFT(1000.0, lam / 1000.0, "low"), ProductIAFT(1000.0, lam / 1000.0, "low")
+    d = symmetric_system(kind, grid, 5, 19, ft, seed=3)
+    sym = d["sym"]
+    dW = SO.update_w_kspace(d["G_ibz"], d["X"], d["V"], ft, sym)
+    ref = SO.eval_Sigma_all_kspace(d["G_ibz"], dW, d["X"], sym, d["D"])
+    c = capi.Context(sym["nk"], 5, 19, ft.nt_f, ft.nw_b, d["grid"], mode=mode)
+    c.set_ir(pft)
+    c.set_kmesh(d["kpts_lex"], d["lattv"], d["chi_lex"])
+    c.set_thc(d["X_lex"], d["V_lex"])
+    c.set_symmetry(sym, d["D"])
+    S, _ = c.gw_iteration(d["G_ibz"])
+    assert np.abs(S - ref).max() < tol
+    c.set_gcache_limit(0)  # every slice projected on its own
+    S1, _ = c.gw_iteration(d["G_ibz"])
+    assert np.abs(S1 - S).max() < 1e-12
+    assert np.abs(ref).max() > 1e-3
+    c.close()
