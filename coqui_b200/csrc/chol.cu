@@ -21,6 +21,8 @@
 #include <cstdint>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "chol.cuh"
@@ -29,14 +31,9 @@ namespace cq {
 
 namespace {
 
-__device__ __forceinline__ double2 cmul_(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-// a * conj(b)
-__device__ __forceinline__ double2 cmulc_(double2 a, double2 b) {
-  return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
 __device__ __forceinline__ double2 conj_(double2 a) { return make_double2(a.x, -a.y); }
+
+#include "chol_diag.cuh"
 
 // The blocked algorithm (chol_blk.cuh) with 32 x 32 blocks and 64 threads: two staging blocks
 // (34 KB) per problem let six problems share an SM, so that one problem's barriers and loads

@@ -4,7 +4,7 @@
 //   (CTAs per SM for the launch bounds), DMMA (block products on the FP64 tensor cores; needs
 //   CB = 32 and CT = 64), AR x AC (a thread's accumulator tile: 2 x 8 for DMMA, else RT x CTT
 //   with the thread grid TWR = CB / RT by TWC = CB / CTT, CT = TWR * TWC)
-// and the complex helpers cmul_, cmulc_, conj_.  (No include guard: it is meant to be
+// and conj_, factor_invert_diag.  (No include guard: it is meant to be
 // included more than once.)
 // smem tile <- global block (rows r0.., cols c0..) of an ld x ld row-major matrix, rb x cb valid
 __device__ __forceinline__ void load_blk(double2* S, const double2* G, int64_t ld, int64_t r0,
@@ -245,76 +245,13 @@ __device__ __forceinline__ void acc_init(double2 (&acc)[AR][AC], const double2* 
   }
 }
 
-// In-place Cholesky of the lower triangle of S (n x n); adds sum ln C_ii to *ld_acc
-// (thread 0) and sets *bad if a pivot is not positive.  One barrier per column: column c is
-// used unscaled (times 1/d_c) in its rank-1 update and scaled during the next column's step.
-__device__ void factor_diag(double2* S, int n, double* ld_acc, int* bad) {
-  double prev_inv = 1.0, prev_d = 1.0;
-  for (int c = 0; c < n; ++c) {
-    __syncthreads();
-    double d = S[c * PITCH + c].x;
-    const bool good = d > 0.0;
-    d = good ? sqrt(d) : 1.0;
-    const double inv = 1.0 / d;
-    if (c > 0) {  // finish column c - 1: diagonal and scaled entries below it
-      if (threadIdx.x == 0) S[(c - 1) * PITCH + c - 1] = make_double2(prev_d, 0.0);
-      for (int r = c + threadIdx.x; r < n; r += CT) {
-        S[r * PITCH + c - 1].x *= prev_inv;
-        S[r * PITCH + c - 1].y *= prev_inv;
-      }
-    }
-    const int m = n - c - 1;
-    const double inv2 = inv * inv;
-    for (int idx = threadIdx.x; idx < m * m; idx += CT) {
-      const int r = c + 1 + idx / m, s = c + 1 + idx % m;
-      if (s <= r) {
-        const double2 u = cmulc_(S[r * PITCH + c], S[s * PITCH + c]);
-        S[r * PITCH + s].x -= u.x * inv2;
-        S[r * PITCH + s].y -= u.y * inv2;
-      }
-    }
-    if (threadIdx.x == 0) {
-      if (!good) *bad = 1;
-      *ld_acc += log(d);
-    }
-    prev_inv = inv;
-    prev_d = d;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) S[(n - 1) * PITCH + n - 1] = make_double2(prev_d, 0.0);
-  __syncthreads();
-}
-
-// Sinv = inverse of the lower-triangular S (n x n): forward substitution with one column
-// per group of CT / CB lanes of a warp (partial dot products reduced by shuffles).
-__device__ void invert_lower(const double2* S, double2* Sinv, int n) {
-  constexpr int LPC = CT / CB;  // lanes per column
-  for (int i = threadIdx.x; i < CB * CB; i += CT) Sinv[(i / CB) * PITCH + i % CB] = make_double2(0, 0);
-  __syncthreads();
-  const int c = threadIdx.x / LPC, sub = threadIdx.x % LPC;
-  const bool col = c < n;
-  if (col && sub == 0) Sinv[c * PITCH + c] = make_double2(1.0 / S[c * PITCH + c].x, 0.0);
-  __syncwarp();
-  for (int r = 1; r < n; ++r) {
-    double ax = 0, ay = 0;
-    if (col && r > c)
-      for (int k = c + sub; k < r; k += LPC) {
-        const double2 u = cmul_(S[r * PITCH + k], Sinv[k * PITCH + c]);
-        ax += u.x;
-        ay += u.y;
-      }
-#pragma unroll
-    for (int off = LPC / 2; off > 0; off >>= 1) {
-      ax += __shfl_xor_sync(0xffffffffu, ax, off);
-      ay += __shfl_xor_sync(0xffffffffu, ay, off);
-    }
-    if (col && r > c && sub == 0) {
-      const double inv = -1.0 / S[r * PITCH + r].x;
-      Sinv[r * PITCH + c] = make_double2(ax * inv, ay * inv);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
+// Sinv = inverse of the Cholesky factor of S (n x n, lower triangle); adds sum ln C_ii to *ld_acc
+// and sets *bad if a pivot is not positive.
+__device__ __forceinline__ void factor_invert(const double2* S, double2* Sinv, int n,
+                                              double* ld_acc, int* bad) {
+  factor_invert_diag<CT>([&](int r, int c) { return S[r * PITCH + c]; },
+                         [&](int r, int c) -> double2& { return Sinv[r * PITCH + c]; }, n, ld_acc,
+                         bad);
 }
 
 // Column j of X = C^{-1} below the diagonal within its diagonal group (blocks j+1 .. gend-1):
@@ -386,8 +323,7 @@ __device__ void tiled_diag(const float2* M, double2* A, int64_t n, int j, double
   else
     load_blk(S0, A, n, j0, j0, jb, jb);
   __syncthreads();
-  factor_diag(S0, jb, &s_ld, &s_bad);
-  invert_lower(S0, S1, jb);
+  factor_invert(S0, S1, jb, &s_ld, &s_bad);
   store_blk_adjU(S1, A, n, j0, jb);
   if (threadIdx.x == 0) {
     *logdet += 2.0 * s_ld;
@@ -497,8 +433,7 @@ __device__ __forceinline__ void chol_inv_problem(const float2* __restrict__ M,
     else
       load_blk(S0, A, n, j0, j0, jb, jb);
     __syncthreads();
-    factor_diag(S0, jb, &s_ld, &s_bad);
-    invert_lower(S0, S1, jb);
+    factor_invert(S0, S1, jb, &s_ld, &s_bad);
     // C_jj is not needed again; the upper triangle of the diagonal block keeps C_jj^{-H}
     if (INV) store_blk_adjU(S1, A, n, j0, jb);
     __syncthreads();
@@ -624,8 +559,7 @@ __device__ __forceinline__ void chol_inv_problem_left(const float2* __restrict__
 #pragma unroll
       for (int jj = 0; jj < AC; ++jj) S0[acc_row(i, jj) * PITCH + acc_col(i, jj)] = acc[i][jj];
     __syncthreads();
-    factor_diag(S0, jb, &s_ld, &s_bad);
-    invert_lower(S0, S1, jb);
+    factor_invert(S0, S1, jb, &s_ld, &s_bad);
     store_blk_adjU(S1, A, n, j0, jb);  // C_jj^{-H} in the upper triangle
     __syncthreads();
     // 2. panel: L_ib,j = [(I - M)_ib,j - sum_kb L_ib,kb L_j,kb^H] C_jj^{-H}

@@ -1,9 +1,9 @@
 // Left-looking blocked FP64 Cholesky / log-determinant / group inverse of one problem per CTA,
 // four warps, 32 x 32 blocks, two panel row blocks per step.
 //
-// Included once inside a namespace (chol.cu) that provides cmul_, cmulc_ and conj_.  The
+// Included once inside a namespace (chol.cu) that provides conj_ and factor_invert_diag.  The
 // arithmetic of every element is that of the two-warp kernel in chol_blk.cuh (same products
-// in the same order, same diagonal factorisation and inverse), so results are bit-identical;
+// in the same order, same diagonal elimination), so results are bit-identical;
 // what differs is the data movement:
 //  * the panel of block column j is formed two row blocks at a time (warps 0-1 on row block
 //    i, warps 2-3 on row block i + 1), so each block L_j,k is read once per pair: 24 KB of
@@ -188,76 +188,6 @@ __device__ __forceinline__ void to_smem(double2* S, const double2 (&acc)[AR][8],
     for (int j = 0; j < 8; ++j) S[sidx(fr_row(tr0, i), fr_col(j))] = acc[i][j];
 }
 
-// In-place Cholesky of the lower triangle of S (n x n), sum ln C_ii added to *ld_acc by thread
-// 0, *bad set for a non-positive pivot (the column step of chol_blk.cuh's factor_diag).
-__device__ void factor_diag(double2* S, int n, double* ld_acc, int* bad) {
-  double prev_inv = 1.0, prev_d = 1.0;
-  for (int c = 0; c < n; ++c) {
-    __syncthreads();
-    double d = S[sidx(c, c)].x;
-    const bool good = d > 0.0;
-    d = good ? sqrt(d) : 1.0;
-    const double inv = 1.0 / d;
-    if (c > 0) {
-      if (threadIdx.x == 0) S[sidx(c - 1, c - 1)] = make_double2(prev_d, 0.0);
-      for (int r = c + threadIdx.x; r < n; r += NT) {
-        double2& e = S[sidx(r, c - 1)];
-        e.x *= prev_inv;
-        e.y *= prev_inv;
-      }
-    }
-    const int m = n - c - 1;
-    const double inv2 = inv * inv;
-    for (int idx = threadIdx.x; idx < m * m; idx += NT) {
-      const int r = c + 1 + idx / m, s = c + 1 + idx % m;
-      if (s <= r) {
-        const double2 u = cmulc_(S[sidx(r, c)], S[sidx(s, c)]);
-        double2& e = S[sidx(r, s)];
-        e.x -= u.x * inv2;
-        e.y -= u.y * inv2;
-      }
-    }
-    if (threadIdx.x == 0) {
-      if (!good) *bad = 1;
-      *ld_acc += log(d);
-    }
-    prev_inv = inv;
-    prev_d = d;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) S[sidx(n - 1, n - 1)] = make_double2(prev_d, 0.0);
-  __syncthreads();
-}
-
-// Sinv = inverse of the lower-triangular S (n x n): forward substitution, one column per lane
-// pair (threads 0-63; the partial sums of a pair are combined by one shuffle, as in the
-// two-warp kernel).
-__device__ void invert_lower(const double2* S, double2* Sinv, int n) {
-  for (int i = threadIdx.x; i < CB * CB; i += NT) Sinv[i] = make_double2(0, 0);
-  __syncthreads();
-  const int c = threadIdx.x >> 1, sub = threadIdx.x & 1;
-  const bool col = c < n;
-  if (col && sub == 0) Sinv[sidx(c, c)] = make_double2(1.0 / S[sidx(c, c)].x, 0.0);
-  __syncwarp();
-  for (int r = 1; r < n; ++r) {
-    double ax = 0, ay = 0;
-    if (col && r > c)
-      for (int k = c + sub; k < r; k += 2) {
-        const double2 u = cmul_(S[sidx(r, k)], Sinv[sidx(k, c)]);
-        ax += u.x;
-        ay += u.y;
-      }
-    ax += __shfl_xor_sync(0xffffffffu, ax, 1);
-    ay += __shfl_xor_sync(0xffffffffu, ay, 1);
-    if (col && r > c && sub == 0) {
-      const double inv = -1.0 / S[sidx(r, r)].x;
-      Sinv[sidx(r, c)] = make_double2(ax * inv, ay * inv);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-}
-
 // Column j of X = C^{-1} below the diagonal inside its group (blocks j+1 .. gend-1):
 // X_ij = -C_ii^{-1} sum_{k=j}^{i-1} C_ik X_kj, kept as its adjoint in the upper block (j, i).
 __device__ void inverse_column(double2* A, int64_t n, int j, int gend, double2* S0, double2* S1) {
@@ -418,8 +348,9 @@ __device__ __forceinline__ void chol_problem(const MT* __restrict__ M, double2* 
       to_smem(F(0), acc, w);
     }
     __syncthreads();
-    factor_diag(F(0), jb, &s_ld, &s_bad);
-    invert_lower(F(0), F(1), jb);
+    factor_invert_diag<NT>([&](int r, int c) { return F(0)[sidx(r, c)]; },
+                           [&](int r, int c) -> double2& { return F(1)[sidx(r, c)]; }, jb, &s_ld,
+                           &s_bad);
     store_adjU(F(1), A, n, j0, jb);  // C_jj^{-H} in the upper triangle
     __syncthreads();
 
