@@ -955,7 +955,6 @@ int coqui_b200_create(coqui_b200_ctx** out, const coqui_b200_dims* dims) {
     CQ_CHECK_CUDA(cudaStreamCreateWithFlags(&c->cs, cudaStreamNonBlocking));
     CQ_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_st, cudaEventDisableTiming));
     c->prof.st = c->st;
-    cq::upload_twiddles();
     c->launch_base = cq::launches_total();
   });
   if (rc != COQUI_B200_OK) {
@@ -1612,15 +1611,29 @@ void ensure_v_R(Ctx* c) {
 // R -> k, back-projection) with D(k) = X Dm X^H in place of G(tau) and V(R) in place of W(R).
 // J: rho_Q = (2/nk) sum_k (X Dm X^H)_QQ (the R = 0 diagonal of thc_hf.icc:184-190),
 // J = V(q=0) rho (:194-196), F += X^H diag(J) X.
-void hf_device(Ctx* c, const double2* Dm, const double2* S, bool hartree, bool exchange, int div,
-               double madelung, double2* F) {
+//
+// The Hartree part takes T = X Dm from the exchange's projection, before the back-projection
+// reuses its buffer.
+void hf_device(Ctx* c, const double2* Dm, bool hartree, bool exchange, double2* F) {
   cq::Prof::Scope sc(&c->prof, "hf");
   const int64_t nk = c->nk, nb = c->nb, Np = c->Np, ncol = Np * Np;
   const int64_t nF = nk * nb * nb;
+  const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
   if (exchange) {
     ensure_v_R(c);
     c->hfp.ensure((size_t)nk * ncol);
-    p2a_fp64(c, Dm, c->hfp.p, 1);
+    p2a_fp64(c, Dm, c->hfp.p, 1);  // leaves T = X Dm in Tproj
+  } else if (hartree) {
+    c->Tproj.ensure((size_t)nk * Np * nb);
+    zgemm_rm(c, 'N', 'N', Np, nb, nb, one, c->X.p, nb, Np * nb, Dm, nb, nb * nb, zero,
+             c->Tproj.p, nb, Np * nb, nk);
+  }
+  if (hartree) {
+    c->hfv.ensure(2 * Np);
+    cq::aux_diag(c->Tproj.p, c->X.p, c->hfv.p, nk, Np, nb, 2.0 / (double)nk, c->st);
+    cq::matvec(c->V.p, c->hfv.p, c->hfv.p + Np, Np, c->st);
+  }
+  if (exchange) {
     cq::launch_sigma_fused<double>(c->hfp.p, nullptr, c->VR.p, c->hfp.p, nullptr, ncol, c->g,
                                    c->st);
     a2p_fp64(c, c->hfp.p, F, 1);
@@ -1629,24 +1642,21 @@ void hf_device(Ctx* c, const double2* Dm, const double2* S, bool hartree, bool e
   }
   if (hartree) {
     c->Tproj.ensure((size_t)nk * Np * nb);
-    c->hfv.ensure(2 * Np);
-    const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
-    zgemm_rm(c, 'N', 'N', Np, nb, nb, one, c->X.p, nb, Np * nb, Dm, nb, nb * nb, zero,
-             c->Tproj.p, nb, Np * nb, nk);
-    cq::aux_diag(c->Tproj.p, c->X.p, c->hfv.p, nk, Np, nb, 2.0 / (double)nk, c->st);
-    zgemm_rm(c, 'N', 'N', Np, 1, Np, one, c->V.p, Np, 0, c->hfv.p, 1, 0, zero, c->hfv.p + Np, 1,
-             0, 1);
     cq::scale_rows(c->X.p, c->hfv.p + Np, c->Tproj.p, nk, Np, nb, c->st);
     zgemm_rm(c, 'C', 'N', nb, nb, Np, one, c->X.p, nb, Np * nb, c->Tproj.p, nb, Np * nb, one, F,
              nb, nb * nb, nk);
   }
-  if (exchange && div == 1) {
-    c->hft.ensure(nF);
-    zgemm_rm(c, 'N', 'N', nb, nb, nb, make_double2(1, 0), S, nb, nb * nb, Dm, nb, nb * nb,
-             make_double2(0, 0), c->hft.p, nb, nb * nb, nk);
-    zgemm_rm(c, 'N', 'N', nb, nb, nb, make_double2(-madelung, 0), c->hft.p, nb, nb * nb, S, nb,
-             nb * nb, make_double2(1, 0), F, nb, nb * nb, nk);
-  }
+}
+
+// HF_K_correction (hf_t.cpp:45-84): F -= madelung S Dm S
+void hf_gygi_device(Ctx* c, const double2* Dm, const double2* S, double madelung, double2* F) {
+  cq::Prof::Scope sc(&c->prof, "hf");
+  const int64_t nk = c->nk, nb = c->nb;
+  c->hft.ensure(nk * nb * nb);
+  zgemm_rm(c, 'N', 'N', nb, nb, nb, make_double2(1, 0), S, nb, nb * nb, Dm, nb, nb * nb,
+           make_double2(0, 0), c->hft.p, nb, nb * nb, nk);
+  zgemm_rm(c, 'N', 'N', nb, nb, nb, make_double2(-madelung, 0), c->hft.p, nb, nb * nb, S, nb,
+           nb * nb, make_double2(1, 0), F, nb, nb * nb, nk);
 }
 
 // One GW iteration of the resident G as a CUDA graph (update_w + Sigma, no host transfers).
@@ -2157,13 +2167,15 @@ int coqui_b200_hf_evaluate(coqui_b200_ctx* c, const double* Dm_skij, const doubl
     c->hfd.ensure(n);
     c->hff.ensure(n);
     upload(c, c->hfd.p, Dm_skij, n * sizeof(double2));
-    if (gygi) {
-      c->hfs.ensure(n);
-      upload(c, c->hfs.p, S_skij, n * sizeof(double2));
-    }
     c->mark("h2d_Dm");
-    hf_device(c, c->hfd.p, gygi ? c->hfs.p : nullptr, hartree != 0, exchange != 0,
-              div_treatment, madelung, c->hff.p);
+    hf_device(c, c->hfd.p, hartree != 0, exchange != 0, c->hff.p);
+    if (gygi) {  // S crosses on the copy stream while J and K are formed
+      c->hfs.ensure(n);
+      cq::copy_to_device(c->hfs.p, S_skij, n * sizeof(double2), c->cs);
+      CQ_CHECK_CUDA(cudaEventRecord(c->ev_st, c->cs));
+      CQ_CHECK_CUDA(cudaStreamWaitEvent(c->st, c->ev_st, 0));
+      hf_gygi_device(c, c->hfd.p, c->hfs.p, madelung, c->hff.p);
+    }
     c->mark("HF");
     download(c, F_skij, c->hff.p, n * sizeof(double2));
     c->mark("d2h_F");
@@ -2201,7 +2213,8 @@ int coqui_b200_scgw_iteration(coqui_b200_ctx* c, const double* G_tskij, int64_t 
     }
     if (c->hf_on) {  // scf_driver.cpp:94-114: F = J + K of the current density matrix
       if (it == 1) dm_from_g(c);
-      hf_device(c, c->Dm.p, c->Sov.p, true, true, c->hf_div, c->hf_madelung, c->F.p);
+      hf_device(c, c->Dm.p, true, true, c->F.p);
+      if (c->hf_div == 1) hf_gygi_device(c, c->Dm.p, c->Sov.p, c->hf_madelung, c->F.p);
       c->mark("HF");
     }
     update_w_device(c);

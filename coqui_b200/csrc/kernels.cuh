@@ -11,8 +11,6 @@ struct KGrid {
   int nk() const { return n0 * n1 * n2; }
 };
 
-void upload_twiddles();
-
 // tau slices of one Pi / Sigma launch, in elements: slice b works on G(tau) at Gp + b sp (Sigma
 // is written beside it with the same stride), G(beta - tau) at Gn + b sn and Pi / W at + b sw;
 // Sigma(beta - tau) is formed for the first n_minus slices.  One launch over a whole tau chunk:

@@ -276,6 +276,29 @@ __global__ void __launch_bounds__(256) k_aux_diag(const double2* __restrict__ T,
   if (lane == 0) rho[Q] = make_double2(scale * sr, scale * si);
 }
 
+// y = A x for a row-major n x n matrix, one warp per row.  (As an n x 1 product on the FP64 GEMM's
+// 128 x 32 tiles this took 83 us at n = 512, four CTAs walking the whole K.)
+__global__ void __launch_bounds__(256) k_matvec(const double2* __restrict__ A,
+                                                const double2* __restrict__ x,
+                                                double2* __restrict__ y, int64_t n) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + threadIdx.x / 32;
+  const int lane = threadIdx.x & 31;
+  if (r >= n) return;
+  const double2* a = A + r * n;
+  double sr = 0, si = 0;
+#pragma unroll 4
+  for (int64_t j = lane; j < n; j += 32) {
+    const double2 u = a[j], v = x[j];
+    sr = fma(u.x, v.x, fma(-u.y, v.y, sr));
+    si = fma(u.x, v.y, fma(u.y, v.x, si));
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    sr += __shfl_down_sync(0xffffffffu, sr, o);
+    si += __shfl_down_sync(0xffffffffu, si, o);
+  }
+  if (lane == 0) y[r] = make_double2(sr, si);
+}
+
 // Y[k, P, b] = d[P] X[k, P, b]
 __global__ void k_scale_rows(const double2* __restrict__ X, const double2* __restrict__ d,
                              double2* __restrict__ Y, int64_t nk, int64_t Np, int64_t nb) {
@@ -307,6 +330,12 @@ void scale_slices(double2* A, const double* f, int64_t nslice, int64_t per, cuda
 void aux_diag(const double2* T, const double2* X, double2* rho, int64_t nk, int64_t Np,
               int64_t nb, double scale, cudaStream_t s) {
   k_aux_diag<<<(unsigned)((Np + 7) / 8), 256, 0, s>>>(T, X, rho, nk, Np, nb, scale);
+  count_launch();
+  CQ_CHECK_CUDA(cudaGetLastError());
+}
+
+void matvec(const double2* A, const double2* x, double2* y, int64_t n, cudaStream_t s) {
+  k_matvec<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, x, y, n);
   count_launch();
   CQ_CHECK_CUDA(cudaGetLastError());
 }

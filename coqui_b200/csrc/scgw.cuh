@@ -47,6 +47,8 @@ void add_diag(double2* A, const double2* d, int64_t nb, int64_t nmat, cudaStream
 // for T = X Dm per k (the diagonal of X Dm X^H summed over k), and Y[k,P,b] = d[P] X[k,P,b].
 void aux_diag(const double2* T, const double2* X, double2* rho, int64_t nk, int64_t Np,
               int64_t nb, double scale, cudaStream_t s);
+// y = A x, A a row-major n x n complex128 matrix
+void matvec(const double2* A, const double2* x, double2* y, int64_t n, cudaStream_t s);
 void scale_rows(const double2* X, const double2* d, double2* Y, int64_t nk, int64_t Np,
                 int64_t nb, cudaStream_t s);
 
