@@ -276,6 +276,12 @@ template <typename F> __device__ __forceinline__ void with_n(int n, F&& f) {
   }
 }
 
+// The same with the length known at compile time when N0 > 0 (n is then N0).
+template <int N0, typename F> __device__ __forceinline__ void with_n0(int n, F&& f) {
+  if constexpr (N0 > 0) f(std::integral_constant<int, N0>{});
+  else with_n(n, f);
+}
+
 // One in-shared-memory DFT dimension (the middle one, stride n2) of a tile.
 template <typename C, int TILE, int NC>
 __device__ __forceinline__ void mid_pass(C* A, int n1, int n2, int nk, int sign) {
@@ -597,11 +603,19 @@ __global__ void __launch_bounds__(NC * TILE) k_dft_plane(cplx_t<R>* __restrict__
   }
 }
 
+// The outermost dimension holds up to three operands of n0 values per thread; with n0 only known
+// at run time the kernels carried the registers of its largest value (144 in complex64: one
+// block of eight warps per SM), so n0 is a template argument on grids that are not cubic: Sigma of
+// a 5 x 3 x 2 grid at N_mu 203 1.18 -> 0.49 ms, Pi 0.47 -> 0.35 ms (24 tau slices).
+template <typename R, int N0> constexpr int fused_blocks() {
+  return N0 == 0 ? 1 : sizeof(R) == 4 ? (N0 <= 4 ? 4 : N0 <= 6 ? 3 : 2) : (N0 <= 4 ? 2 : 1);
+}
+
 // Pi(t) columns: Pi = f_qR[ scale Gp(R) o conj(Gn(R)) ] with G(R) = f_Rk G(k), four shared-
 // memory sweeps per tile (load + innermost DFT, middle DFT, outermost DFT + product + inverse,
 // middle inverse, innermost inverse + store).
-template <typename R, int TILE, int NC>
-__global__ void __launch_bounds__(256) k_pi_fused(const cplx_t<R>* __restrict__ Gp,
+template <typename R, int TILE, int NC, int N0>
+__global__ void __launch_bounds__(256, (fused_blocks<R, N0>())) k_pi_fused(const cplx_t<R>* __restrict__ Gp,
                                                   const cplx_t<R>* __restrict__ Gn,
                                                   cplx_t<R>* __restrict__ Pi, int64_t ncol,
                                                   int rn0, int rn1, int rn2, R scale,
@@ -623,8 +637,8 @@ __global__ void __launch_bounds__(256) k_pi_fused(const cplx_t<R>* __restrict__ 
     mid_pass<C, TILE, NC>(A, n1, n2, nk, -1);
     mid_pass<C, TILE, NC>(B, n1, n2, nk, -1);
     __syncthreads();
-    with_n(n0, [&](auto N0) {
-      constexpr int N = decltype(N0)::value;
+    with_n0<N0>(n0, [&](auto NN) {
+      constexpr int N = decltype(NN)::value;
       outer_pointwise<C, TILE, N>(A, B, false, n1 * n2, [](C (&)[N], int, int) {},
                                   [&](C (&a)[N], C (&b)[N], C (&)[N]) {
 #pragma unroll
@@ -643,8 +657,8 @@ __global__ void __launch_bounds__(256) k_pi_fused(const cplx_t<R>* __restrict__ 
 
 // Sigma(t) columns (both halves): S = f_kR[ -(f_Rk G) o W_R ] (scale = -1/nk), W_R read from
 // global memory inside the outermost-dimension sweep.  In place (S may alias G).
-template <typename R, int TILE, int NC>
-__global__ void __launch_bounds__(256) k_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm,
+template <typename R, int TILE, int NC, int N0>
+__global__ void __launch_bounds__(256, (fused_blocks<R, N0>())) k_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm,
                                                      const cplx_t<R>* __restrict__ WR,
                                                      cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol,
                                                      int rn0, int rn1, int rn2, R scale,
@@ -670,8 +684,8 @@ __global__ void __launch_bounds__(256) k_sigma_fused(const cplx_t<R>* Gp, const 
     if (has_m) mid_pass<C, TILE, NC>(B, n1, n2, nk, -1);
     __syncthreads();
     const int stride = n1 * n2;
-    with_n(n0, [&](auto N0) {
-      constexpr int N = decltype(N0)::value;
+    with_n0<N0>(n0, [&](auto NN) {
+      constexpr int N = decltype(NN)::value;
       outer_pointwise<C, TILE, N>(A, has_m ? B : nullptr, true, stride,
                                   [&](C (&w)[N], int inner, int c) {
         const int64_t col = col0 + c;
@@ -863,6 +877,24 @@ static int cubic_edge(KGrid g) {
   return 0;
 }
 
+// f with the outermost edge as a constant when the grid is not cubic (NC == 0), else with 0
+template <int NC, typename F> static void with_edge(int n0, F&& f) {
+  if constexpr (NC > 0) {
+    f(std::integral_constant<int, 0>{});
+  } else {
+    switch (n0) {
+      case 1: f(std::integral_constant<int, 1>{}); break;
+      case 2: f(std::integral_constant<int, 2>{}); break;
+      case 3: f(std::integral_constant<int, 3>{}); break;
+      case 4: f(std::integral_constant<int, 4>{}); break;
+      case 5: f(std::integral_constant<int, 5>{}); break;
+      case 6: f(std::integral_constant<int, 6>{}); break;
+      case 7: f(std::integral_constant<int, 7>{}); break;
+      default: f(std::integral_constant<int, 8>{}); break;
+    }
+  }
+}
+
 #define CQ_DISPATCH_NC(g, ...)                 \
   switch (cubic_edge(g)) {                     \
     case 1: { constexpr int NCV = 1; __VA_ARGS__; } break; \
@@ -941,9 +973,11 @@ void launch_pi_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gn, cplx_t<R>* Pi, in
     set_smem((const void*)k_pi_plane<R, T, NCV>, smem);                                      \
     k_pi_plane<R, T, NCV><<<grid, 2 * NCV * T, smem, s>>>(Gp, Gn, Pi, ncol, scale, ts);      \
   } else {                                                                                   \
-    set_smem((const void*)k_pi_fused<R, T, NCV>, smem);                                      \
-    k_pi_fused<R, T, NCV><<<grid, 256, smem, s>>>(Gp, Gn, Pi, ncol, g.n0, g.n1, g.n2, scale,  \
-                                                  ts);                                       \
+    with_edge<NCV>(g.n0, [&](auto N0) {                                                       \
+      auto fn = k_pi_fused<R, T, NCV, decltype(N0)::value>;                                   \
+      set_smem((const void*)fn, smem);                                                        \
+      fn<<<grid, 256, smem, s>>>(Gp, Gn, Pi, ncol, g.n0, g.n1, g.n2, scale, ts);              \
+    });                                                                                       \
   })
   if (tile == 32) {
     CQ_PI_LAUNCH(32)
@@ -982,9 +1016,11 @@ void launch_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm, const cplx_t<R
     k_sigma_plane<R, T, NCV><<<grid, 2 * NCV * T, smem3, s>>>(Gp, Gm, WR, Sp, Sm, ncol, scale, \
                                                               ts);                            \
   } else {                                                                                    \
-    set_smem((const void*)k_sigma_fused<R, T, NCV>, smem);                                    \
-    k_sigma_fused<R, T, NCV><<<grid, 256, smem, s>>>(Gp, Gm, WR, Sp, Sm, ncol, g.n0, g.n1,    \
-                                                     g.n2, scale, ts);                        \
+    with_edge<NCV>(g.n0, [&](auto N0) {                                                       \
+      auto fn = k_sigma_fused<R, T, NCV, decltype(N0)::value>;                                \
+      set_smem((const void*)fn, smem);                                                        \
+      fn<<<grid, 256, smem, s>>>(Gp, Gm, WR, Sp, Sm, ncol, g.n0, g.n1, g.n2, scale, ts);      \
+    });                                                                                       \
   })
   if (tile == 32) {
     CQ_SIGMA_LAUNCH(32)
