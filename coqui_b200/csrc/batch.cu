@@ -104,7 +104,7 @@ template <typename F> int bguarded(Batch* b, F&& f) {
     CQ_CHECK_CUDA(cudaSetDevice(b->dev));
     f();
     if (b->st) CQ_CHECK_CUDA(cudaStreamSynchronize(b->st));
-    if (cq::tc_take_error())
+    if (cq::tc_take_flags(cq::kTcTimeout))
       throw cq::Error(COQUI_B200_ETIMEDOUT, "a tensor-core kernel gave up a bounded wait");
     b->err.clear();
     return COQUI_B200_OK;

@@ -118,10 +118,18 @@ struct coqui_b200_ctx {
   int64_t gcache_limit = -1;  // bytes; -1: half the free memory at first use
 
   // Dyson results per (iW, q) problem on the device
-  DevBuf<int> dinfo;
+  // trace, ln det and status of every problem in one block, read back by one copy
+  DevBuf<unsigned char> dres;
+  double2* dtrace = nullptr;
+  double* dlogdet = nullptr;
+  int* dinfo = nullptr;
+  void ensure_results(int64_t n) {
+    dres.ensure((size_t)n * (sizeof(double2) + sizeof(double) + sizeof(int)));
+    dtrace = reinterpret_cast<double2*>(dres.p);
+    dlogdet = reinterpret_cast<double*>(dtrace + n);
+    dinfo = reinterpret_cast<int*>(dlogdet + n);
+  }
   DevBuf<int> flag;  // input checks
-  DevBuf<double> dlogdet;
-  DevBuf<double2> dtrace;
   // CUDA graph of the resident-G GW iteration (captured on the first of consecutive calls)
   bool capturing = false;
   // host buffers baked into the captured graph (nullptr: resident G / Sigma left on the device)
@@ -131,6 +139,8 @@ struct coqui_b200_ctx {
   bool defer_dyson_check = false;
   cudaGraphExec_t gexec = nullptr;
   int64_t calls = 0, graph_call = -2, graph_launches = 0;
+  // last call with a pageable G that ran, or may replay, the GW iteration / the RPA energy
+  int64_t plain_call = -2, rplain_call = -2;
   // the same for the RPA energy (polarizability, tau -> w, factorisations)
   cudaGraphExec_t rexec = nullptr;
   const double* rgraph_g = nullptr;
@@ -246,9 +256,9 @@ template <typename F> int guarded(Ctx* c, F&& f) {
     f();
     if (c->st) CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));
     if (c->cs) CQ_CHECK_CUDA(cudaStreamSynchronize(c->cs));
-    if (cq::tc_take_nonfinite())
-      throw Error(COQUI_B200_EINVAL, "G holds NaN or Inf values");
-    if (cq::tc_take_error())
+    const int flags = cq::tc_take_flags(cq::kTcNonfinite | cq::kTcTimeout);
+    if (flags & cq::kTcNonfinite) throw Error(COQUI_B200_EINVAL, "G holds NaN or Inf values");
+    if (flags & cq::kTcTimeout)
       throw Error(COQUI_B200_ETIMEDOUT, "a tensor-core kernel gave up a bounded wait");
     c->err.clear();
     return COQUI_B200_OK;
@@ -259,7 +269,7 @@ template <typename F> int guarded(Ctx* c, F&& f) {
     // positive pivots, say): report it as such
     bool nonfinite = false;
     try {
-      nonfinite = cq::tc_take_nonfinite() != 0;
+      nonfinite = cq::tc_take_flags(cq::kTcNonfinite) != 0;
     } catch (const Error&) {
     }
     if (nonfinite) {
@@ -1270,12 +1280,10 @@ void dyson_all(Ctx* c, bool want_w, bool want_e, std::vector<double>* logdet,
   a.PW = c->PW.p;
   a.prof = &c->prof;
   const int64_t nprob = c->nwh * c->nq;
-  c->dinfo.ensure(nprob);
-  c->dlogdet.ensure(nprob);
-  c->dtrace.ensure(nprob);
-  a.info = c->dinfo.p;
-  a.logdet = c->dlogdet.p;
-  a.trace = c->dtrace.p;
+  c->ensure_results(nprob);
+  a.info = c->dinfo;
+  a.logdet = c->dlogdet;
+  a.trace = c->dtrace;
   a.defer_check = c->capturing || c->defer_dyson_check;
   a.keep_scratch = c->capturing;
   std::vector<double> ld;
@@ -1660,22 +1668,34 @@ void hf_gygi_device(Ctx* c, const double2* Dm, const double2* S, double madelung
 }
 
 // One GW iteration of the resident G as a CUDA graph (update_w + Sigma, no host transfers).
-// status of every (iW, q) factorisation of the last Dyson step, left on the device
-void check_dyson_status(Ctx* c) {
+// Status of every (iW, q) factorisation of the last Dyson step, left on the device; with ld and
+// tr also the log-determinants and traces, in the same copy.
+void check_dyson_status(Ctx* c, std::vector<double>* ld = nullptr,
+                        std::vector<double2>* tr = nullptr) {
   const int64_t nprob = c->nwh * c->nq;
-  std::vector<int> info(nprob);
-  CQ_CHECK_CUDA(cudaMemcpyAsync(info.data(), c->dinfo.p, nprob * sizeof(int), cudaMemcpyDeviceToHost,
-                                c->st));
+  const size_t head = (size_t)nprob * (sizeof(double2) + sizeof(double)), tail = nprob * sizeof(int);
+  std::vector<unsigned char> h((ld ? head : 0) + tail);
+  CQ_CHECK_CUDA(cudaMemcpyAsync(h.data(), c->dres.p + (ld ? 0 : head), h.size(),
+                                cudaMemcpyDeviceToHost, c->st));
   CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));
+  std::vector<int> info(nprob);
+  std::memcpy(info.data(), h.data() + (ld ? head : 0), tail);
+  if (ld) {
+    tr->resize(nprob);
+    ld->resize(nprob);
+    std::memcpy(tr->data(), h.data(), nprob * sizeof(double2));
+    std::memcpy(ld->data(), h.data() + nprob * sizeof(double2), nprob * sizeof(double));
+  }
   for (int64_t i = 0; i < nprob; ++i)
     CQ_REQUIRE(info[i] == 0, COQUI_B200_ENOTHPD, "I - L^H Pi L is not positive definite");
 }
 
 // G_host / S_host: page-locked host buffers copied in / out inside the graph (chunked on the
 // copy stream as in the directly launched path), or nullptr for the resident G and a Sigma
-// left on the device.  The graph is replayed by the next call with the same buffers.
-void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host) {
-  c->begin_timing();
+// left on the device.  The graph is replayed by the next call with the same buffers.  `timed`:
+// the caller marks the call's phases.
+void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host, bool timed = false) {
+  if (!timed) c->begin_timing();
   const bool replay = c->gexec && c->graph_call == c->calls - 1 && c->graph_g == G_host &&
                       c->graph_s == S_host;
   if (!replay) {
@@ -1713,15 +1733,15 @@ void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host) {
   c->mark("GW_ITERATION_GRAPH");
   c->graph_call = c->calls;
   check_dyson_status(c);  // factorisation status of every (iW, q) problem of this iteration
-  c->end_timing();
+  if (!timed) c->end_timing();
 }
 
 // RPA energy of the resident G (or of a page-locked host G copied inside the graph) as one
 // CUDA graph: polarizability, tau -> w, the factorisations with their log-determinants and
 // traces left on the device; E_c is summed on the host from those afterwards.  Replayed by
 // the next call with the same G argument.
-void rpa_energy_graph(Ctx* c, const double* G_host, double* e_rpa) {
-  c->begin_timing();
+void rpa_energy_graph(Ctx* c, const double* G_host, double* e_rpa, bool timed = false) {
+  if (!timed) c->begin_timing();
   const bool replay = c->rexec && c->rgraph_call == c->calls - 1 && c->rgraph_g == G_host;
   if (!replay) {
     if (c->rexec) {
@@ -1757,19 +1777,13 @@ void rpa_energy_graph(Ctx* c, const double* G_host, double* e_rpa) {
   CQ_CHECK_CUDA(cudaGraphLaunch(c->rexec, c->st));
   c->mark("RPA_GRAPH");
   c->rgraph_call = c->calls;
-  check_dyson_status(c);
-  const int64_t nprob = c->nwh * c->nq;
-  std::vector<double> ld(nprob);
-  std::vector<double2> tr(nprob);
-  CQ_CHECK_CUDA(cudaMemcpyAsync(ld.data(), c->dlogdet.p, nprob * sizeof(double),
-                                cudaMemcpyDeviceToHost, c->st));
-  CQ_CHECK_CUDA(cudaMemcpyAsync(tr.data(), c->dtrace.p, nprob * sizeof(double2),
-                                cudaMemcpyDeviceToHost, c->st));
-  CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));
+  std::vector<double> ld;
+  std::vector<double2> tr;
+  check_dyson_status(c, &ld, &tr);
   for (double v : ld)
     CQ_REQUIRE(std::isfinite(v), COQUI_B200_ENOTHPD, "I - Pi V is not positive definite");
   *e_rpa = rpa_energy_from(c, ld, tr);
-  c->end_timing();
+  if (!timed) c->end_timing();
 }
 }  // namespace
 
@@ -1881,6 +1895,26 @@ int coqui_b200_gw_iteration(coqui_b200_ctx* c, const double* G_tskij, double* Si
       gw_iteration_graph(c, G_tskij, Sigma_tskij);
       return;
     }
+    // A pageable G: the second of consecutive such calls captures the iteration of the resident
+    // G, the following ones replay it between the copies (79 launches of the 8-k, N_mu 128
+    // iteration left the GPU idle for a quarter of its 1.05 ms); the first call runs directly,
+    // since capturing costs more than one call saves.
+    const bool plain = !eps_inv_head && c->mode == COQUI_B200_MIXED && !c->prof.on &&
+                       !div_active(c) && G_tskij && !cq::host_is_pinned(G_tskij);
+    if (plain && c->plain_call == c->calls - 1) {
+      c->plain_call = c->calls;
+      c->begin_timing();
+      upload_G(c, G_tskij);
+      c->mark("h2d_G");
+      gw_iteration_graph(c, nullptr, nullptr, true);
+      if (Sigma_tskij) {
+        download(c, Sigma_tskij, c->Sig.p, (size_t)c->nt * c->nk * c->nb * c->nb * sizeof(double2));
+        c->mark("d2h_Sigma");
+      }
+      c->end_timing();
+      return;
+    }
+    if (plain) c->plain_call = c->calls;
     c->begin_timing();
     upload_G(c, G_tskij);
     c->mark("h2d_G");
@@ -1983,6 +2017,18 @@ int coqui_b200_rpa_energy(coqui_b200_ctx* c, const double* G_tskij, double* e_rp
       rpa_energy_graph(c, G_tskij, e_rpa);
       return;
     }
+    // a pageable G, as in coqui_b200_gw_iteration
+    const bool plain = c->mode == COQUI_B200_MIXED && !c->prof.on && G_tskij;
+    if (plain && c->rplain_call == c->calls - 1) {
+      c->rplain_call = c->calls;
+      c->begin_timing();
+      upload_G(c, G_tskij);
+      c->mark("h2d_G");
+      rpa_energy_graph(c, nullptr, e_rpa, true);
+      c->end_timing();
+      return;
+    }
+    if (plain) c->rplain_call = c->calls;
     c->begin_timing();
     upload_G(c, G_tskij);
     c->mark("h2d_G");

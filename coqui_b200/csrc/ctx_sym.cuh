@@ -143,12 +143,10 @@ void sym_dyson(Ctx* c, bool want_w, bool want_e, std::vector<double>* ld,
   a.PW = S.PWi.p;
   a.prof = &c->prof;
   const int64_t nprob = c->nwh * S.nq_ibz;
-  c->dinfo.ensure(nprob);
-  c->dlogdet.ensure(nprob);
-  c->dtrace.ensure(nprob);
-  a.info = c->dinfo.p;
-  a.logdet = c->dlogdet.p;
-  a.trace = c->dtrace.p;
+  c->ensure_results(nprob);
+  a.info = c->dinfo;
+  a.logdet = c->dlogdet;
+  a.trace = c->dtrace;
   cq::dyson_run(a, c->dyn, c->st, ld, tr);
 }
 

@@ -229,13 +229,18 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
   // Chunks of the flattened (w, q) problem list (per-q operands addressed periodically), as
   // many problems per chunk as ~60% of the free device memory allows, so the factorisation
   // kernel sees whole waves of problems (one CTA per problem)
-  size_t fr = 0, tot = 0;
-  CQ_CHECK_CUDA(cudaMemGetInfo(&fr, &tot));
-  size_t budget = std::max(scratch.n, (size_t)(kScratchShare * (double)(fr + scratch.n)));
+  // (the free memory is not asked for once the scratch holds every problem: the query takes
+  // 0.1 ms and more on a machine whose other GPUs are busy)
+  const int64_t nprob = nw * nq;
+  size_t budget = scratch.n;
+  if (scratch.n < per * (size_t)nprob + 1024) {
+    size_t fr = 0, tot = 0;
+    CQ_CHECK_CUDA(cudaMemGetInfo(&fr, &tot));
+    budget = std::max(scratch.n, (size_t)(kScratchShare * (double)(fr + scratch.n)));
+  }
   // while a graph is captured the scratch keeps its size (no device allocation or free inside
   // the capture) when it holds at least one problem
   if (a.keep_scratch && scratch.n >= per + 1024) budget = scratch.n - 1024;
-  const int64_t nprob = nw * nq;
   int64_t nbq = std::max<int64_t>(1, std::min<int64_t>(nprob, (int64_t)(budget / per)));
   if (nbq < nprob) {
     // several chunks: whole waves of the one-CTA factorisation per chunk (a chunk of 1.5 waves

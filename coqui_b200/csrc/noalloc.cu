@@ -158,7 +158,7 @@ extern "C" COQUI_B200_API int coqui_b200_primary_to_aux_noalloc(
     tc_cgemm_nt(T, false, false, nb, Np * nb, Xs, true, true, nb, Np * nb, out, Np, Np * Np, Np,
                 Np, nb, nk, s);
     CQ_CHECK_CUDA(cudaStreamSynchronize(s));
-    if (tc_take_error()) {
+    if (tc_take_flags(kTcTimeout)) {
       set_msg(errbuf, errlen, "a tensor-core kernel gave up a bounded wait");
       return COQUI_B200_ETIMEDOUT;
     }

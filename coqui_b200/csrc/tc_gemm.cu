@@ -33,10 +33,10 @@ namespace cq {
 
 namespace {
 
-__device__ int g_tc_error = 0;
-// set when an input of the primary -> auxiliary projection holds NaN or Inf (the split-TF32
-// products do not carry non-finite values through reliably, so they are caught on the way in)
-__device__ int g_nonfinite = 0;
+// what the kernels report to the host, one copy for both: [0] a bounded wait was given up; [1] an
+// input of the primary -> auxiliary projection holds NaN or Inf (the split-TF32 products do not
+// carry non-finite values through reliably, so they are caught on the way in)
+__device__ int g_flags[2] = {0, 0};
 // time limit of every bounded wait (ns); 2 s unless a test shortens it
 constexpr unsigned long long kDefaultWaitNs = 2000000000ull;
 __device__ unsigned long long g_tc_wait_ns = kDefaultWaitNs;
@@ -149,7 +149,7 @@ __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, uin
     for (uint32_t i = 1;; ++i) {
       if (mbar_try(bar, parity)) return true;
       if ((i & 15u) == 0 && global_ns() - t0 > limit) {
-        atomicExch(&g_tc_error, 1);
+        atomicExch(&g_flags[0], 1);
         return false;
       }
     }
@@ -160,7 +160,7 @@ __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, uin
   for (;;) {
     if (mbar_try_hint(bar, parity, hint)) return true;
     if (global_ns() - t0 > limit) {
-      atomicExch(&g_tc_error, 1);
+      atomicExch(&g_flags[0], 1);
       return false;
     }
   }
@@ -1135,23 +1135,22 @@ void tc_cgemm_nt(const void* A, bool a_split, bool conj_a, int64_t lda, int64_t 
   else dispatch_n<false, false>(p, batch, s);
 }
 
-int tc_take_nonfinite() {
-  int h = 0, z = 0;
-  CQ_CHECK_CUDA(cudaMemcpyFromSymbol(&h, g_nonfinite, sizeof(int)));
-  if (h) CQ_CHECK_CUDA(cudaMemcpyToSymbol(g_nonfinite, &z, sizeof(int)));
-  return h;
-}
-
 void tc_set_wait_ns(int64_t ns) {
   const unsigned long long v = ns > 0 ? (unsigned long long)ns : kDefaultWaitNs;
   CQ_CHECK_CUDA(cudaMemcpyToSymbol(g_tc_wait_ns, &v, sizeof(v)));
 }
 
-int tc_take_error() {
-  int h = 0, z = 0;
-  CQ_CHECK_CUDA(cudaMemcpyFromSymbol(&h, g_tc_error, sizeof(int)));
-  if (h) CQ_CHECK_CUDA(cudaMemcpyToSymbol(g_tc_error, &z, sizeof(int)));
-  return h;
+int tc_take_flags(int mask) {
+  int h[2] = {0, 0};
+  const int z = 0, bit[2] = {kTcTimeout, kTcNonfinite};
+  CQ_CHECK_CUDA(cudaMemcpyFromSymbol(h, g_flags, sizeof(h)));
+  int got = 0;
+  for (int i = 0; i < 2; ++i)
+    if (h[i] && (mask & bit[i])) {
+      CQ_CHECK_CUDA(cudaMemcpyToSymbol(g_flags, &z, sizeof(int), i * sizeof(int)));
+      got |= bit[i];
+    }
+  return got;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1199,7 +1198,7 @@ __global__ void k_transpose_c64(const double2* __restrict__ in, float2* __restri
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = i / (rows * cols), e = i % (rows * cols);
     const double2 x = in[i];
-    if (!isfinite(x.x) || !isfinite(x.y)) atomicExch(&g_nonfinite, 1);
+    if (!isfinite(x.x) || !isfinite(x.y)) atomicExch(&g_flags[1], 1);
     out[b * rows * cols + (e % cols) * rows + e / cols] = make_float2((float)x.x, (float)x.y);
   }
 }

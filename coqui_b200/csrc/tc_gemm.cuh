@@ -96,12 +96,10 @@ int64_t tc_tuned_shapes();
 bool tc_set_forced_cfg(int cfg);
 int tc_num_cfgs();
 
-// Returns (and clears) the device flag set when a bounded wait inside a tensor-core kernel
-// gave up (nonzero = a kernel timed out).
-int tc_take_error();
-// Whether a primary -> auxiliary projection since the last call saw NaN or Inf in G (read and
-// cleared).
-int tc_take_nonfinite();
+// What tensor-core kernels reported since the last call, of the kinds in `mask`, read and cleared:
+// a bounded wait was given up; a primary -> auxiliary projection saw NaN or Inf in G.
+constexpr int kTcTimeout = 1, kTcNonfinite = 2;
+int tc_take_flags(int mask);
 // Time limit of the tensor-core kernels' bounded waits on the current device (ns; <= 0: the
 // default 2 s).
 void tc_set_wait_ns(int64_t ns);

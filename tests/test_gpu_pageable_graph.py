@@ -1,0 +1,54 @@
+"""Consecutive calls with ordinary numpy arrays run directly, then capture, then replay the GW
+iteration and the RPA energy of the resident G.  Every call of such a run gives what a fresh
+context gives for its own inputs, also when the inputs, the THC data or the entry point change in
+between, and non-finite inputs are refused on a replayed call too."""
+import numpy as np
+import pytest
+
+from coqui_b200 import capi
+from coqui_b200.iaft import IAFT
+from coqui_b200.synthetic import make_system
+
+pytestmark = pytest.mark.gpu
+
+FT = IAFT(1000.0, 10.0, "low")
+
+
+def context(s):
+    c = capi.Context(s.nk, s.nb, s.Np, FT.nt_f, FT.nw_b, s.kp_grid, mode=capi.MIXED)
+    c.set_ir(FT)
+    c.set_kmesh(s.kpts, s.lattv, s.chi_bar)
+    c.set_thc(s.X, s.V)
+    return c
+
+
+@pytest.mark.parametrize("grid,Np", [((1, 1, 1), 40), ((2, 2, 2), 130), ((3, 2, 1), 33)])
+def test_replayed_calls_match_fresh_contexts(grid, Np):
+    s, s2 = (make_system(grid, 7, 3, Np, seed=i) for i in (1, 2))
+    Gs = [s.G0(FT), s2.G0(FT)]
+    sigma, energy = {}, {}
+    for t, sys in enumerate((s, s2)):
+        for i, G in enumerate(Gs):
+            c = context(sys)
+            sigma[t, i] = c.gw_iteration(G)[0]
+            c.close()
+            c = context(sys)
+            energy[t, i] = c.rpa_energy(G)
+            c.close()
+    c = context(s)
+    for i in (0, 1, 0, 1, 1):
+        assert np.array_equal(c.gw_iteration(Gs[i])[0], sigma[0, i])
+    for i in (1, 0, 0, 1):
+        assert c.rpa_energy(Gs[i]) == energy[0, i]
+    c.set_thc(s2.X, s2.V)
+    for i in (0, 1, 0):
+        assert np.array_equal(c.gw_iteration(Gs[i])[0], sigma[1, i])
+    bad = Gs[0].copy()
+    bad[3, 0, 0, 1, 1] = np.nan
+    with pytest.raises(capi.CoquiB200Error) as e:
+        c.gw_iteration(bad)
+    assert e.value.code == -1
+    for i in (1, 0, 1):
+        assert np.array_equal(c.gw_iteration(Gs[i])[0], sigma[1, i])
+        assert c.rpa_energy(Gs[i]) == energy[1, i]
+    c.close()
