@@ -63,6 +63,7 @@ struct SymState {
   cq::TcOperand Xtc;              // mixed form: Xs packed for the tensor-core projection
   DevBuf<double2> Li, LHi, Vi;    // (nq_ibz, Np, Np) at the IBZ q-points
   DevBuf<float2> Lci, LHci;
+  cq::TcFactor Lpi, LHpi;
   DevBuf<double2> Gi;             // (nt, nk_ibz, nb, nb) G on the IBZ k-points
   DevBuf<unsigned char> PWi;      // (nmax, nq_ibz, Np, Np) Pi / W on the IBZ q-points
   DevBuf<unsigned char> Sq;       // (nsym, nk_ibz, Np, Np) Sigma_PQ rows of one tau
@@ -104,7 +105,9 @@ struct coqui_b200_ctx {
   DevBuf<double2> eps;
   DevBuf<unsigned char> Gp, Gn, PW;  // storage precision, bytes
   DevBuf<unsigned char> dyn;         // Dyson scratch
-  DevBuf<float2> Lc, LHc;            // complex64 L, L^H for the tensor-core Dyson products
+  // L, L^H for the tensor-core Dyson products: packed above one inverse group, else complex64
+  DevBuf<float2> Lc, LHc;
+  cq::TcFactor Lp, LHp;
   cq::TcOperand Xtc;                 // packed X for the tensor-core projections
   DevBuf<double2> Gx;                // primary_to_aux staging (the resident G stays intact)
 
@@ -998,6 +1001,8 @@ void coqui_b200_destroy(coqui_b200_ctx* c) {
   c->dyn.release();
   c->Lc.release();
   c->LHc.release();
+  c->Lp.release();
+  c->LHp.release();
   c->Xtc.release();
   for (auto& m : c->marks) cudaEventDestroy(m.second);
   if (c->st) cudaStreamDestroy(c->st);
@@ -1162,10 +1167,15 @@ int coqui_b200_set_thc(coqui_b200_ctx* c, const double* X_skPa, const double* V_
     cq::launch_zero_upper_and_adjoint(c->L.p, c->LH.p, Np, nk, c->st);
     if (c->mode == COQUI_B200_MIXED) {
       cq::tc_pack_X(c->Xtc, c->X.p, nk, Np, nb, c->st);
-      c->Lc.ensure((size_t)nk * Np * Np);
-      c->LHc.ensure((size_t)nk * Np * Np);
-      cq::to_c64(c->L.p, c->Lc.p, Np, Np, nk, false, c->st);
-      cq::to_c64(c->LH.p, c->LHc.p, Np, Np, nk, false, c->st);
+      if (Np > cq::kInvGroup) {
+        cq::tc_pack_factor(c->Lp, c->L.p, Np, nk, c->st);
+        cq::tc_pack_factor(c->LHp, c->LH.p, Np, nk, c->st);
+      } else {
+        c->Lc.ensure((size_t)nk * Np * Np);
+        c->LHc.ensure((size_t)nk * Np * Np);
+        cq::to_c64(c->L.p, c->Lc.p, Np, Np, nk, false, c->st);
+        cq::to_c64(c->LH.p, c->LHc.p, Np, Np, nk, false, c->st);
+      }
     }
     CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));
     c->have_thc = true;
@@ -1272,6 +1282,8 @@ void dyson_all(Ctx* c, bool want_w, bool want_e, std::vector<double>* logdet,
   a.L = c->L.p;
   a.LH = c->LH.p;
   a.V = c->V.p;
+  a.Lp = c->Lp.view();
+  a.LHp = c->LHp.view();
   a.Lc = c->Lc.p;
   a.LHc = c->LHc.p;
   a.want_w = want_w;

@@ -71,7 +71,15 @@ void sym_prepare_thc(Ctx* c) {
   S.LHi.ensure((size_t)nqi * pp);
   S.Vi.ensure((size_t)nqi * pp);
   const bool mixed = (c->mode == COQUI_B200_MIXED);
-  if (mixed) {
+  const bool packed = mixed && Np > cq::kInvGroup;
+  if (packed) {
+    for (auto f : {std::make_pair(&S.Lpi, &c->Lp), std::make_pair(&S.LHpi, &c->LHp)}) {
+      f.first->n = f.second->n;
+      f.first->stride = f.second->stride;
+      f.first->packed.ensure((size_t)nqi * f.second->stride);
+      f.first->inv.ensure(nqi);
+    }
+  } else if (mixed) {
     S.Lci.ensure((size_t)nqi * pp);
     S.LHci.ensure((size_t)nqi * pp);
   }
@@ -81,7 +89,15 @@ void sym_prepare_thc(Ctx* c) {
     CQ_CHECK_CUDA(cudaMemcpyAsync(S.Li.p + i * pp, c->L.p + q * pp, b, cudaMemcpyDeviceToDevice, c->st));
     CQ_CHECK_CUDA(cudaMemcpyAsync(S.LHi.p + i * pp, c->LH.p + q * pp, b, cudaMemcpyDeviceToDevice, c->st));
     CQ_CHECK_CUDA(cudaMemcpyAsync(S.Vi.p + i * pp, c->V.p + q * pp, b, cudaMemcpyDeviceToDevice, c->st));
-    if (mixed) {
+    if (packed) {
+      for (auto f : {std::make_pair(&S.Lpi, &c->Lp), std::make_pair(&S.LHpi, &c->LHp)}) {
+        const int64_t st = f.first->stride;
+        CQ_CHECK_CUDA(cudaMemcpyAsync(f.first->packed.p + i * st, f.second->packed.p + q * st, st,
+                                      cudaMemcpyDeviceToDevice, c->st));
+        CQ_CHECK_CUDA(cudaMemcpyAsync(f.first->inv.p + i, f.second->inv.p + q, sizeof(float),
+                                      cudaMemcpyDeviceToDevice, c->st));
+      }
+    } else if (mixed) {
       const size_t bc = pp * sizeof(float2);
       CQ_CHECK_CUDA(cudaMemcpyAsync(S.Lci.p + i * pp, c->Lc.p + q * pp, bc, cudaMemcpyDeviceToDevice, c->st));
       CQ_CHECK_CUDA(cudaMemcpyAsync(S.LHci.p + i * pp, c->LHc.p + q * pp, bc, cudaMemcpyDeviceToDevice, c->st));
@@ -135,6 +151,8 @@ void sym_dyson(Ctx* c, bool want_w, bool want_e, std::vector<double>* ld,
   a.L = S.Li.p;
   a.LH = S.LHi.p;
   a.V = S.Vi.p;
+  a.Lp = S.Lpi.view();
+  a.LHp = S.LHpi.view();
   a.Lc = S.Lci.p;
   a.LHc = S.LHci.p;
   a.want_w = want_w;

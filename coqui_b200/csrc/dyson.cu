@@ -39,39 +39,45 @@ __global__ void __launch_bounds__(256) k_herm_sum(const float2* __restrict__ DH,
   herm_sum_pair(DH + off, F + off, E + off, Np, I, J);
 }
 
-// Hermitian completion: A[i][j] = conj(A[j][i]) for j > i (32 x 32 tiles on or above the
-// diagonal, the lower tile read through shared memory); complex64 or complex128
-template <typename C>
-__global__ void k_mirror_upper(C* __restrict__ A, int64_t n, int64_t stride) {
+// Hermitian completion: A[i][j] = conj(A[j][i]) for j > i (LOWER: for j < i), one 32 x 32 tile
+// read through shared memory per block; complex64 or complex128
+template <typename C, bool LOWER>
+__global__ void k_mirror(C* __restrict__ A, int64_t n, int64_t stride) {
   __shared__ C tile[32][33];
-  const int64_t i0 = (int64_t)blockIdx.y * 32, j0 = (int64_t)blockIdx.x * 32;
-  if (j0 < i0) return;
+  const int64_t i0 = (int64_t)blockIdx.y * 32, j0 = (int64_t)blockIdx.x * 32;  // tile written
+  if (LOWER ? j0 > i0 : j0 < i0) return;
   C* a = A + (int64_t)blockIdx.z * stride;
-  for (int ty = threadIdx.y; ty < 32; ty += blockDim.y) {  // lower tile (j0.., i0..)
+  for (int ty = threadIdx.y; ty < 32; ty += blockDim.y) {  // the transposed tile (j0.., i0..)
     const int64_t r = j0 + ty, c = i0 + threadIdx.x;
     tile[ty][threadIdx.x] = (r < n && c < n) ? a[r * n + c] : mk<C>(0.0, 0.0);
   }
   __syncthreads();
   for (int ty = threadIdx.y; ty < 32; ty += blockDim.y) {
     const int64_t i = i0 + ty, j = j0 + threadIdx.x;
-    if (i < n && j < n && j > i) {
+    if (i < n && j < n && (LOWER ? j < i : j > i)) {
       const C v = tile[threadIdx.x][ty];  // A[j][i]
       a[i * n + j] = mk<C>(v.x, -v.y);
     }
   }
 }
 
-template <typename C>
-void mirror_upper(C* A, int64_t n, int64_t nbatch, cudaStream_t s, int64_t stride) {
-  CQ_REQUIRE(nbatch <= 65535, COQUI_B200_EINVAL, "mirror: too many problems per launch");
+template <typename C, bool LOWER = false>
+void mirror(C* A, int64_t n, int64_t nbatch, cudaStream_t s, int64_t stride) {
   const unsigned t = (unsigned)((n + 31) / 32);
-  k_mirror_upper<C><<<dim3(t, t, (unsigned)nbatch), dim3(32, 8), 0, s>>>(A, n, stride > 0 ? stride : n * n);
-  count_launch();
-  CQ_CHECK_CUDA(cudaGetLastError());
+  stride = stride > 0 ? stride : n * n;
+  for (int64_t b0 = 0; b0 < nbatch; b0 += 65535) {
+    const unsigned nb = (unsigned)std::min<int64_t>(65535, nbatch - b0);
+    k_mirror<C, LOWER><<<dim3(t, t, nb), dim3(32, 8), 0, s>>>(A + b0 * stride, n, stride);
+    count_launch();
+    CQ_CHECK_CUDA(cudaGetLastError());
+  }
 }
 
 void launch_mirror_upper(float2* A, int64_t n, int64_t nbatch, cudaStream_t s, int64_t stride) {
-  mirror_upper<float2>(A, n, nbatch, s, stride);
+  mirror<float2>(A, n, nbatch, s, stride);
+}
+void launch_mirror_lower(float2* A, int64_t n, int64_t nbatch, cudaStream_t s, int64_t stride) {
+  mirror<float2, true>(A, n, nbatch, s, stride);
 }
 
 // FP64 form: E = Z + Z^H + F (Hermitian, written whole) with Z = D^H upper triangular and F
@@ -209,14 +215,15 @@ size_t dyson_bytes_per_problem(int64_t Np, bool mixed, bool want_w) {
   const size_t NN = (size_t)Np * Np, es = mixed ? sizeof(float2) : sizeof(double2);
   return NN * (es + (m_in_pi(Np, mixed, want_w) ? 0 : es) + sizeof(double2) +
                (mixed && want_w ? sizeof(double2) : 0)) +
-         64;
+         (size_t)2 * Np * sizeof(uint32_t) + 64;
 }
 constexpr double kScratchShare = 0.6;  // of the free device memory, per chunk
+constexpr size_t kScratchSlack = 2048;  // the carved arrays start 256 bytes aligned
 }  // namespace
 
 size_t dyson_reserve_bytes(int64_t Np, int64_t nprob, bool mixed) {
   const int64_t n = std::min<int64_t>(nprob, 2 * chol_wave_size());
-  return (size_t)((double)(dyson_bytes_per_problem(Np, mixed, true) * (size_t)n + 1024) /
+  return (size_t)((double)(dyson_bytes_per_problem(Np, mixed, true) * (size_t)n + kScratchSlack) /
                   kScratchShare);
 }
 
@@ -233,14 +240,14 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
   // 0.1 ms and more on a machine whose other GPUs are busy)
   const int64_t nprob = nw * nq;
   size_t budget = scratch.n;
-  if (scratch.n < per * (size_t)nprob + 1024) {
+  if (scratch.n < per * (size_t)nprob + kScratchSlack) {
     size_t fr = 0, tot = 0;
     CQ_CHECK_CUDA(cudaMemGetInfo(&fr, &tot));
     budget = std::max(scratch.n, (size_t)(kScratchShare * (double)(fr + scratch.n)));
   }
   // while a graph is captured the scratch keeps its size (no device allocation or free inside
   // the capture) when it holds at least one problem
-  if (a.keep_scratch && scratch.n >= per + 1024) budget = scratch.n - 1024;
+  if (a.keep_scratch && scratch.n >= per + kScratchSlack) budget = scratch.n - kScratchSlack;
   int64_t nbq = std::max<int64_t>(1, std::min<int64_t>(nprob, (int64_t)(budget / per)));
   if (nbq < nprob) {
     // several chunks: whole waves of the one-CTA factorisation per chunk (a chunk of 1.5 waves
@@ -248,7 +255,7 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
     const int64_t wave = chol_wave_size();
     if (nbq >= wave) nbq = nbq / wave * wave;
   }
-  scratch.ensure(per * nbq + 1024);
+  scratch.ensure(per * nbq + kScratchSlack);
   unsigned char* base = scratch.p;
   auto carve = [&](size_t bytes) {
     unsigned char* p = base;
@@ -259,6 +266,11 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
   unsigned char* Mb0 = mpi ? nullptr : carve(nbq * NN * es);
   double2* A = (double2*)carve(nbq * NN * sizeof(double2));
   double2* Y = a.mixed && a.want_w ? (double2*)carve(nbq * NN * sizeof(double2)) : nullptr;
+  // the long-K products with a factor of V run on packed factors (tc_fac.cuh) above one inverse
+  // group; smaller matrices fill fewer than two of its tiles and keep the autotuned tiles
+  const bool fac = a.mixed && Np > kInvGroup;
+  uint32_t* rm0 = (uint32_t*)carve((size_t)nbq * Np * sizeof(uint32_t));  // row maxima: Pi, then E
+  uint32_t* rm1 = (uint32_t*)carve((size_t)nbq * Np * sizeof(uint32_t));  // P1, then T
   CQ_REQUIRE(a.info && a.logdet && a.trace, COQUI_B200_EINVAL, "dyson_run: result arrays missing");
 
   if (a.want_e) {
@@ -275,7 +287,16 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
     // M = L^H (Pi L)
     {
       Prof::Scope sc(a.prof, "dyson_M_gemm");
-      if (a.mixed) {
+      if (fac) {
+        // P1 = L^H Pi on and above the diagonal (the lower triangle of M = L^H P1^H reads
+        // P1(j, k) at k >= i >= j only), then M's lower triangle; Pi Hermitian
+        tc_row_max((const float2*)Pi, rm0, nb * Np, Np, s);
+        CQ_CHECK_CUDA(cudaMemsetAsync(rm1, 0, (size_t)nb * Np * sizeof(uint32_t), s));
+        tc_factor_product(a.LHp, true, nq, q0, (const float2*)Pi, true, rm0, (float2*)T1, rm1, 1, nb,
+                          s);
+        tc_factor_product(a.LHp, true, nq, q0, (const float2*)T1, true, rm1, (float2*)Mb, nullptr, -1,
+                          nb, s);
+      } else if (a.mixed) {
         // P1 = L^H Pi  (Pi Hermitian: B(k, n) = Pi[k][n] = conj(Pi[n][k]))
         // Only P1's tiles on and above the diagonal are needed: the lower triangle of M reads
         // Q = P1^H at (a, j) with a >= i >= j.  The others are written as zeros, which only
@@ -400,6 +421,18 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
       const int64_t nt32 = (Np + 31) / 32;
       k_herm_sum<<<dim3((unsigned)(nt32 * (nt32 + 1) / 2), (unsigned)nb), 256, 0, s>>>(Z, F, E, Np);
       count_launch();
+      if (fac) {
+        // T = L E on and below the diagonal, then the upper triangle of W from the other side,
+        // W(j, i) = sum_{k <= j} L(j, k) conj(T(i, k)) for i >= j, which reads no other T.
+        // (E's row maxima by a pass of their own: raised by k_herm_sum's tiles with atomics they
+        // cost it 0.8 ms at 4x4x4 / 512, the pass 0.47 ms.)
+        tc_row_max(E, rm0, nb * Np, Np, s);
+        CQ_CHECK_CUDA(cudaMemsetAsync(rm1, 0, (size_t)nb * Np * sizeof(uint32_t), s));
+        tc_factor_product(a.Lp, false, nq, q0, E, true, rm0, F, rm1, -1, nb, s);
+        tc_factor_product(a.Lp, false, nq, q0, F, true, rm1, (float2*)Pi, nullptr, 1, nb, s);
+        launch_mirror_lower((float2*)Pi, Np, nb, s);
+        continue;
+      }
       // W is Hermitian: its lower triangle W_ij (j <= i) = sum_{k <= j} T_ik conj(L_jk) needs
       // T = L E only on and below the diagonal tiles, and the upper triangle is its mirror.
       // T = L E  (E Hermitian: B(k, n) = conj(E[n][k]))
@@ -464,7 +497,7 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
       w.C = (double2*)Pi;
       w.batch = nb;
       zgemm(w, s);
-      mirror_upper<double2>((double2*)Pi, Np, nb, s, 0);
+      mirror<double2>((double2*)Pi, Np, nb, s, 0);
     }
   }
   if (!a.defer_check) {

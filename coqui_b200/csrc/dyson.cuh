@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "tc_gemm.cuh"
 
 namespace cq {
 
@@ -70,6 +71,8 @@ __device__ __forceinline__ void herm_sum_pair(const float2* __restrict__ d,
 // A[i][j] = conj(A[j][i]) for j > i, nbatch n x n complex64 matrices `stride` elements apart
 // (0: n * n).
 void launch_mirror_upper(float2* A, int64_t n, int64_t nbatch, cudaStream_t s, int64_t stride = 0);
+// The same from the upper triangle to the lower one.
+void launch_mirror_lower(float2* A, int64_t n, int64_t nbatch, cudaStream_t s, int64_t stride = 0);
 
 // Zero the strict upper triangle of L and write LH = L^H (row-major), batched.
 void launch_zero_upper_and_adjoint(double2* L, double2* LH, int64_t Np, int64_t nbatch,
@@ -80,7 +83,9 @@ struct DysonArgs {
   const double2* L = nullptr;   // (nq, Np, Np) lower Cholesky factors of V
   const double2* LH = nullptr;  // (nq, Np, Np) L^H
   const double2* V = nullptr;   // (nq, Np, Np)
-  const float2* Lc = nullptr;   // mixed form: L and L^H as complex64 tensor-core operands
+  // mixed form: L and L^H as tensor-core operands, packed (Np > kInvGroup) or complex64
+  TcFactorView Lp, LHp;
+  const float2* Lc = nullptr;
   const float2* LHc = nullptr;
   bool want_w = true, want_e = false, mixed = true;
   unsigned char* PW = nullptr;  // (nw, nq, Np, Np): Pi(iW) in, W(iW) out (if want_w)

@@ -26,6 +26,8 @@
 #include <string>
 #include <type_traits>
 
+#include <cuda_fp16.h>
+
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 
@@ -222,6 +224,9 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
+
+constexpr int kFacN = 128;  // complex columns of a tile of the factor products
+#include "tc_fac.cuh"
 
 // Two consecutive complex values (k, k+1) of one operand row, as loaded from global.
 template <bool C128> struct Pair;
@@ -1151,6 +1156,71 @@ int tc_take_flags(int mask) {
       got |= bit[i];
     }
   return got;
+}
+
+// ---------------------------------------------------------------------------------------
+// factor products (tc_fac.cuh)
+// ---------------------------------------------------------------------------------------
+void tc_pack_factor(TcFactor& f, const double2* L, int64_t n, int64_t nmat, cudaStream_t s) {
+  CQ_REQUIRE(nmat <= 65535, COQUI_B200_EUNSUPPORTED, "tc_pack_factor: too many matrices");
+  f.n = n;
+  f.stride = (n + kBM - 1) / kBM * ((n + kFacKC - 1) / kFacKC) * kFacTile;
+  f.packed.ensure((size_t)nmat * f.stride);
+  f.inv.ensure(nmat);
+  DevBuf<uint32_t> mx;
+  mx.ensure(nmat);
+  CQ_CHECK_CUDA(cudaMemsetAsync(mx.p, 0, nmat * sizeof(uint32_t), s));
+  const unsigned g = grid_for(n * n, 256, 64);
+  k_fac_max<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, n);
+  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, f.packed.p, f.inv.p, n, f.stride);
+  count_launch(2);
+  CQ_CHECK_CUDA(cudaGetLastError());
+  CQ_CHECK_CUDA(cudaStreamSynchronize(s));  // mx is freed on return
+}
+
+void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q0, const float2* Bt,
+                       bool conj_b, const uint32_t* row_max, float2* C, uint32_t* out_max, int half,
+                       int64_t batch, cudaStream_t s) {
+  const int64_t n = f.n;
+  FacParams p;
+  p.A = f.packed;
+  p.sA = f.stride;
+  p.invA = f.inv;
+  p.a_mod = mod;
+  p.B = Bt;
+  p.ldb = p.ldc = n;
+  p.sB = p.sC = n * n;
+  p.n = n;
+  p.conj_b = conj_b;
+  p.upper_a = upper;
+  p.half = half;
+  p.b_al = rows_aligned(Bt, false, n, n * n);
+  static bool attr_set[64] = {};
+  int dev = 0;
+  CQ_CHECK_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !attr_set[dev]) {
+    CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac, cudaFuncAttributeMaxDynamicSharedMemorySize, kFacSmem));
+    if (dev < 64) attr_set[dev] = true;
+  }
+  const unsigned t = (unsigned)((n + kBM - 1) / kBM);
+  for (int64_t b0 = 0; b0 < batch; b0 += 65535) {
+    const int64_t nb = std::min<int64_t>(65535, batch - b0);
+    p.a_q0 = (q0 + b0) % mod;
+    p.B = Bt + b0 * n * n;
+    p.rmB = row_max + b0 * n;
+    p.C = C + b0 * n * n;
+    p.rmC = out_max ? out_max + b0 * n : nullptr;
+    k_tc_fac<<<dim3(t, t, (unsigned)nb), kFacThreads, kFacSmem, s>>>(p);
+    count_launch();
+    CQ_CHECK_CUDA(cudaGetLastError());
+  }
+}
+
+void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s) {
+  CQ_REQUIRE(rows <= (int64_t)8 * 2147483647, COQUI_B200_EUNSUPPORTED, "tc_row_max: too many rows");
+  k_row_max<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(A, rm, rows, n);
+  count_launch();
+  CQ_CHECK_CUDA(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------------------

@@ -69,6 +69,35 @@ void tc_cgemm_nt(const void* A, bool a_split, bool conj_a, int64_t lda, int64_t 
                  int64_t sC, int64_t M, int64_t N, int64_t K, int64_t batch, cudaStream_t s,
                  const TcStructure& st = TcStructure{});
 
+// Triangular n x n factors packed for tc_factor_product (split FP16 tiles, tc_fac.cuh).
+struct TcFactorView {
+  const unsigned char* packed = nullptr;  // matrices `stride` bytes apart
+  const float* inv = nullptr;             // 1 / scale of each
+  int64_t n = 0, stride = 0;
+};
+struct TcFactor {
+  DevBuf<unsigned char> packed;
+  DevBuf<float> inv;
+  int64_t n = 0, stride = 0;
+  TcFactorView view() const { return {packed.p, inv.p, n, stride}; }
+  void release() {
+    packed.release();
+    inv.release();
+  }
+};
+void tc_pack_factor(TcFactor& f, const double2* L, int64_t n, int64_t nmat, cudaStream_t s);
+
+// C[b](m, n) = sum_k A(m, k) opB(Bt[b])(n, k) for b < batch: A the packed factor (q0 + b) % mod,
+// upper (k >= m) or lower (k <= m) triangular; Bt and C row-major n x n complex64, conj_b
+// conjugates Bt.  row_max holds the row maxima of Bt (bits of the largest |re|, |im| as float,
+// (batch, n)); those of C are raised in out_max (may be null).  half < 0: only the 128 x 128 tiles
+// on or below the diagonal are formed and written, half > 0: on or above it.
+void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q0, const float2* Bt,
+                       bool conj_b, const uint32_t* row_max, float2* C, uint32_t* out_max, int half,
+                       int64_t batch, cudaStream_t s);
+// Row maxima of a (rows, n) complex64 array, as tc_factor_product reads them.
+void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s);
+
 // One group of a grouped product: a batched "NT" product as tc_cgemm_nt describes.
 struct TcGroup {
   const void* A = nullptr;
