@@ -12,6 +12,7 @@
 //     group per molecule, batched over tau or iW);
 //   * the FP64 factorisations of all (m, iW) problems are one grouped launch.
 #include <algorithm>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -80,6 +81,13 @@ struct coqui_b200_batch {
   std::vector<double2> Twt_pos, Ttw_pos;
   DevBuf<double> dTwtR, dTtwR;
   DevBuf<float2> Xs, XTs, Ls, LHs;  // complex64 tensor-core operands
+  // L, L^H packed for the factor products (molecules above one inverse group; the others use
+  // Ls, LHs), and the row maxima those products read: Pi then E, P1 then T
+  std::vector<std::unique_ptr<cq::TcFactor>> Lp, LHp;
+  DevBuf<uint32_t> rm0, rm1;
+  std::vector<int64_t> offR;
+  int64_t nR = 0;
+  bool fac(int64_t m) const { return Np[m] > cq::kInvGroup; }
   DevBuf<double2> G, Sig, Ltmp, LHtmp;
   DevBuf<float2> Gt, T, UT, Sab, cache, PW;
   DevBuf<float2> T1, Mb, Zb, Zl;
@@ -179,8 +187,35 @@ void batch_gw(Batch* b) {
   cq::launch_ir_transform_real<float>(b->PW.p, cols, (int)nth, (int)nwh, b->dTwtR.p, s);
   // ---- Dyson per (m, iW): M = L^H Pi L, I - M = C C^H, W = L (D + D^H + D^H D) L^H ----
   std::vector<cq::TcGroup> p1, p2;
+  std::vector<cq::TcFactorGroup> f1, f2;
+  std::vector<cq::TcRowMaxGroup> r1;
+  auto factor_group = [&](const cq::TcFactor& f, bool upper, const float2* Bt, int64_t sB,
+                          const uint32_t* rm, float2* C, int64_t sC, uint32_t* out_max, int half) {
+    cq::TcFactorGroup g;
+    g.f = f.view();
+    g.upper = upper;
+    g.conj_b = true;
+    g.Bt = Bt;
+    g.sB = sB;
+    g.row_max = rm;
+    g.C = C;
+    g.sC = sC;
+    g.out_max = out_max;
+    g.half = half;
+    g.batch = nwh;
+    return g;
+  };
+  CQ_CHECK_CUDA(cudaMemsetAsync(b->rm1.p, 0, b->nR * sizeof(uint32_t), s));
   for (int64_t m = 0; m < b->nmol; ++m) {
     const int64_t Np = b->Np[m], NN = Np * Np;
+    if (b->fac(m)) {
+      float2 *T1 = b->T1.p + b->offD[m], *Pi = b->PW.p + b->offPQ[m];
+      uint32_t *m0 = b->rm0.p + b->offR[m], *m1 = b->rm1.p + b->offR[m];
+      r1.push_back(cq::TcRowMaxGroup{Pi, Np, cols, nwh, m0, 0});
+      f1.push_back(factor_group(*b->LHp[m], true, Pi, cols, m0, T1, NN, m1, 1));
+      f2.push_back(factor_group(*b->LHp[m], true, T1, NN, m1, b->Mb.p + b->offD[m], NN, nullptr, -1));
+      continue;
+    }
     cq::TcStructure s1;
     s1.a_upper = true;
     s1.upper_zero = true;  // M's lower triangle reads P1 on and above the diagonal only
@@ -194,6 +229,9 @@ void batch_gw(Batch* b) {
   }
   cq::tc_cgemm_grouped(p1, b->gtab, s);
   cq::tc_cgemm_grouped(p2, b->gtab, s);
+  cq::tc_row_max_grouped(r1, b->gtab, s);
+  cq::tc_factor_grouped(f1, b->gtab, s);
+  cq::tc_factor_grouped(f2, b->gtab, s);
   std::vector<cq::CholProblem> cp;
   for (int64_t m = 0; m < b->nmol; ++m)
     for (int64_t w = 0; w < nwh; ++w) {
@@ -295,6 +333,8 @@ void batch_gw(Batch* b) {
                                a.r1, bl, a.b1, nwh, s);
   }
   std::vector<cq::TcGroup> f, t4, t5;
+  std::vector<cq::TcFactorGroup> f4, f5;
+  std::vector<cq::TcRowMaxGroup> r4;
   std::vector<cq::HermProblem> hp;
   for (int64_t m = 0; m < b->nmol; ++m) {
     const int64_t Np = b->Np[m], NN = Np * Np;
@@ -308,6 +348,13 @@ void batch_gw(Batch* b) {
     f.push_back(group(Z, false, false, Np, NN, Z, false, true, Np, NN, F, Np, NN, Np, Np, Np, nwh, s3));
     for (int64_t w = 0; w < nwh; ++w)
       hp.push_back(cq::HermProblem{Z + w * NN, F + w * NN, E + w * NN, Np});
+    if (b->fac(m)) {  // T on and below the diagonal, W's upper triangle from the other side
+      uint32_t *m0 = b->rm0.p + b->offR[m], *m1 = b->rm1.p + b->offR[m];
+      r4.push_back(cq::TcRowMaxGroup{E, Np, NN, nwh, m0, 0});
+      f4.push_back(factor_group(*b->Lp[m], false, E, NN, m0, F, NN, m1, -1));
+      f5.push_back(factor_group(*b->Lp[m], false, F, NN, m1, b->PW.p + b->offPQ[m], cols, nullptr, 1));
+      continue;
+    }
     cq::TcStructure s4;
     s4.a_lower = true;
     s4.lower_only = true;  // W is Hermitian: its lower triangle needs T only down there
@@ -331,8 +378,15 @@ void batch_gw(Batch* b) {
   CQ_CHECK_CUDA(cudaGetLastError());
   cq::tc_cgemm_grouped(t4, b->gtab, s);
   cq::tc_cgemm_grouped(t5, b->gtab, s);
-  for (int64_t m = 0; m < b->nmol; ++m)  // upper triangle of W from the lower one
-    cq::launch_mirror_upper(b->PW.p + b->offPQ[m], b->Np[m], nwh, s, cols);
+  CQ_CHECK_CUDA(cudaMemsetAsync(b->rm1.p, 0, b->nR * sizeof(uint32_t), s));
+  cq::tc_row_max_grouped(r4, b->gtab, s);
+  cq::tc_factor_grouped(f4, b->gtab, s);
+  cq::tc_factor_grouped(f5, b->gtab, s);
+  for (int64_t m = 0; m < b->nmol; ++m)  // the other triangle of W
+    if (b->fac(m))
+      cq::launch_mirror_lower(b->PW.p + b->offPQ[m], b->Np[m], nwh, s, cols);
+    else
+      cq::launch_mirror_upper(b->PW.p + b->offPQ[m], b->Np[m], nwh, s, cols);
   cq::launch_ir_transform_real<float>(b->PW.p, cols, (int)nwh, (int)nth, b->dTtwR.p, s);
   // ---- Sigma_PQ(t) = -G_PQ(t) o W(t) in place in the cache (both halves), then X^H S X ----
   float2* gn = b->cache.p + (nt - 1) * cols;
@@ -400,7 +454,11 @@ int coqui_b200_batch_create(coqui_b200_batch** out, int64_t nmol, const int64_t*
       b->cols += Np[m] * Np[m];
       b->nX += Np[m] * nb[m];
       b->nG += nt_f * nb[m] * nb[m];
-      b->nL += Np[m] * Np[m];
+      if (!b->fac(m)) b->nL += Np[m] * Np[m];
+      b->offR.push_back(b->nR);
+      b->nR += b->nwh * Np[m];
+      b->Lp.emplace_back(new cq::TcFactor());
+      b->LHp.emplace_back(new cq::TcFactor());
       b->nD += b->nwh * Np[m] * Np[m];
       b->nmax = std::max(b->nmax, Np[m]);
     }
@@ -422,6 +480,8 @@ int coqui_b200_batch_create(coqui_b200_batch** out, int64_t nmol, const int64_t*
     b->Zb.ensure(b->nD);
     b->Zl.ensure(b->nD);
     b->Ab.ensure(b->nD);
+    b->rm0.ensure(b->nR);
+    b->rm1.ensure(b->nR);
     std::vector<int64_t> offs(b->offG);
     b->dofG.ensure(nmol);
     b->dnb.ensure(nmol);
@@ -505,8 +565,13 @@ int coqui_b200_batch_set_thc(coqui_b200_batch* b, int64_t m, const double* X_Pa,
     cq::launch_zero_upper_and_adjoint(L.p, LH.p, Np, 1, b->st);
     cq::to_c64(X.p, b->Xs.p + b->offX[m], Np, nb, 1, false, b->st);
     cq::to_c64(X.p, b->XTs.p + b->offX[m], Np, nb, 1, true, b->st);
-    cq::to_c64(L.p, b->Ls.p + b->offL[m], Np, Np, 1, false, b->st);
-    cq::to_c64(LH.p, b->LHs.p + b->offL[m], Np, Np, 1, false, b->st);
+    if (b->fac(m)) {
+      cq::tc_pack_factor(*b->Lp[m], L.p, Np, 1, b->st);
+      cq::tc_pack_factor(*b->LHp[m], LH.p, Np, 1, b->st);
+    } else {
+      cq::to_c64(L.p, b->Ls.p + b->offL[m], Np, Np, 1, false, b->st);
+      cq::to_c64(LH.p, b->LHs.p + b->offL[m], Np, Np, 1, false, b->st);
+    }
     CQ_CHECK_CUDA(cudaStreamSynchronize(b->st));
     b->have_thc[m] = 1;
   });

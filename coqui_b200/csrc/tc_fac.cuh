@@ -342,6 +342,36 @@ __global__ void __launch_bounds__(kFacThreads, 1) k_tc_fac(const __grid_constant
   fac_tile(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
 }
 
+// Products of different sizes in one launch (a group each); the flattened tile index picks the
+// group by binary search.
+struct FacGroupDev {
+  FacParams p;
+  int64_t tiles, tile_begin;  // tiles per matrix edge
+};
+__global__ void __launch_bounds__(kFacThreads, 1)
+    k_tc_fac_grouped(const FacGroupDev* __restrict__ groups, int ngroups) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ FacParams sp;
+  __shared__ int64_t s_bz, s_m0, s_n0;
+  if (threadIdx.x == 0) {
+    const int64_t t = blockIdx.x;
+    int lo = 0, hi = ngroups - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) / 2;
+      if (groups[mid].tile_begin <= t) lo = mid;
+      else hi = mid - 1;
+    }
+    const FacGroupDev& g = groups[lo];
+    const int64_t local = t - g.tile_begin, per = g.tiles * g.tiles, r = local % per;
+    sp = g.p;
+    s_bz = local / per;
+    s_m0 = r / g.tiles * kBM;
+    s_n0 = r % g.tiles * kFacN;
+  }
+  __syncthreads();
+  fac_tile(sp, s_bz, s_m0, s_n0, smem_raw);
+}
+
 // Largest |re|, |im| of each matrix of nmat n x n complex128 matrices (bits of a float, rounded up)
 __global__ void k_fac_max(const double2* __restrict__ L, uint32_t* __restrict__ mx, int64_t n) {
   const double2* a = L + (int64_t)blockIdx.y * n * n;
@@ -388,14 +418,29 @@ __global__ void k_fac_pack(const double2* __restrict__ L, const uint32_t* __rest
 }
 
 // Row maxima (bits of the largest |re|, |im|) of a complex64 n-column matrix, one warp per row
-__global__ void __launch_bounds__(256) k_row_max(const float2* __restrict__ A,
-                                                 uint32_t* __restrict__ rm, int64_t rows, int64_t n) {
-  const int64_t r = (int64_t)blockIdx.x * 8 + threadIdx.x / 32;
-  if (r >= rows) return;
-  const float2* a = A + r * n;
+__device__ __forceinline__ void row_max(const float2* __restrict__ a, uint32_t* rm, int64_t n) {
   float m = 0.f;
 #pragma unroll 4
   for (int64_t i = threadIdx.x & 31; i < n; i += 32) m = fmaxf(m, fmaxf(fabsf(a[i].x), fabsf(a[i].y)));
   const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-  if ((threadIdx.x & 31) == 0) rm[r] = w;
+  if ((threadIdx.x & 31) == 0) *rm = w;
+}
+__global__ void __launch_bounds__(256) k_row_max(const float2* __restrict__ A,
+                                                 uint32_t* __restrict__ rm, int64_t rows, int64_t n) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + threadIdx.x / 32;
+  if (r < rows) row_max(A + r * n, rm + r, n);
+}
+// the same for matrices of different sizes: group g has `batch` matrices of n rows, sA apart
+__global__ void __launch_bounds__(256) k_row_max_grouped(const TcRowMaxGroup* __restrict__ groups,
+                                                         int ngroups) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + threadIdx.x / 32;
+  int lo = 0, hi = ngroups - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (groups[mid].row_begin <= r) lo = mid;
+    else hi = mid - 1;
+  }
+  const TcRowMaxGroup g = groups[lo];
+  const int64_t l = r - g.row_begin;
+  if (l < g.n * g.batch) row_max(g.A + l / g.n * g.sA + l % g.n * g.n, g.rm + l, g.n);
 }

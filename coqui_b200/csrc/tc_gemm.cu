@@ -1178,6 +1178,82 @@ void tc_pack_factor(TcFactor& f, const double2* L, int64_t n, int64_t nmat, cuda
   CQ_CHECK_CUDA(cudaStreamSynchronize(s));  // mx is freed on return
 }
 
+namespace {
+void fac_smem_attr() {
+  static bool set[64] = {};
+  int dev = 0;
+  CQ_CHECK_CUDA(cudaGetDevice(&dev));
+  if (dev < 64 && set[dev]) return;
+  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac, cudaFuncAttributeMaxDynamicSharedMemorySize, kFacSmem));
+  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kFacSmem));
+  if (dev < 64) set[dev] = true;
+}
+}  // namespace
+
+void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned char>& table,
+                       cudaStream_t s) {
+  if (groups.empty()) return;
+  // longest K first, as in tc_cgemm_grouped
+  std::vector<TcFactorGroup> order(groups);
+  std::stable_sort(order.begin(), order.end(),
+                   [](const TcFactorGroup& x, const TcFactorGroup& y) { return x.f.n > y.f.n; });
+  std::vector<FacGroupDev> h;
+  int64_t total = 0;
+  for (const TcFactorGroup& g : order) {
+    const int64_t n = g.f.n;
+    FacGroupDev d;
+    d.p.A = g.f.packed;
+    d.p.sA = 0;
+    d.p.a_mod = 1;
+    d.p.a_q0 = 0;
+    d.p.invA = g.f.inv;
+    d.p.B = g.Bt;
+    d.p.ldb = d.p.ldc = n;
+    d.p.sB = g.sB;
+    d.p.rmB = g.row_max;
+    d.p.C = g.C;
+    d.p.sC = g.sC;
+    d.p.rmC = g.out_max;
+    d.p.n = n;
+    d.p.conj_b = g.conj_b;
+    d.p.upper_a = g.upper;
+    d.p.half = g.half;
+    d.p.b_al = rows_aligned(g.Bt, false, n, g.sB);
+    d.tiles = (n + kBM - 1) / kBM;
+    d.tile_begin = total;
+    total += d.tiles * d.tiles * g.batch;
+    h.push_back(d);
+  }
+  CQ_REQUIRE(total <= 2147483647, COQUI_B200_EINVAL, "tc_factor_grouped: too many tiles");
+  fac_smem_attr();
+  table.ensure(h.size() * sizeof(FacGroupDev));
+  CQ_CHECK_CUDA(cudaMemcpyAsync(table.p, h.data(), h.size() * sizeof(FacGroupDev),
+                                cudaMemcpyHostToDevice, s));
+  k_tc_fac_grouped<<<(unsigned)total, kFacThreads, kFacSmem, s>>>((const FacGroupDev*)table.p,
+                                                                  (int)h.size());
+  count_launch();
+  CQ_CHECK_CUDA(cudaGetLastError());
+}
+
+void tc_row_max_grouped(std::vector<TcRowMaxGroup> groups, DevBuf<unsigned char>& table,
+                        cudaStream_t s) {
+  if (groups.empty()) return;
+  int64_t rows = 0;
+  for (TcRowMaxGroup& g : groups) {
+    g.row_begin = rows;
+    rows += g.n * g.batch;
+  }
+  CQ_REQUIRE(rows <= (int64_t)8 * 2147483647, COQUI_B200_EINVAL, "tc_row_max: too many rows");
+  table.ensure(groups.size() * sizeof(TcRowMaxGroup));
+  CQ_CHECK_CUDA(cudaMemcpyAsync(table.p, groups.data(), groups.size() * sizeof(TcRowMaxGroup),
+                                cudaMemcpyHostToDevice, s));
+  k_row_max_grouped<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>((const TcRowMaxGroup*)table.p,
+                                                              (int)groups.size());
+  count_launch();
+  CQ_CHECK_CUDA(cudaGetLastError());
+}
+
 void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q0, const float2* Bt,
                        bool conj_b, const uint32_t* row_max, float2* C, uint32_t* out_max, int half,
                        int64_t batch, cudaStream_t s) {
@@ -1195,13 +1271,7 @@ void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q
   p.upper_a = upper;
   p.half = half;
   p.b_al = rows_aligned(Bt, false, n, n * n);
-  static bool attr_set[64] = {};
-  int dev = 0;
-  CQ_CHECK_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !attr_set[dev]) {
-    CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac, cudaFuncAttributeMaxDynamicSharedMemorySize, kFacSmem));
-    if (dev < 64) attr_set[dev] = true;
-  }
+  fac_smem_attr();
   const unsigned t = (unsigned)((n + kBM - 1) / kBM);
   for (int64_t b0 = 0; b0 < batch; b0 += 65535) {
     const int64_t nb = std::min<int64_t>(65535, batch - b0);

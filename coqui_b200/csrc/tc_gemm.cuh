@@ -95,6 +95,31 @@ void tc_pack_factor(TcFactor& f, const double2* L, int64_t n, int64_t nmat, cuda
 void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q0, const float2* Bt,
                        bool conj_b, const uint32_t* row_max, float2* C, uint32_t* out_max, int half,
                        int64_t batch, cudaStream_t s);
+// The same for groups of different sizes in one launch; a group's Bt and C hold `batch` matrices
+// sB and sC elements apart, all with one factor.  table: device copy of the descriptors.
+struct TcFactorGroup {
+  TcFactorView f;
+  bool upper = false, conj_b = false;
+  const float2* Bt = nullptr;
+  int64_t sB = 0;
+  const uint32_t* row_max = nullptr;
+  float2* C = nullptr;
+  int64_t sC = 0;
+  uint32_t* out_max = nullptr;
+  int half = 0;
+  int64_t batch = 1;
+};
+void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned char>& table,
+                       cudaStream_t s);
+// Row maxima of `batch` n x n complex64 matrices sA apart into rm (batch, n), for every group.
+struct TcRowMaxGroup {
+  const float2* A;
+  int64_t n, sA, batch;
+  uint32_t* rm;
+  int64_t row_begin;  // filled in by the call
+};
+void tc_row_max_grouped(std::vector<TcRowMaxGroup> groups, DevBuf<unsigned char>& table,
+                        cudaStream_t s);
 // Row maxima of a (rows, n) complex64 array, as tc_factor_product reads them.
 void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s);
 
