@@ -611,6 +611,12 @@ float mlp_backward(Mlp& n, const float* x, const float* t, int64_t B, cudaStream
   float* g = n.g.p;
   const __nv_bfloat16* W = n.wb.p;
   std::vector<float> part;
+  // one workspace for every split reduction below (growing it step by step would free and
+  // allocate between the kernels of a first call): the widest weight gradient's slices, the
+  // output layer's and the input layer's block sums
+  const int64_t widest = std::max({H * H, H * n.din, H * D});
+  n.part.ensure(std::max({(2 * 148 + (H * H + 16383) / 16384) * widest / std::max<int64_t>(1, (H * H) / 16384),
+                          148 * (D * H + H + D + 1), 592 * (H * std::min<int64_t>(n.din, 8) + H)}));
   if (fused_out(n)) {
     mlp_hidden(n, x, B, s);
     const unsigned blocks = out_blocks(B);
