@@ -566,8 +566,8 @@ int coqui_b200_batch_set_thc(coqui_b200_batch* b, int64_t m, const double* X_Pa,
     cq::to_c64(X.p, b->Xs.p + b->offX[m], Np, nb, 1, false, b->st);
     cq::to_c64(X.p, b->XTs.p + b->offX[m], Np, nb, 1, true, b->st);
     if (b->fac(m)) {
-      cq::tc_pack_factor(*b->Lp[m], L.p, Np, 1, b->st);
-      cq::tc_pack_factor(*b->LHp[m], LH.p, Np, 1, b->st);
+      cq::tc_pack_matrix(*b->Lp[m], L.p, Np, Np, 1, b->st);
+      cq::tc_pack_matrix(*b->LHp[m], LH.p, Np, Np, 1, b->st);
     } else {
       cq::to_c64(L.p, b->Ls.p + b->offL[m], Np, Np, 1, false, b->st);
       cq::to_c64(LH.p, b->LHs.p + b->offL[m], Np, Np, 1, false, b->st);

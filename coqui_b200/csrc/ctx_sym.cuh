@@ -74,7 +74,8 @@ void sym_prepare_thc(Ctx* c) {
   const bool packed = mixed && Np > cq::kInvGroup;
   if (packed) {
     for (auto f : {std::make_pair(&S.Lpi, &c->Lp), std::make_pair(&S.LHpi, &c->LHp)}) {
-      f.first->n = f.second->n;
+      f.first->M = f.second->M;
+      f.first->K = f.second->K;
       f.first->stride = f.second->stride;
       f.first->packed.ensure((size_t)nqi * f.second->stride);
       f.first->inv.ensure(nqi);

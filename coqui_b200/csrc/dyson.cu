@@ -292,9 +292,9 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
         // P1(j, k) at k >= i >= j only), then M's lower triangle; Pi Hermitian
         tc_row_max((const float2*)Pi, rm0, nb * Np, Np, s);
         CQ_CHECK_CUDA(cudaMemsetAsync(rm1, 0, (size_t)nb * Np * sizeof(uint32_t), s));
-        tc_factor_product(a.LHp, true, nq, q0, (const float2*)Pi, true, rm0, (float2*)T1, rm1, 1, nb,
+        tc_packed_product(a.LHp, 1, nq, q0, (const float2*)Pi, true, Np, rm0, (float2*)T1, rm1, 1, nb,
                           s);
-        tc_factor_product(a.LHp, true, nq, q0, (const float2*)T1, true, rm1, (float2*)Mb, nullptr, -1,
+        tc_packed_product(a.LHp, 1, nq, q0, (const float2*)T1, true, Np, rm1, (float2*)Mb, nullptr, -1,
                           nb, s);
       } else if (a.mixed) {
         // P1 = L^H Pi  (Pi Hermitian: B(k, n) = Pi[k][n] = conj(Pi[n][k]))
@@ -426,8 +426,8 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
         // cost it 0.8 ms at 4x4x4 / 512, the pass 0.47 ms.)
         tc_row_max(E, rm0, nb * Np, Np, s);
         CQ_CHECK_CUDA(cudaMemsetAsync(rm1, 0, (size_t)nb * Np * sizeof(uint32_t), s));
-        tc_factor_product(a.Lp, false, nq, q0, E, true, rm0, F, rm1, -1, nb, s);
-        tc_factor_product(a.Lp, false, nq, q0, F, true, rm1, (float2*)Pi, nullptr, 1, nb, s);
+        tc_packed_product(a.Lp, -1, nq, q0, E, true, Np, rm0, F, rm1, -1, nb, s);
+        tc_packed_product(a.Lp, -1, nq, q0, F, true, Np, rm1, (float2*)Pi, nullptr, 1, nb, s);
         launch_mirror_lower((float2*)Pi, Np, nb, s);
         continue;
       }

@@ -29,12 +29,15 @@ constexpr int kFacKC = 32;                                  // complex K per sta
 constexpr int kFacTile = 2 * kBM * 128;                     // bytes of a packed A tile (hi, lo)
 constexpr int kFacBPlane = 2 * kFacN * 128;                 // bytes of a B plane (256 real rows)
 constexpr int kFacStage = kFacTile + 2 * kFacBPlane;        // 96 KB
-constexpr int kFacStages = 2;
 constexpr int kFacThreads = 320;
-constexpr int kFacSmem = kFacStages * kFacStage + 1024 /*align*/ + 256 /*barriers*/ + 512 /*scales*/;
+// ST stages: two for long K; one for K of a few blocks, where a second CTA on the SM (96 KB each)
+// covers the first one's start and epilogue
+template <int ST> constexpr int fac_smem() {
+  return ST * kFacStage + 1024 /*align*/ + 256 /*barriers*/ + 512 /*scales*/;
+}
+template <int ST> constexpr int fac_epi_cols() { return ST == 2 ? kFacN : kFacN / 2; }
 constexpr uint32_t kFacIdesc = (1u << 4) | ((uint32_t)(2 * kFacN >> 3) << 17) |
                                ((uint32_t)(kBM >> 4) << 24);  // F16 x F16 -> F32, K-major
-constexpr int kFacPitch = kFacN + 4;                        // floats per row of a warp's buffer
 
 // 2^(14 - exponent) of a row or matrix maximum (bits of a non-negative float): the scaled values
 // stay below 2^15; 1 for zero and non-finite maxima (those values then propagate as they are)
@@ -74,8 +77,10 @@ struct FacParams {
   float2* C;
   int64_t ldc, sC;
   uint32_t* rmC;           // (batch, n) row maxima of C, raised by atomics; may be null
-  int64_t n;               // M = N = K
-  int conj_b, upper_a, half;  // half < 0: tiles on or below the diagonal, > 0: on or above
+  int64_t M, N, K;
+  int conj_b;
+  int tri;   // A is upper (> 0: k >= m) or lower (< 0: k <= m) triangular, or full (0)
+  int half;  // < 0: tiles on or below the diagonal only, > 0: on or above
   int b_al;
 };
 
@@ -85,7 +90,7 @@ struct FacStaging {
   __device__ __forceinline__ void load(const FacParams& p, const float2* base, uint32_t ok,
                                        int64_t k0) {
     const int64_t k = k0 + 4 * (threadIdx.x & 7);
-    if (k0 + kFacKC <= p.n && p.b_al) {
+    if (k0 + kFacKC <= p.K && p.b_al) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float4* q = reinterpret_cast<const float4*>(base + (int64_t)(32 * j) * p.ldb + k0);
@@ -100,7 +105,7 @@ struct FacStaging {
         float2 w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          w[i] = (((ok >> j) & 1u) && k + i < p.n) ? __ldg(q + i) : make_float2(0.f, 0.f);
+          w[i] = (((ok >> j) & 1u) && k + i < p.K) ? __ldg(q + i) : make_float2(0.f, 0.f);
         v[j][0] = make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
         v[j][1] = make_float4(w[2].x, w[2].y, w[3].x, w[3].y);
       }
@@ -139,27 +144,28 @@ struct FacStaging {
   }
 };
 
+template <int ST>
 __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t m0, int64_t n0,
                                          unsigned char* smem_raw) {
   if (p.half < 0 && n0 > m0) return;  // tiles strictly above the diagonal
   if (p.half > 0 && n0 < m0) return;  // strictly below
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full_b = reinterpret_cast<uint64_t*>(smem + kFacStages * kFacStage);
-  uint64_t *full_a = full_b + kFacStages, *empty = full_a + kFacStages;
-  uint64_t *acc_bar = empty + kFacStages, *done_bar = acc_bar + 1;
+  uint64_t* full_b = reinterpret_cast<uint64_t*>(smem + ST * kFacStage);
+  uint64_t *full_a = full_b + ST, *empty = full_a + ST;
+  uint64_t *acc_bar = empty + ST, *done_bar = acc_bar + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
-  float* scale = reinterpret_cast<float*>(smem + kFacStages * kFacStage + 256);
+  float* scale = reinterpret_cast<float*>(smem + ST * kFacStage + 256);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  // the factor is zero beyond its triangle
-  const int kbs = (int)((p.n + kFacKC - 1) / kFacKC);
-  const int kb_lo = p.upper_a ? (int)(m0 / kFacKC) : 0;
-  const int kb_hi = p.upper_a ? kbs : min(kbs, (int)((m0 + kBM) / kFacKC));
+  // a triangular factor is zero beyond its triangle
+  const int kbs = (int)((p.K + kFacKC - 1) / kFacKC);
+  const int kb_lo = p.tri > 0 ? (int)(m0 / kFacKC) : 0;
+  const int kb_hi = p.tri < 0 ? min(kbs, (int)((m0 + kBM) / kFacKC)) : kbs;
   const int nkb = kb_hi - kb_lo;
   const int64_t ia = (p.a_q0 + bz) % p.a_mod;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kFacStages; ++s) {
+    for (int s = 0; s < ST; ++s) {
       mbar_init(smem_u32(&full_b[s]), 8);  // one arrival per producer warp
       mbar_init(smem_u32(&full_a[s]), 1);
       mbar_init(smem_u32(&empty[s]), 1);
@@ -171,7 +177,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
   if (threadIdx.x < kFacN) {
     // takes both powers of two out of column n0 + threadIdx.x
     const int64_t c = n0 + threadIdx.x;
-    const int e = c < p.n ? fac_exp(p.rmB[bz * p.n + c]) : 14;
+    const int e = c < p.N ? fac_exp(p.rmB[bz * p.N + c]) : 14;
     scale[threadIdx.x] = p.invA[ia] * pow2f(e - 14);
   }
   if (warp == 8) {
@@ -196,30 +202,38 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int64_t row = n0 + r + 32 * j;
-      if (row < p.n) rows |= 1u << j;
-      sc[j] = pow2f(14 - (row < p.n ? fac_exp(p.rmB[bz * p.n + row]) : 14));
+      if (row < p.N) rows |= 1u << j;
+      sc[j] = pow2f(14 - (row < p.N ? fac_exp(p.rmB[bz * p.N + row]) : 14));
     }
     auto step = [&](FacStaging& st, int it) -> bool {
-      const int s = it % kFacStages;
-      if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(it / kFacStages) & 1u) ^ 1u)) return false;
+      const int s = it % ST;
+      if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(it / ST) & 1u) ^ 1u)) return false;
       const uint32_t hi = smem_u32(smem + s * kFacStage + kFacTile);
       st.store(sc, p.conj_b, hi, hi + kFacBPlane);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&full_b[s]));
-      if (it + 2 < nkb) st.load(p, base, rows, (int64_t)(kb_lo + it + 2) * kFacKC);
+      if (it + ST < nkb) st.load(p, base, rows, (int64_t)(kb_lo + it + ST) * kFacKC);
       return true;
     };
-    FacStaging st0, st1;
+    FacStaging st0;
     st0.load(p, base, rows, (int64_t)kb_lo * kFacKC);
-    if (nkb > 1) st1.load(p, base, rows, (int64_t)(kb_lo + 1) * kFacKC);
-    for (int it = 0; it < nkb; it += 2) {
-      if (!step(st0, it)) { ok = false; break; }
-      if (it + 1 < nkb && !step(st1, it + 1)) { ok = false; break; }
+    if constexpr (ST == 2) {
+      FacStaging st1;
+      if (nkb > 1) st1.load(p, base, rows, (int64_t)(kb_lo + 1) * kFacKC);
+      for (int it = 0; it < nkb; it += 2) {
+        if (!step(st0, it)) { ok = false; break; }
+        if (it + 1 < nkb && !step(st1, it + 1)) { ok = false; break; }
+      }
+    } else {
+      for (int it = 0; it < nkb; ++it)
+        if (!step(st0, it)) { ok = false; break; }
     }
     // ---------------- epilogue: TMEM -> registers (scaled) -> smem -> coalesced rows -----------
     const int q = warp & 3, h = warp >> 2;  // TMEM lane quadrant, column half
-    float* buf = reinterpret_cast<float*>(smem) + warp * 32 * kFacPitch;
+    constexpr int EC = fac_epi_cols<ST>(), PITCH = EC + 4;  // columns drained at a time
+    static_assert(8 * 32 * PITCH * 4 <= ST * kFacStage, "epilogue buffer");
+    float* buf = reinterpret_cast<float*>(smem) + warp * 32 * PITCH;
     bool have = false;
     if (ok) {
       have = mbar_wait(smem_u32(acc_bar), 0u);
@@ -227,68 +241,75 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     }
     // all producers are past their last stage before it is reused
     asm volatile("bar.sync 1, %0;" ::"r"(256) : "memory");
-    const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * kFacN);
     float mx = 0.f;
 #pragma unroll 1
-    for (int j = 0; j < kFacN / 32; ++j) {
-      uint32_t v[32];
-      if (have) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-            "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
-            "%28, %29, %30, %31}, [%32];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-              "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-              "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-              "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
-              "=r"(v[31])
-            : "r"(trow + (uint32_t)(j * 32)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      } else {
+    for (int c0 = 0; c0 < kFacN; c0 += EC) {
+      const int col = h * kFacN + c0;  // first real column of this piece
+      const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)col;
+#pragma unroll 1
+      for (int j = 0; j < EC / 32; ++j) {
+        uint32_t v[32];
+        if (have) {
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+              "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
+              "%28, %29, %30, %31}, [%32];"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+                "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+                "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+                "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
+                "=r"(v[31])
+              : "r"(trow + (uint32_t)(j * 32)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        } else {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) v[x] = 0u;
+          for (int x = 0; x < 32; ++x) v[x] = 0u;
+        }
+        const float4* sc4 = reinterpret_cast<const float4*>(scale + (col + j * 32) / 2);
+        float4* dst = reinterpret_cast<float4*>(buf + lane * PITCH + j * 32);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {  // four complex columns
+          const float4 f = sc4[x];
+          const float o[8] = {
+              __uint_as_float(v[8 * x]) * f.x,     __uint_as_float(v[8 * x + 1]) * f.x,
+              __uint_as_float(v[8 * x + 2]) * f.y, __uint_as_float(v[8 * x + 3]) * f.y,
+              __uint_as_float(v[8 * x + 4]) * f.z, __uint_as_float(v[8 * x + 5]) * f.z,
+              __uint_as_float(v[8 * x + 6]) * f.w, __uint_as_float(v[8 * x + 7]) * f.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(o[i]));
+          dst[2 * x] = make_float4(o[0], o[1], o[2], o[3]);
+          dst[2 * x + 1] = make_float4(o[4], o[5], o[6], o[7]);
+        }
       }
-      const float4* sc4 = reinterpret_cast<const float4*>(scale + (h * kFacN + j * 32) / 2);
-      float4* dst = reinterpret_cast<float4*>(buf + lane * kFacPitch + j * 32);
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {  // four complex columns
-        const float4 f = sc4[x];
-        const float o[8] = {__uint_as_float(v[8 * x]) * f.x,     __uint_as_float(v[8 * x + 1]) * f.x,
-                            __uint_as_float(v[8 * x + 2]) * f.y, __uint_as_float(v[8 * x + 3]) * f.y,
-                            __uint_as_float(v[8 * x + 4]) * f.z, __uint_as_float(v[8 * x + 5]) * f.z,
-                            __uint_as_float(v[8 * x + 6]) * f.w, __uint_as_float(v[8 * x + 7]) * f.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(o[i]));
-        dst[2 * x] = make_float4(o[0], o[1], o[2], o[3]);
-        dst[2 * x + 1] = make_float4(o[4], o[5], o[6], o[7]);
-      }
-    }
-    if (p.rmC && m0 + q * 32 + lane < p.n)
-      atomicMax(p.rmC + bz * p.n + m0 + q * 32 + lane, __float_as_uint(mx));
-    __syncwarp();
-    const int64_t nh = n0 + h * (kFacN / 2);
+      __syncwarp();
+      // EC / 4 lanes (16 bytes each) per row
+      constexpr int LPR = EC / 4;
 #pragma unroll 4
-    for (int rr = 0; rr < 32; ++rr) {
-      const int64_t m = m0 + q * 32 + rr;
-      if (m >= p.n) break;
-      float2* crow = p.C + bz * p.sC + m * p.ldc + nh + 2 * lane;
-      const float4 val = *reinterpret_cast<const float4*>(buf + rr * kFacPitch + 4 * lane);
-      const int64_t n = nh + 2 * lane;
-      if (n + 1 < p.n && ((reinterpret_cast<uintptr_t>(crow) & 15) == 0)) {
-        *reinterpret_cast<float4*>(crow) = val;
-      } else {
-        if (n < p.n) crow[0] = make_float2(val.x, val.y);
-        if (n + 1 < p.n) crow[1] = make_float2(val.z, val.w);
+      for (int i = lane; i < 32 * LPR; i += 32) {
+        const int rr = i / LPR, x = (i % LPR) * 4;
+        const int64_t m = m0 + q * 32 + rr, n = n0 + (col + x) / 2;
+        if (m >= p.M) continue;
+        float2* cp = p.C + bz * p.sC + m * p.ldc + n;
+        const float4 val = *reinterpret_cast<const float4*>(buf + rr * PITCH + x);
+        if (n + 1 < p.N && ((reinterpret_cast<uintptr_t>(cp) & 15) == 0)) {
+          *reinterpret_cast<float4*>(cp) = val;
+        } else {
+          if (n < p.N) cp[0] = make_float2(val.x, val.y);
+          if (n + 1 < p.N) cp[1] = make_float2(val.z, val.w);
+        }
       }
+      __syncwarp();
     }
+    if (p.rmC && m0 + q * 32 + lane < p.M)
+      atomicMax(p.rmC + bz * p.M + m0 + q * 32 + lane, __float_as_uint(mx));
   } else if (warp == 8) {
     if (lane == 0) {
       // ---------------- MMA issuer ----------------
       bool ok = true;
       for (int it = 0; it < nkb; ++it) {
-        const int s = it % kFacStages;
-        const uint32_t ph = (uint32_t)(it / kFacStages) & 1u;
+        const int s = it % ST;
+        const uint32_t ph = (uint32_t)(it / ST) & 1u;
         if (!mbar_wait(smem_u32(&full_a[s]), ph) || !mbar_wait(smem_u32(&full_b[s]), ph)) {
           ok = false;
           break;
@@ -317,14 +338,14 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     const unsigned char* a = p.A + ia * p.sA + ((m0 / kBM) * kbs + kb_lo) * (int64_t)kFacTile;
     int issued = 0;
     for (; issued < nkb; ++issued) {
-      const int s = issued % kFacStages;
-      if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(issued / kFacStages) & 1u) ^ 1u)) break;
+      const int s = issued % ST;
+      if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(issued / ST) & 1u) ^ 1u)) break;
       bulk_load(smem_u32(smem + s * kFacStage), a + (int64_t)issued * kFacTile, kFacTile,
                 smem_u32(&full_a[s]));
     }
     // every copy issued has landed before the CTA ends, also when a wait gave up
-    for (int it = max(0, issued - kFacStages); it < issued; ++it)
-      mbar_drain(smem_u32(&full_a[it % kFacStages]), (uint32_t)(it / kFacStages) & 1u);
+    for (int it = max(0, issued - ST); it < issued; ++it)
+      mbar_drain(smem_u32(&full_a[it % ST]), (uint32_t)(it / ST) & 1u);
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -337,9 +358,10 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
   }
 }
 
-__global__ void __launch_bounds__(kFacThreads, 1) k_tc_fac(const __grid_constant__ FacParams p) {
+template <int ST>
+__global__ void __launch_bounds__(kFacThreads, 3 - ST) k_tc_fac(const __grid_constant__ FacParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  fac_tile(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
+  fac_tile<ST>(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
 }
 
 // Products of different sizes in one launch (a group each); the flattened tile index picks the
@@ -369,14 +391,14 @@ __global__ void __launch_bounds__(kFacThreads, 1)
     s_n0 = r % g.tiles * kFacN;
   }
   __syncthreads();
-  fac_tile(sp, s_bz, s_m0, s_n0, smem_raw);
+  fac_tile<2>(sp, s_bz, s_m0, s_n0, smem_raw);
 }
 
-// Largest |re|, |im| of each matrix of nmat n x n complex128 matrices (bits of a float, rounded up)
+// Largest |re|, |im| of each of the complex128 matrices of n elements (bits of a float, rounded up)
 __global__ void k_fac_max(const double2* __restrict__ L, uint32_t* __restrict__ mx, int64_t n) {
-  const double2* a = L + (int64_t)blockIdx.y * n * n;
+  const double2* a = L + (int64_t)blockIdx.y * n;
   float m = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * n;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     m = fmaxf(m, __double2float_ru(fmax(fabs(a[i].x), fabs(a[i].y))));
   const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
@@ -384,17 +406,17 @@ __global__ void k_fac_max(const double2* __restrict__ L, uint32_t* __restrict__ 
 }
 
 // The packed tiles of a factor: tile (mt, kb) holds rows 128 mt .. and complex K 32 kb .. as a
-// 128 x 64 FP16 hi plane and a lo plane in the swizzled order of shared memory, zeros beyond n.
-// One thread per 16-byte chunk (four values).
+// 128 x 64 FP16 hi plane and a lo plane in the swizzled order of shared memory, zeros beyond the
+// matrix.  One thread per 16-byte chunk (four values).
 __global__ void k_fac_pack(const double2* __restrict__ L, const uint32_t* __restrict__ mx,
-                           unsigned char* __restrict__ out, float* __restrict__ inv, int64_t n,
-                           int64_t sA) {
-  const int64_t q = blockIdx.y, kbs = (n + kFacKC - 1) / kFacKC;
+                           unsigned char* __restrict__ out, float* __restrict__ inv, int64_t M,
+                           int64_t K, int64_t sA) {
+  const int64_t q = blockIdx.y, kbs = (K + kFacKC - 1) / kFacKC;
   const int e = fac_exp(mx[q]);
   const double s = (double)pow2f(14 - e);
   if (blockIdx.x == 0 && threadIdx.x == 0) inv[q] = pow2f(e - 14);
-  const double2* a = L + q * n * n;
-  const int64_t chunks = (n + kBM - 1) / kBM * kbs * kBM * 8;
+  const double2* a = L + q * M * K;
+  const int64_t chunks = (M + kBM - 1) / kBM * kbs * kBM * 8;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < chunks;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i & 7), r = (int)((i >> 3) % kBM);
@@ -403,7 +425,7 @@ __global__ void k_fac_pack(const double2* __restrict__ L, const uint32_t* __rest
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       double2 v = make_double2(0.0, 0.0);
-      if (m < n && k + j < n) v = a[m * n + k + j];
+      if (m < M && k + j < K) v = a[m * K + k + j];
       const double x = s * v.x, y = s * v.y;
       const __half hx = __double2half(x), hy = __double2half(y);
       const __half lx = __double2half(x - (double)__half2float(hx));

@@ -1161,18 +1161,19 @@ int tc_take_flags(int mask) {
 // ---------------------------------------------------------------------------------------
 // factor products (tc_fac.cuh)
 // ---------------------------------------------------------------------------------------
-void tc_pack_factor(TcFactor& f, const double2* L, int64_t n, int64_t nmat, cudaStream_t s) {
-  CQ_REQUIRE(nmat <= 65535, COQUI_B200_EUNSUPPORTED, "tc_pack_factor: too many matrices");
-  f.n = n;
-  f.stride = (n + kBM - 1) / kBM * ((n + kFacKC - 1) / kFacKC) * kFacTile;
+void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, cudaStream_t s) {
+  CQ_REQUIRE(nmat <= 65535, COQUI_B200_EUNSUPPORTED, "tc_pack_matrix: too many matrices");
+  f.M = M;
+  f.K = K;
+  f.stride = (M + kBM - 1) / kBM * ((K + kFacKC - 1) / kFacKC) * kFacTile;
   f.packed.ensure((size_t)nmat * f.stride);
   f.inv.ensure(nmat);
   DevBuf<uint32_t> mx;
   mx.ensure(nmat);
   CQ_CHECK_CUDA(cudaMemsetAsync(mx.p, 0, nmat * sizeof(uint32_t), s));
-  const unsigned g = grid_for(n * n, 256, 64);
-  k_fac_max<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, n);
-  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, f.packed.p, f.inv.p, n, f.stride);
+  const unsigned g = grid_for(M * K, 256, 64);
+  k_fac_max<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, M * K);
+  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, f.packed.p, f.inv.p, M, K, f.stride);
   count_launch(2);
   CQ_CHECK_CUDA(cudaGetLastError());
   CQ_CHECK_CUDA(cudaStreamSynchronize(s));  // mx is freed on return
@@ -1184,9 +1185,12 @@ void fac_smem_attr() {
   int dev = 0;
   CQ_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && set[dev]) return;
-  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac, cudaFuncAttributeMaxDynamicSharedMemorySize, kFacSmem));
+  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     fac_smem<1>()));
+  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     fac_smem<2>()));
   CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kFacSmem));
+                                     fac_smem<2>()));
   if (dev < 64) set[dev] = true;
 }
 }  // namespace
@@ -1197,11 +1201,11 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
   // longest K first, as in tc_cgemm_grouped
   std::vector<TcFactorGroup> order(groups);
   std::stable_sort(order.begin(), order.end(),
-                   [](const TcFactorGroup& x, const TcFactorGroup& y) { return x.f.n > y.f.n; });
+                   [](const TcFactorGroup& x, const TcFactorGroup& y) { return x.f.K > y.f.K; });
   std::vector<FacGroupDev> h;
   int64_t total = 0;
   for (const TcFactorGroup& g : order) {
-    const int64_t n = g.f.n;
+    const int64_t n = g.f.K;
     FacGroupDev d;
     d.p.A = g.f.packed;
     d.p.sA = 0;
@@ -1215,9 +1219,9 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
     d.p.C = g.C;
     d.p.sC = g.sC;
     d.p.rmC = g.out_max;
-    d.p.n = n;
+    d.p.M = d.p.N = d.p.K = n;
     d.p.conj_b = g.conj_b;
-    d.p.upper_a = g.upper;
+    d.p.tri = g.upper ? 1 : -1;
     d.p.half = g.half;
     d.p.b_al = rows_aligned(g.Bt, false, n, g.sB);
     d.tiles = (n + kBM - 1) / kBM;
@@ -1230,7 +1234,7 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
   table.ensure(h.size() * sizeof(FacGroupDev));
   CQ_CHECK_CUDA(cudaMemcpyAsync(table.p, h.data(), h.size() * sizeof(FacGroupDev),
                                 cudaMemcpyHostToDevice, s));
-  k_tc_fac_grouped<<<(unsigned)total, kFacThreads, kFacSmem, s>>>((const FacGroupDev*)table.p,
+  k_tc_fac_grouped<<<(unsigned)total, kFacThreads, fac_smem<2>(), s>>>((const FacGroupDev*)table.p,
                                                                   (int)h.size());
   count_launch();
   CQ_CHECK_CUDA(cudaGetLastError());
@@ -1254,33 +1258,38 @@ void tc_row_max_grouped(std::vector<TcRowMaxGroup> groups, DevBuf<unsigned char>
   CQ_CHECK_CUDA(cudaGetLastError());
 }
 
-void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q0, const float2* Bt,
-                       bool conj_b, const uint32_t* row_max, float2* C, uint32_t* out_max, int half,
-                       int64_t batch, cudaStream_t s) {
-  const int64_t n = f.n;
+void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, const float2* Bt,
+                       bool conj_b, int64_t N, const uint32_t* row_max, float2* C,
+                       uint32_t* out_max, int half, int64_t batch, cudaStream_t s) {
   FacParams p;
   p.A = f.packed;
   p.sA = f.stride;
   p.invA = f.inv;
   p.a_mod = mod;
-  p.B = Bt;
-  p.ldb = p.ldc = n;
-  p.sB = p.sC = n * n;
-  p.n = n;
+  p.M = f.M;
+  p.N = N;
+  p.K = f.K;
+  p.ldb = f.K;
+  p.ldc = N;
+  p.sB = N * f.K;
+  p.sC = f.M * N;
   p.conj_b = conj_b;
-  p.upper_a = upper;
+  p.tri = tri;
   p.half = half;
-  p.b_al = rows_aligned(Bt, false, n, n * n);
+  p.b_al = rows_aligned(Bt, false, p.ldb, p.sB);
   fac_smem_attr();
-  const unsigned t = (unsigned)((n + kBM - 1) / kBM);
+  const unsigned tn = (unsigned)((N + kFacN - 1) / kFacN), tm = (unsigned)((p.M + kBM - 1) / kBM);
   for (int64_t b0 = 0; b0 < batch; b0 += 65535) {
-    const int64_t nb = std::min<int64_t>(65535, batch - b0);
+    const unsigned nb = (unsigned)std::min<int64_t>(65535, batch - b0);
     p.a_q0 = (q0 + b0) % mod;
-    p.B = Bt + b0 * n * n;
-    p.rmB = row_max + b0 * n;
-    p.C = C + b0 * n * n;
-    p.rmC = out_max ? out_max + b0 * n : nullptr;
-    k_tc_fac<<<dim3(t, t, (unsigned)nb), kFacThreads, kFacSmem, s>>>(p);
+    p.B = Bt + b0 * p.sB;
+    p.rmB = row_max + b0 * N;
+    p.C = C + b0 * p.sC;
+    p.rmC = out_max ? out_max + b0 * p.M : nullptr;
+    if (p.K <= 4 * kFacKC)
+      k_tc_fac<1><<<dim3(tn, tm, nb), kFacThreads, fac_smem<1>(), s>>>(p);
+    else
+      k_tc_fac<2><<<dim3(tn, tm, nb), kFacThreads, fac_smem<2>(), s>>>(p);
     count_launch();
     CQ_CHECK_CUDA(cudaGetLastError());
   }
@@ -1343,6 +1352,16 @@ __global__ void k_transpose_c64(const double2* __restrict__ in, float2* __restri
   }
 }
 
+// out = in as complex64, NaN and Inf reported
+__global__ void k_c64_checked(const double2* __restrict__ in, float2* __restrict__ out, int64_t total) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double2 x = in[i];
+    if (!isfinite(x.x) || !isfinite(x.y)) atomicExch(&g_flags[1], 1);
+    out[i] = make_float2((float)x.x, (float)x.y);
+  }
+}
+
 // out[b] = in[b]^T, (rows x cols) complex64 blocks; 32 x 32 tiles through shared memory
 __global__ void k_transpose_f2(const float2* __restrict__ in, float2* __restrict__ out,
                                int64_t rows, int64_t cols) {
@@ -1385,6 +1404,13 @@ void to_c64(const double2* in, float2* out, int64_t rows, int64_t cols, int64_t 
   CQ_CHECK_CUDA(cudaGetLastError());
 }
 
+// Whether the primary -> aux projection runs on packed X (short K: two one-stage CTAs per SM).
+// Both forms timed, ms per GW iteration (TF32 form / packed): 4x4x4, nb 64, N_mu 512 4.02 / 3.60;
+// 3x3x3, 96, 1024 7.94 / 6.36; 3x3x3, 48, 384 1.00 / 1.00; 6x6x6, 24, 200 2.94 / 2.40; 4x4x4, 28,
+// 140 1.15 / 1.03; smaller nb pads most of a 32-wide K block, and one 128-row tile (N_mu <= 128)
+// keeps the narrower autotuned tiles.
+static bool packed_projection(int64_t Np, int64_t nb) { return Np > 128 && nb >= 24; }
+
 void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t nb,
                cudaStream_t s) {
   op.X = X;
@@ -1395,6 +1421,7 @@ void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t 
   float2* Xc = (float2*)op.packed.p;
   to_c64(X, Xc, Np, nb, nk, false, s);                 // X   (nk, Np, nb)
   to_c64(X, Xc + nk * Np * nb, Np, nb, nk, true, s);   // X^T (nk, nb, Np)
+  if (packed_projection(Np, nb)) tc_pack_matrix(op.Xp, X, Np, nb, nk, s);
 }
 
 void tc_project_p2a(TcOperand& op, const double2* Gk, float2* out, int64_t nk, int64_t Np,
@@ -1404,12 +1431,24 @@ void tc_project_p2a(TcOperand& op, const double2* Gk, float2* out, int64_t nk, i
   float2* T = (float2*)op.tmp.p;
   float2* Gt = T + nbatch * Np * nb;
   const int64_t tg = nbatch * nb * nb;
-  k_transpose_c64<<<grid_for(tg, 256), 256, 0, s>>>(Gk, Gt, nb, nb, tg);
-  count_launch();
   // problem b = (tau, k) uses X^k: X is addressed periodically with period nk
   TcStructure sx_a, sx_b;
   sx_a.a_mod = nk;
   sx_b.b_mod = nk;
+  if (packed_projection(Np, nb)) {
+    // out = X Y^T with Y = conj(X) G^T (Np x nb): Bt[b][c] = G[b][c]
+    op.rm.ensure((size_t)nbatch * Np);
+    k_c64_checked<<<grid_for(tg, 256), 256, 0, s>>>(Gk, Gt, tg);
+    count_launch();
+    CQ_CHECK_CUDA(cudaGetLastError());
+    tc_cgemm_nt(Xs, false, true, nb, Np * nb, Gt, false, false, nb, nb * nb, T, nb, Np * nb, Np, nb,
+                nb, nbatch, s, sx_a);
+    tc_row_max(T, op.rm.p, nbatch * Np, nb, s);
+    tc_packed_product(op.Xp.view(), 0, nk, 0, T, false, Np, op.rm.p, out, nullptr, 0, nbatch, s);
+    return;
+  }
+  k_transpose_c64<<<grid_for(tg, 256), 256, 0, s>>>(Gk, Gt, nb, nb, tg);
+  count_launch();
   // T = X G  (Np x nb, K = nb): Bt[j][i] = G[i][j]
   tc_cgemm_nt(Xs, false, false, nb, Np * nb, Gt, false, false, nb, nb * nb, T, nb, Np * nb, Np,
               nb, nb, nbatch, s, sx_a);
@@ -1425,7 +1464,9 @@ void tc_project_a2p(TcOperand& op, const float2* Sk, double2* out, int64_t nk, i
   float2* UT = (float2*)op.tmp.p;
   float2* Sab = UT + nbatch * Np * nb;
   // U = S X (Np x nb, K = Np) with the Np rows on the 128-row tiles, then U^T (the big product
-  // would waste half of every tile with the nb rows of U^T = X^T S^T on them)
+  // would waste half of every tile with the nb rows of U^T = X^T S^T on them; on packed X^T, which
+  // writes U^T at once, it takes 2.65 instead of 3.1 ms at 4x4x4 / 512, but the pass for S's row
+  // maxima costs 1.1)
   op.tmp2.ensure((size_t)nbatch * Np * nb * sizeof(float2));
   float2* U = (float2*)op.tmp2.p;
   TcStructure sb;

@@ -5,13 +5,46 @@
 
 namespace cq {
 
+// Matrices A (M x K) packed for tc_packed_product (split FP16 tiles, tc_fac.cuh).
+struct TcFactorView {
+  const unsigned char* packed = nullptr;  // matrices `stride` bytes apart
+  const float* inv = nullptr;             // 1 / scale of each
+  int64_t M = 0, K = 0, stride = 0;
+};
+struct TcFactor {
+  DevBuf<unsigned char> packed;
+  DevBuf<float> inv;
+  int64_t M = 0, K = 0, stride = 0;
+  TcFactorView view() const { return {packed.p, inv.p, M, K, stride}; }
+  void release() {
+    packed.release();
+    inv.release();
+  }
+};
+// nmat row-major complex128 matrices
+void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, cudaStream_t s);
+
+// C[b](m, n) = sum_k A(m, k) opB(Bt[b])(n, k) for b < batch: A the packed matrix (q0 + b) % mod,
+// upper (tri > 0: k >= m) or lower (tri < 0: k <= m) triangular or full; Bt (N x K) and C (M x N)
+// row-major complex64, one after the other; conj_b conjugates Bt.  row_max holds the row maxima of
+// Bt (bits of the largest |re|, |im| as float, (batch, N)); those of C are raised in out_max
+// ((batch, M), may be null).  half < 0: only the 128 x 128 tiles on or below the diagonal are formed
+// and written, half > 0: on or above it.
+void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, const float2* Bt,
+                       bool conj_b, int64_t N, const uint32_t* row_max, float2* C,
+                       uint32_t* out_max, int half, int64_t batch, cudaStream_t s);
+
 // THC collocation X (nk, Np, nb) prepared for the projection GEMMs.
 struct TcOperand {
   const double2* X = nullptr;
   int64_t nk = 0, Np = 0, nb = 0;
   DevBuf<unsigned char> packed;  // complex64 X (nk, Np, nb) then X^T (nk, nb, Np)
+  TcFactor Xp;                   // X packed, where the primary -> aux projection uses it
+  DevBuf<uint32_t> rm;           // row maxima of a call's operand
   DevBuf<unsigned char> tmp, tmp2;  // per-call intermediates
   void release() {
+    Xp.release();
+    rm.release();
     packed.release();
     tmp.release();
     tmp2.release();
@@ -69,33 +102,8 @@ void tc_cgemm_nt(const void* A, bool a_split, bool conj_a, int64_t lda, int64_t 
                  int64_t sC, int64_t M, int64_t N, int64_t K, int64_t batch, cudaStream_t s,
                  const TcStructure& st = TcStructure{});
 
-// Triangular n x n factors packed for tc_factor_product (split FP16 tiles, tc_fac.cuh).
-struct TcFactorView {
-  const unsigned char* packed = nullptr;  // matrices `stride` bytes apart
-  const float* inv = nullptr;             // 1 / scale of each
-  int64_t n = 0, stride = 0;
-};
-struct TcFactor {
-  DevBuf<unsigned char> packed;
-  DevBuf<float> inv;
-  int64_t n = 0, stride = 0;
-  TcFactorView view() const { return {packed.p, inv.p, n, stride}; }
-  void release() {
-    packed.release();
-    inv.release();
-  }
-};
-void tc_pack_factor(TcFactor& f, const double2* L, int64_t n, int64_t nmat, cudaStream_t s);
-
-// C[b](m, n) = sum_k A(m, k) opB(Bt[b])(n, k) for b < batch: A the packed factor (q0 + b) % mod,
-// upper (k >= m) or lower (k <= m) triangular; Bt and C row-major n x n complex64, conj_b
-// conjugates Bt.  row_max holds the row maxima of Bt (bits of the largest |re|, |im| as float,
-// (batch, n)); those of C are raised in out_max (may be null).  half < 0: only the 128 x 128 tiles
-// on or below the diagonal are formed and written, half > 0: on or above it.
-void tc_factor_product(const TcFactorView& f, bool upper, int64_t mod, int64_t q0, const float2* Bt,
-                       bool conj_b, const uint32_t* row_max, float2* C, uint32_t* out_max, int half,
-                       int64_t batch, cudaStream_t s);
-// The same for groups of different sizes in one launch; a group's Bt and C hold `batch` matrices
+// Products of square triangular factors (M = N = K) of different sizes in one launch; a group's Bt
+// and C hold `batch` matrices
 // sB and sC elements apart, all with one factor.  table: device copy of the descriptors.
 struct TcFactorGroup {
   TcFactorView f;
@@ -120,7 +128,7 @@ struct TcRowMaxGroup {
 };
 void tc_row_max_grouped(std::vector<TcRowMaxGroup> groups, DevBuf<unsigned char>& table,
                         cudaStream_t s);
-// Row maxima of a (rows, n) complex64 array, as tc_factor_product reads them.
+// Row maxima of a (rows, n) complex64 array, as tc_packed_product reads them.
 void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s);
 
 // One group of a grouped product: a batched "NT" product as tc_cgemm_nt describes.
