@@ -1286,7 +1286,10 @@ void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, 
     p.rmB = row_max + b0 * N;
     p.C = C + b0 * p.sC;
     p.rmC = out_max ? out_max + b0 * p.M : nullptr;
-    if (p.K <= 4 * kFacKC)
+    // one stage and two CTAs per SM while a tile has few K blocks: M products of 30 q at N_mu 203
+    // 0.504 against 0.516 ms, of 32 at 256 0.563 against 0.591; at 384 1.14 against 1.11 and at
+    // 1024 12.6 against 11.4 ms two stages are ahead
+    if (p.K <= 256)
       k_tc_fac<1><<<dim3(tn, tm, nb), kFacThreads, fac_smem<1>(), s>>>(p);
     else
       k_tc_fac<2><<<dim3(tn, tm, nb), kFacThreads, fac_smem<2>(), s>>>(p);
