@@ -1168,15 +1168,13 @@ void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t
   f.stride = (M + kBM - 1) / kBM * ((K + kFacKC - 1) / kFacKC) * kFacTile;
   f.packed.ensure((size_t)nmat * f.stride);
   f.inv.ensure(nmat);
-  DevBuf<uint32_t> mx;
-  mx.ensure(nmat);
-  CQ_CHECK_CUDA(cudaMemsetAsync(mx.p, 0, nmat * sizeof(uint32_t), s));
+  f.mx.ensure(nmat);
+  CQ_CHECK_CUDA(cudaMemsetAsync(f.mx.p, 0, nmat * sizeof(uint32_t), s));
   const unsigned g = grid_for(M * K, 256, 64);
-  k_fac_max<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, M * K);
-  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, mx.p, f.packed.p, f.inv.p, M, K, f.stride);
+  k_fac_max<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, f.mx.p, M * K);
+  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, f.mx.p, f.packed.p, f.inv.p, M, K, f.stride);
   count_launch(2);
   CQ_CHECK_CUDA(cudaGetLastError());
-  CQ_CHECK_CUDA(cudaStreamSynchronize(s));  // mx is freed on return
 }
 
 namespace {

@@ -14,11 +14,13 @@ struct TcFactorView {
 struct TcFactor {
   DevBuf<unsigned char> packed;
   DevBuf<float> inv;
+  DevBuf<uint32_t> mx;  // largest element of each, kept for the next packing
   int64_t M = 0, K = 0, stride = 0;
   TcFactorView view() const { return {packed.p, inv.p, M, K, stride}; }
   void release() {
     packed.release();
     inv.release();
+    mx.release();
   }
 };
 // nmat row-major complex128 matrices
