@@ -232,9 +232,11 @@ void batch_gw(Batch* b, const double* const* G_list, double* const* Sigma_list) 
     if (b->fac(m)) {
       float2 *T1 = b->T1.p + b->offD[m], *Pi = b->PW.p + b->offPQ[m];
       uint32_t *m0 = b->rm0.p + b->offR[m], *m1 = b->rm1.p + b->offR[m];
-      r1.push_back(cq::TcRowMaxGroup{Pi, Np, cols, nwh, m0, 0});
+      r1.push_back(cq::TcRowMaxGroup{Pi, Np, cols, nwh, m0, b->LHp[m]->view().ks, 0});
       f1.push_back(factor_group(*b->LHp[m], true, Pi, cols, m0, T1, NN, m1, 1));
+      f1.back().ks_c = true;
       f2.push_back(factor_group(*b->LHp[m], true, T1, NN, m1, b->Mb.p + b->offD[m], NN, nullptr, -1));
+      f2.back().b_has_ks = true;
       continue;
     }
     cq::TcStructure s1;
@@ -371,7 +373,7 @@ void batch_gw(Batch* b, const double* const* G_list, double* const* Sigma_list) 
       hp.push_back(cq::HermProblem{Z + w * NN, F + w * NN, E + w * NN, Np});
     if (b->fac(m)) {  // T on and below the diagonal, W's upper triangle from the other side
       uint32_t *m0 = b->rm0.p + b->offR[m], *m1 = b->rm1.p + b->offR[m];
-      r4.push_back(cq::TcRowMaxGroup{E, Np, NN, nwh, m0, 0});
+      r4.push_back(cq::TcRowMaxGroup{E, Np, NN, nwh, m0, nullptr, 0});
       f4.push_back(factor_group(*b->Lp[m], false, E, NN, m0, F, NN, m1, -1));
       f5.push_back(factor_group(*b->Lp[m], false, F, NN, m1, b->PW.p + b->offPQ[m], cols, nullptr, 1));
       continue;
@@ -606,8 +608,8 @@ int coqui_b200_batch_set_thc(coqui_b200_batch* b, int64_t m, const double* X_Pa,
     cq::to_c64(X.p, b->Xs.p + b->offX[m], Np, nb, 1, false, b->st);
     cq::to_c64(X.p, b->XTs.p + b->offX[m], Np, nb, 1, true, b->st);
     if (b->fac(m)) {
-      cq::tc_pack_matrix(*b->Lp[m], L.p, Np, Np, 1, b->st);
-      cq::tc_pack_matrix(*b->LHp[m], LH.p, Np, Np, 1, b->st);
+      cq::tc_pack_matrix(*b->Lp[m], L.p, Np, Np, 1, false, b->st);
+      cq::tc_pack_matrix(*b->LHp[m], LH.p, Np, Np, 1, true, b->st);
     } else {
       cq::to_c64(L.p, b->Ls.p + b->offL[m], Np, Np, 1, false, b->st);
       cq::to_c64(LH.p, b->LHs.p + b->offL[m], Np, Np, 1, false, b->st);

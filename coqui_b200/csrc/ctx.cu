@@ -1168,8 +1168,8 @@ int coqui_b200_set_thc(coqui_b200_ctx* c, const double* X_skPa, const double* V_
     if (c->mode == COQUI_B200_MIXED) {
       cq::tc_pack_X(c->Xtc, c->X.p, nk, Np, nb, c->st);
       if (Np > cq::kInvGroup) {
-        cq::tc_pack_matrix(c->Lp, c->L.p, Np, Np, nk, c->st);
-        cq::tc_pack_matrix(c->LHp, c->LH.p, Np, Np, nk, c->st);
+        cq::tc_pack_matrix(c->Lp, c->L.p, Np, Np, nk, false, c->st);
+        cq::tc_pack_matrix(c->LHp, c->LH.p, Np, Np, nk, true, c->st);
       } else {
         c->Lc.ensure((size_t)nk * Np * Np);
         c->LHc.ensure((size_t)nk * Np * Np);

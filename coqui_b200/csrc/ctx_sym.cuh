@@ -73,13 +73,8 @@ void sym_prepare_thc(Ctx* c) {
   const bool mixed = (c->mode == COQUI_B200_MIXED);
   const bool packed = mixed && Np > cq::kInvGroup;
   if (packed) {
-    for (auto f : {std::make_pair(&S.Lpi, &c->Lp), std::make_pair(&S.LHpi, &c->LHp)}) {
-      f.first->M = f.second->M;
-      f.first->K = f.second->K;
-      f.first->stride = f.second->stride;
-      f.first->packed.ensure((size_t)nqi * f.second->stride);
-      f.first->inv.ensure(nqi);
-    }
+    cq::tc_gather_matrices(S.Lpi, c->Lp, S.q_lex, c->st);
+    cq::tc_gather_matrices(S.LHpi, c->LHp, S.q_lex, c->st);
   } else if (mixed) {
     S.Lci.ensure((size_t)nqi * pp);
     S.LHci.ensure((size_t)nqi * pp);
@@ -90,15 +85,7 @@ void sym_prepare_thc(Ctx* c) {
     CQ_CHECK_CUDA(cudaMemcpyAsync(S.Li.p + i * pp, c->L.p + q * pp, b, cudaMemcpyDeviceToDevice, c->st));
     CQ_CHECK_CUDA(cudaMemcpyAsync(S.LHi.p + i * pp, c->LH.p + q * pp, b, cudaMemcpyDeviceToDevice, c->st));
     CQ_CHECK_CUDA(cudaMemcpyAsync(S.Vi.p + i * pp, c->V.p + q * pp, b, cudaMemcpyDeviceToDevice, c->st));
-    if (packed) {
-      for (auto f : {std::make_pair(&S.Lpi, &c->Lp), std::make_pair(&S.LHpi, &c->LHp)}) {
-        const int64_t st = f.first->stride;
-        CQ_CHECK_CUDA(cudaMemcpyAsync(f.first->packed.p + i * st, f.second->packed.p + q * st, st,
-                                      cudaMemcpyDeviceToDevice, c->st));
-        CQ_CHECK_CUDA(cudaMemcpyAsync(f.first->inv.p + i, f.second->inv.p + q, sizeof(float),
-                                      cudaMemcpyDeviceToDevice, c->st));
-      }
-    } else if (mixed) {
+    if (mixed && !packed) {
       const size_t bc = pp * sizeof(float2);
       CQ_CHECK_CUDA(cudaMemcpyAsync(S.Lci.p + i * pp, c->Lc.p + q * pp, bc, cudaMemcpyDeviceToDevice, c->st));
       CQ_CHECK_CUDA(cudaMemcpyAsync(S.LHci.p + i * pp, c->LHc.p + q * pp, bc, cudaMemcpyDeviceToDevice, c->st));

@@ -290,12 +290,13 @@ void dyson_run(const DysonArgs& a, DevBuf<unsigned char>& scratch, cudaStream_t 
       if (fac) {
         // P1 = L^H Pi on and above the diagonal (the lower triangle of M = L^H P1^H reads
         // P1(j, k) at k >= i >= j only), then M's lower triangle; Pi Hermitian
-        tc_row_max((const float2*)Pi, rm0, nb * Np, Np, s);
+        // (of a graded V, P1's columns leave with the scales that the second product wants)
+        tc_row_max((const float2*)Pi, rm0, nb * Np, Np, s, a.LHp.ks, Np, nq, q0);
         CQ_CHECK_CUDA(cudaMemsetAsync(rm1, 0, (size_t)nb * Np * sizeof(uint32_t), s));
         tc_packed_product(a.LHp, 1, nq, q0, (const float2*)Pi, true, Np, rm0, (float2*)T1, rm1, 1, nb,
-                          s);
+                          s, false, true);
         tc_packed_product(a.LHp, 1, nq, q0, (const float2*)T1, true, Np, rm1, (float2*)Mb, nullptr, -1,
-                          nb, s);
+                          nb, s, true);
       } else if (a.mixed) {
         // P1 = L^H Pi  (Pi Hermitian: B(k, n) = Pi[k][n] = conj(Pi[n][k]))
         // Only P1's tiles on and above the diagonal are needed: the lower triangle of M reads

@@ -10,10 +10,19 @@
 //  * the factor is laid out once per set_thc as the very shared-memory tiles the MMA reads (hi and
 //    lo planes, 128-byte swizzle), so a K block of A is one 32 KB bulk copy;
 //  * the words are FP16: half the bytes per value and twice the K per MMA.  hi = fp16(s x),
-//    lo = fp16(s x - hi) carry 22 bits, as hi + lo TF32 do, for every value within 2^-18 of the
-//    largest of its row (of its matrix for the factor); s is a power of two from that maximum,
-//    which the kernel that produced the operand left in an array, and the epilogue takes the
-//    powers out again.  Half as many additions into the FP32 accumulator round toward zero.
+//    lo = fp16(s x - hi) carry 22 bits for every value within 2^-18 of the largest of its row; s is
+//    a power of two from that maximum (of a row of Bt: from a pass over it or from the epilogue
+//    that wrote it), and the epilogue takes the powers out again.  Half as many additions into the
+//    FP32 accumulator round toward zero.
+//
+// FP16 has five exponent bits, where TF32 words have eight, so gradings have to be taken out first.
+// THC data have a free scale per point (X_P -> s_P X_P with V_PQ -> V_PQ / (s_P^2 s_Q^2)): L's rows
+// carry it and Pi its inverse, so in L^H Pi the small elements of one meet the large ones of the
+// other along K.  A factor whose columns differ by more than 2^kFacGrade is packed with them
+// brought to one size by powers of two, `ks`, which the product puts on Bt instead (X's columns in
+// the projection likewise: a free scale per orbital).  Relative error of Sigma at N_mu 300 for s_P
+// spread over 10^3 / 10^5 / 10^6, with one scale per matrix: 1.8e-5 / 3e-3 / 7e-2.
+//
 // Per 32 complex K: 96 KB stored and 144 KB read against 1536 cycles of MMA, and half the
 // conversion work.  Measured (1600 problems of N_mu 512 / 675 of 1024): the M products
 // 6.87 -> 4.24 ms / 17.1 -> 9.9 ms, T and W 8.7 -> 4.3 / 18.6 -> 9.9; W of random Hermitian Pi is
@@ -33,7 +42,7 @@ constexpr int kFacThreads = 320;
 // ST stages: two for long K; one for K of a few blocks, where a second CTA on the SM (96 KB each)
 // covers the first one's start and epilogue
 template <int ST> constexpr int fac_smem() {
-  return ST * kFacStage + 1024 /*align*/ + 256 /*barriers*/ + 512 /*scales*/;
+  return ST * kFacStage + 1024 /*align*/ + 256 /*barriers*/ + 512 + 32 /*scales, their exponents*/;
 }
 template <int ST> constexpr int fac_epi_cols() { return ST == 2 ? kFacN : kFacN / 2; }
 constexpr uint32_t kFacIdesc = (1u << 4) | ((uint32_t)(2 * kFacN >> 3) << 17) |
@@ -70,7 +79,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 struct FacParams {
   const unsigned char* A;  // packed factors, sA bytes apart; problem b uses (a_q0 + b) % a_mod
   int64_t sA, a_mod, a_q0;
-  const float* invA;       // 1 / scale of each factor
+  const float* invA;       // 1 / scale of each row of each factor, (a_mod, M)
+  const float* kB;         // powers of two that Bt takes along K, (a_mod, K); may be null
+  const float* nC;         // powers of two that C's columns take, (a_mod, N); may be null
   const float2* B;
   int64_t ldb, sB;
   const uint32_t* rmB;     // (batch, n) row maxima of Bt
@@ -84,12 +95,18 @@ struct FacParams {
   int b_al;
 };
 
-// 32 complex K of four rows of Bt per thread: four values (32 bytes) of rows r + 32 j
-struct FacStaging {
+// 32 complex K of four rows of Bt per thread: four values (32 bytes) of rows r + 32 j; KS: with the
+// scales of these K (one each without a kb)
+template <bool KS> struct FacStaging {
   float4 v[4][2];
-  __device__ __forceinline__ void load(const FacParams& p, const float2* base, uint32_t ok,
-                                       int64_t k0) {
+  float ck[4];
+  __device__ __forceinline__ void load(const FacParams& p, const float2* base, const float* kb,
+                                       uint32_t ok, int64_t k0) {
     const int64_t k = k0 + 4 * (threadIdx.x & 7);
+    if constexpr (KS) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ck[i] = kb && k + i < p.K ? __ldg(kb + k + i) : 1.f;
+    }
     if (k0 + kFacKC <= p.K && p.b_al) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -122,7 +139,8 @@ struct FacStaging {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float4 q = v[j][i >> 1];
-        const float x = sc[j] * ((i & 1) ? q.z : q.x), y = sc[j] * ((i & 1) ? q.w : q.y);
+        const float sk = KS ? sc[j] * ck[i] : sc[j];
+        const float x = sk * ((i & 1) ? q.z : q.x), y = sk * ((i & 1) ? q.w : q.y);
         const __half2 a = __floats2half2_rn(x, y);
         const float2 f = __half22float2(a);
         const __half2 b = __floats2half2_rn(x - f.x, y - f.y);
@@ -144,7 +162,7 @@ struct FacStaging {
   }
 };
 
-template <int ST>
+template <int ST, bool KS>
 __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t m0, int64_t n0,
                                          unsigned char* smem_raw) {
   if (p.half < 0 && n0 > m0) return;  // tiles strictly above the diagonal
@@ -155,6 +173,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
   uint64_t *acc_bar = empty + ST, *done_bar = acc_bar + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
   float* scale = reinterpret_cast<float*>(smem + ST * kFacStage + 256);
+  int* scale_exp = reinterpret_cast<int*>(scale + kFacN);  // smallest and largest, per warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // a triangular factor is zero beyond its triangle
@@ -175,10 +194,17 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < kFacN) {
-    // takes both powers of two out of column n0 + threadIdx.x
+    // takes the power of two of column n0 + threadIdx.x out again
     const int64_t c = n0 + threadIdx.x;
     const int e = c < p.N ? fac_exp(p.rmB[bz * p.N + c]) : 14;
-    scale[threadIdx.x] = p.invA[ia] * pow2f(e - 14);
+    const float f = pow2f(e - 14) * (p.nC && c < p.N ? p.nC[ia * p.N + c] : 1.f);
+    scale[threadIdx.x] = f;
+    const int ef = (int)(__float_as_uint(f) >> 23) - 127;
+    const int lo = __reduce_min_sync(0xffffffffu, ef), hi = __reduce_max_sync(0xffffffffu, ef);
+    if (lane == 0) {
+      scale_exp[2 * warp] = lo;
+      scale_exp[2 * warp + 1] = hi;
+    }
   }
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -197,6 +223,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     bool ok = true;
     const int r = threadIdx.x >> 3;
     const float2* base = p.B + bz * p.sB + (n0 + r) * p.ldb + 4 * (threadIdx.x & 7);
+    const float* kb = KS && p.kB ? p.kB + ia * p.K : nullptr;
     uint32_t rows = 0;
     float sc[4];
 #pragma unroll
@@ -205,7 +232,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
       if (row < p.N) rows |= 1u << j;
       sc[j] = pow2f(14 - (row < p.N ? fac_exp(p.rmB[bz * p.N + row]) : 14));
     }
-    auto step = [&](FacStaging& st, int it) -> bool {
+    auto step = [&](FacStaging<KS>& st, int it) -> bool {
       const int s = it % ST;
       if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(it / ST) & 1u) ^ 1u)) return false;
       const uint32_t hi = smem_u32(smem + s * kFacStage + kFacTile);
@@ -213,14 +240,14 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&full_b[s]));
-      if (it + ST < nkb) st.load(p, base, rows, (int64_t)(kb_lo + it + ST) * kFacKC);
+      if (it + ST < nkb) st.load(p, base, kb, rows, (int64_t)(kb_lo + it + ST) * kFacKC);
       return true;
     };
-    FacStaging st0;
-    st0.load(p, base, rows, (int64_t)kb_lo * kFacKC);
+    FacStaging<KS> st0;
+    st0.load(p, base, kb, rows, (int64_t)kb_lo * kFacKC);
     if constexpr (ST == 2) {
-      FacStaging st1;
-      if (nkb > 1) st1.load(p, base, rows, (int64_t)(kb_lo + 1) * kFacKC);
+      FacStaging<KS> st1;
+      if (nkb > 1) st1.load(p, base, kb, rows, (int64_t)(kb_lo + 1) * kFacKC);
       for (int it = 0; it < nkb; it += 2) {
         if (!step(st0, it)) { ok = false; break; }
         if (it + 1 < nkb && !step(st1, it + 1)) { ok = false; break; }
@@ -242,6 +269,19 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     // all producers are past their last stage before it is reused
     asm volatile("bar.sync 1, %0;" ::"r"(256) : "memory");
     float mx = 0.f;
+    // The row's power of two.  It multiplies the column's first unless that pair leaves the range of
+    // normal floats, which the result need not: then the smaller one goes onto the sum, then the
+    // larger.
+    const int64_t row = m0 + q * 32 + lane;
+    const float ra = row < p.M ? p.invA[ia * p.M + row] : 1.f;
+    bool plain = true;
+    {
+      const int er = (int)(__float_as_uint(ra) >> 23) - 127;
+#pragma unroll
+      for (int w = 0; w < kFacN / 32; ++w)
+        plain = plain && er + scale_exp[2 * w] >= -126 && er + scale_exp[2 * w + 1] <= 127 - 42;
+      plain = __all_sync(0xffffffffu, plain);
+    }
 #pragma unroll 1
     for (int c0 = 0; c0 < kFacN; c0 += EC) {
       const int col = h * kFacN + c0;  // first real column of this piece
@@ -270,12 +310,17 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
         float4* dst = reinterpret_cast<float4*>(buf + lane * PITCH + j * 32);
 #pragma unroll
         for (int x = 0; x < 4; ++x) {  // four complex columns
-          const float4 f = sc4[x];
-          const float o[8] = {
-              __uint_as_float(v[8 * x]) * f.x,     __uint_as_float(v[8 * x + 1]) * f.x,
-              __uint_as_float(v[8 * x + 2]) * f.y, __uint_as_float(v[8 * x + 3]) * f.y,
-              __uint_as_float(v[8 * x + 4]) * f.z, __uint_as_float(v[8 * x + 5]) * f.z,
-              __uint_as_float(v[8 * x + 6]) * f.w, __uint_as_float(v[8 * x + 7]) * f.w};
+          const float4 f4 = sc4[x];
+          const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+          float o[8];
+          if (plain) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[8 * x + i]) * (f[i / 2] * ra);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              o[i] = __uint_as_float(v[8 * x + i]) * fminf(f[i / 2], ra) * fmaxf(f[i / 2], ra);
+          }
 #pragma unroll
           for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(o[i]));
           dst[2 * x] = make_float4(o[0], o[1], o[2], o[3]);
@@ -301,8 +346,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
       }
       __syncwarp();
     }
-    if (p.rmC && m0 + q * 32 + lane < p.M)
-      atomicMax(p.rmC + bz * p.M + m0 + q * 32 + lane, __float_as_uint(mx));
+    if (p.rmC && row < p.M) atomicMax(p.rmC + bz * p.M + row, __float_as_uint(mx));
   } else if (warp == 8) {
     if (lane == 0) {
       // ---------------- MMA issuer ----------------
@@ -358,10 +402,10 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
   }
 }
 
-template <int ST>
+template <int ST, bool KS>
 __global__ void __launch_bounds__(kFacThreads, 3 - ST) k_tc_fac(const __grid_constant__ FacParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  fac_tile<ST>(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
+  fac_tile<ST, KS>(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
 }
 
 // Products of different sizes in one launch (a group each); the flattened tile index picks the
@@ -370,6 +414,7 @@ struct FacGroupDev {
   FacParams p;
   int64_t tiles, tile_begin;  // tiles per matrix edge
 };
+template <bool KS>
 __global__ void __launch_bounds__(kFacThreads, 1)
     k_tc_fac_grouped(const FacGroupDev* __restrict__ groups, int ngroups) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -391,41 +436,98 @@ __global__ void __launch_bounds__(kFacThreads, 1)
     s_n0 = r % g.tiles * kFacN;
   }
   __syncthreads();
-  fac_tile<2>(sp, s_bz, s_m0, s_n0, smem_raw);
+  fac_tile<2, KS>(sp, s_bz, s_m0, s_n0, smem_raw);
 }
 
-// Largest |re|, |im| of each of the complex128 matrices of n elements (bits of a float, rounded up)
-__global__ void k_fac_max(const double2* __restrict__ L, uint32_t* __restrict__ mx, int64_t n) {
-  const double2* a = L + (int64_t)blockIdx.y * n;
+// Packing a factor: column maxima, the powers of two that level graded columns, row maxima of what
+// remains, then the tiles.  Maxima are the bits of the largest |re|, |im| as a float, rounded up.
+__device__ __forceinline__ float fac_abs(double2 v) {
+  return __double2float_ru(fmax(fabs(v.x), fabs(v.y)));
+}
+// one column per thread, eight rows at a time
+__global__ void __launch_bounds__(256) k_fac_colmax(const double2* __restrict__ L,
+                                                    uint32_t* __restrict__ cm, int64_t M, int64_t K) {
+  __shared__ float red[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int64_t q = blockIdx.y, k = (int64_t)blockIdx.x * 32 + x;
+  const double2* a = L + q * M * K;
   float m = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, __double2float_ru(fmax(fabs(a[i].x), fabs(a[i].y))));
+  if (k < K)
+    for (int64_t r = y; r < M; r += 8) m = fmaxf(m, fac_abs(a[r * K + k]));
+  red[y][x] = m;
+  __syncthreads();
+  if (y == 0 && k < K) {
+    for (int j = 1; j < 8; ++j) m = fmaxf(m, red[j][x]);
+    cm[q * K + k] = __float_as_uint(m);
+  }
+}
+// Columns of a matrix may differ by this power of two and stay as they are: an element that small
+// in its row still has its 22 bits if it is within 2^-12 of the largest of its column.
+constexpr int kFacGrade = 6;
+// cm (bits) -> ks: a column's power of two over the largest one's, 0 for an empty column; *graded is
+// set when two columns of a matrix differ by more than 2^kFacGrade
+__global__ void __launch_bounds__(256) k_fac_kscale(uint32_t* __restrict__ cm, int64_t K,
+                                                    int* __restrict__ graded) {
+  __shared__ int lo, hi;
+  if (threadIdx.x == 0) {
+    lo = 1 << 20;
+    hi = -(1 << 20);
+  }
+  __syncthreads();
+  uint32_t* c = cm + (int64_t)blockIdx.x * K;
+  for (int64_t k = threadIdx.x; k < K; k += blockDim.x)
+    if (c[k]) {
+      const int e = min((int)(c[k] >> 23) - 127, 127);
+      atomicMin(&lo, e);
+      atomicMax(&hi, e);
+    }
+  __syncthreads();
+  for (int64_t k = threadIdx.x; k < K; k += blockDim.x)
+    c[k] = c[k] ? __float_as_uint(pow2f(max(min((int)(c[k] >> 23) - 127, 127) - hi, -100))) : 0u;
+  if (threadIdx.x == 0 && hi - lo > kFacGrade && lo < (1 << 20)) *graded = 1;
+}
+// one warp per row, after division by ks (may be null)
+__global__ void __launch_bounds__(256) k_fac_rowmax(const double2* __restrict__ L,
+                                                    const float* __restrict__ ks,
+                                                    uint32_t* __restrict__ rm, int64_t M, int64_t K) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + threadIdx.x / 32, q = blockIdx.y;
+  if (r >= M) return;
+  const double2* a = L + (q * M + r) * K;
+  float m = 0.f;
+  for (int64_t k = threadIdx.x & 31; k < K; k += 32) {
+    const float d = ks ? ks[q * K + k] : 1.f;
+    if (d > 0.f)
+      m = fmaxf(m, __double2float_ru(fmax(fabs(a[k].x), fabs(a[k].y)) / (double)d));
+  }
   const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-  if ((threadIdx.x & 31) == 0) atomicMax(mx + blockIdx.y, w);
+  if ((threadIdx.x & 31) == 0) rm[q * M + r] = w;
 }
 
 // The packed tiles of a factor: tile (mt, kb) holds rows 128 mt .. and complex K 32 kb .. as a
 // 128 x 64 FP16 hi plane and a lo plane in the swizzled order of shared memory, zeros beyond the
 // matrix.  One thread per 16-byte chunk (four values).
-__global__ void k_fac_pack(const double2* __restrict__ L, const uint32_t* __restrict__ mx,
-                           unsigned char* __restrict__ out, float* __restrict__ inv, int64_t M,
-                           int64_t K, int64_t sA) {
+__global__ void k_fac_pack(const double2* __restrict__ L, const float* __restrict__ ks,
+                           const uint32_t* __restrict__ rm, unsigned char* __restrict__ out,
+                           float* __restrict__ inv, int64_t M, int64_t K, int64_t sA) {
   const int64_t q = blockIdx.y, kbs = (K + kFacKC - 1) / kFacKC;
-  const int e = fac_exp(mx[q]);
-  const double s = (double)pow2f(14 - e);
-  if (blockIdx.x == 0 && threadIdx.x == 0) inv[q] = pow2f(e - 14);
   const double2* a = L + q * M * K;
   const int64_t chunks = (M + kBM - 1) / kBM * kbs * kBM * 8;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < chunks;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i & 7), r = (int)((i >> 3) % kBM);
     const int64_t tile = i / (8 * kBM), m = tile / kbs * kBM + r, k = tile % kbs * kFacKC + 4 * c;
+    const int e = m < M ? fac_exp(rm[q * M + m]) : 14;
+    if (m < M && k == 0) inv[q * M + m] = pow2f(e - 14);
     uint32_t h[4], l[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       double2 v = make_double2(0.0, 0.0);
-      if (m < M && k + j < K) v = a[m * K + k + j];
+      double s = (double)pow2f(14 - e);
+      if (m < M && k + j < K) {
+        const float d = ks ? ks[q * K + k + j] : 1.f;
+        if (d > 0.f) v = a[m * K + k + j];
+        if (d > 0.f) s /= (double)d;
+      }
       const double x = s * v.x, y = s * v.y;
       const __half hx = __double2half(x), hy = __double2half(y);
       const __half lx = __double2half(x - (double)__half2float(hx));
@@ -439,18 +541,30 @@ __global__ void k_fac_pack(const double2* __restrict__ L, const uint32_t* __rest
   }
 }
 
-// Row maxima (bits of the largest |re|, |im|) of a complex64 n-column matrix, one warp per row
-__device__ __forceinline__ void row_max(const float2* __restrict__ a, uint32_t* rm, int64_t n) {
+// Row maxima (bits of the largest |re|, |im|) of a complex64 n-column matrix times ks along the row
+// (may be null), one warp per row
+__device__ __forceinline__ void row_max(const float2* __restrict__ a, const float* __restrict__ ks,
+                                        uint32_t* rm, int64_t n) {
   float m = 0.f;
+  if (ks) {
 #pragma unroll 4
-  for (int64_t i = threadIdx.x & 31; i < n; i += 32) m = fmaxf(m, fmaxf(fabsf(a[i].x), fabsf(a[i].y)));
+    for (int64_t i = threadIdx.x & 31; i < n; i += 32)
+      m = fmaxf(m, ks[i] * fmaxf(fabsf(a[i].x), fabsf(a[i].y)));
+  } else {
+#pragma unroll 4
+    for (int64_t i = threadIdx.x & 31; i < n; i += 32)
+      m = fmaxf(m, fmaxf(fabsf(a[i].x), fabsf(a[i].y)));
+  }
   const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
   if ((threadIdx.x & 31) == 0) *rm = w;
 }
+// row r belongs to problem r / per, which takes the scales (q0 + r / per) % mod
 __global__ void __launch_bounds__(256) k_row_max(const float2* __restrict__ A,
-                                                 uint32_t* __restrict__ rm, int64_t rows, int64_t n) {
+                                                 const float* __restrict__ ks,
+                                                 uint32_t* __restrict__ rm, int64_t rows, int64_t n,
+                                                 int64_t per, int64_t mod, int64_t q0) {
   const int64_t r = (int64_t)blockIdx.x * 8 + threadIdx.x / 32;
-  if (r < rows) row_max(A + r * n, rm + r, n);
+  if (r < rows) row_max(A + r * n, ks ? ks + (q0 + r / per) % mod * n : nullptr, rm + r, n);
 }
 // the same for matrices of different sizes: group g has `batch` matrices of n rows, sA apart
 __global__ void __launch_bounds__(256) k_row_max_grouped(const TcRowMaxGroup* __restrict__ groups,
@@ -464,5 +578,5 @@ __global__ void __launch_bounds__(256) k_row_max_grouped(const TcRowMaxGroup* __
   }
   const TcRowMaxGroup g = groups[lo];
   const int64_t l = r - g.row_begin;
-  if (l < g.n * g.batch) row_max(g.A + l / g.n * g.sA + l % g.n * g.n, g.rm + l, g.n);
+  if (l < g.n * g.batch) row_max(g.A + l / g.n * g.sA + l % g.n * g.n, g.ks, g.rm + l, g.n);
 }

@@ -1161,20 +1161,58 @@ int tc_take_flags(int mask) {
 // ---------------------------------------------------------------------------------------
 // factor products (tc_fac.cuh)
 // ---------------------------------------------------------------------------------------
-void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, cudaStream_t s) {
+void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, bool level_k,
+                    cudaStream_t s) {
   CQ_REQUIRE(nmat <= 65535, COQUI_B200_EUNSUPPORTED, "tc_pack_matrix: too many matrices");
   f.M = M;
   f.K = K;
   f.stride = (M + kBM - 1) / kBM * ((K + kFacKC - 1) / kFacKC) * kFacTile;
   f.packed.ensure((size_t)nmat * f.stride);
-  f.inv.ensure(nmat);
-  f.mx.ensure(nmat);
-  CQ_CHECK_CUDA(cudaMemsetAsync(f.mx.p, 0, nmat * sizeof(uint32_t), s));
+  f.inv.ensure((size_t)nmat * M);
+  f.mx.ensure((size_t)nmat * M);
+  f.graded = false;
+  if (level_k) {
+    f.ks.ensure((size_t)nmat * K);
+    f.flag.ensure(1);
+    CQ_CHECK_CUDA(cudaMemsetAsync(f.flag.p, 0, sizeof(int), s));
+    uint32_t* cm = reinterpret_cast<uint32_t*>(f.ks.p);
+    k_fac_colmax<<<dim3((unsigned)((K + 31) / 32), (unsigned)nmat), 256, 0, s>>>(L, cm, M, K);
+    k_fac_kscale<<<(unsigned)nmat, 256, 0, s>>>(cm, K, f.flag.p);
+    count_launch(2);
+    CQ_CHECK_CUDA(cudaGetLastError());
+    int flag = 0;
+    CQ_CHECK_CUDA(cudaMemcpyAsync(&flag, f.flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CQ_CHECK_CUDA(cudaStreamSynchronize(s));
+    f.graded = flag != 0;
+  }
+  const float* ks = f.graded ? f.ks.p : nullptr;
   const unsigned g = grid_for(M * K, 256, 64);
-  k_fac_max<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, f.mx.p, M * K);
-  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, f.mx.p, f.packed.p, f.inv.p, M, K, f.stride);
+  k_fac_rowmax<<<dim3((unsigned)((M + 7) / 8), (unsigned)nmat), 256, 0, s>>>(L, ks, f.mx.p, M, K);
+  k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, ks, f.mx.p, f.packed.p, f.inv.p, M, K,
+                                                     f.stride);
   count_launch(2);
   CQ_CHECK_CUDA(cudaGetLastError());
+}
+
+void tc_gather_matrices(TcFactor& dst, const TcFactor& src, const std::vector<int64_t>& idx,
+                        cudaStream_t s) {
+  const int64_t n = (int64_t)idx.size();
+  dst.M = src.M;
+  dst.K = src.K;
+  dst.stride = src.stride;
+  dst.graded = src.graded;
+  dst.packed.ensure((size_t)n * src.stride);
+  dst.inv.ensure((size_t)n * src.M);
+  if (src.graded) dst.ks.ensure((size_t)n * src.K);
+  for (int64_t i = 0; i < n; ++i) {
+    CQ_CHECK_CUDA(cudaMemcpyAsync(dst.packed.p + i * src.stride, src.packed.p + idx[i] * src.stride,
+                                  src.stride, cudaMemcpyDeviceToDevice, s));
+    CQ_CHECK_CUDA(cudaMemcpyAsync(dst.inv.p + i * src.M, src.inv.p + idx[i] * src.M,
+                                  src.M * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    if (src.graded)
+      CQ_CHECK_CUDA(cudaMemcpyAsync(dst.ks.p + i * src.K, src.ks.p + idx[i] * src.K,
+                                    src.K * sizeof(float), cudaMemcpyDeviceToDevice, s));
+  }
 }
 
 namespace {
@@ -1183,12 +1221,15 @@ void fac_smem_attr() {
   int dev = 0;
   CQ_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && set[dev]) return;
-  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     fac_smem<1>()));
-  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     fac_smem<2>()));
-  CQ_CHECK_CUDA(cudaFuncSetAttribute(k_tc_fac_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     fac_smem<2>()));
+  auto attr = [](const void* f, int bytes) {
+    CQ_CHECK_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  };
+  attr((const void*)k_tc_fac<1, false>, fac_smem<1>());
+  attr((const void*)k_tc_fac<1, true>, fac_smem<1>());
+  attr((const void*)k_tc_fac<2, false>, fac_smem<2>());
+  attr((const void*)k_tc_fac<2, true>, fac_smem<2>());
+  attr((const void*)k_tc_fac_grouped<false>, fac_smem<2>());
+  attr((const void*)k_tc_fac_grouped<true>, fac_smem<2>());
   if (dev < 64) set[dev] = true;
 }
 }  // namespace
@@ -1202,9 +1243,13 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
                    [](const TcFactorGroup& x, const TcFactorGroup& y) { return x.f.K > y.f.K; });
   std::vector<FacGroupDev> h;
   int64_t total = 0;
+  bool scaled = false;
   for (const TcFactorGroup& g : order) {
     const int64_t n = g.f.K;
     FacGroupDev d;
+    d.p.kB = g.b_has_ks ? nullptr : g.f.ks;
+    d.p.nC = g.ks_c ? g.f.ks : nullptr;
+    scaled = scaled || d.p.kB;
     d.p.A = g.f.packed;
     d.p.sA = 0;
     d.p.a_mod = 1;
@@ -1232,8 +1277,8 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
   table.ensure(h.size() * sizeof(FacGroupDev));
   CQ_CHECK_CUDA(cudaMemcpyAsync(table.p, h.data(), h.size() * sizeof(FacGroupDev),
                                 cudaMemcpyHostToDevice, s));
-  k_tc_fac_grouped<<<(unsigned)total, kFacThreads, fac_smem<2>(), s>>>((const FacGroupDev*)table.p,
-                                                                  (int)h.size());
+  auto fn = scaled ? k_tc_fac_grouped<true> : k_tc_fac_grouped<false>;
+  fn<<<(unsigned)total, kFacThreads, fac_smem<2>(), s>>>((const FacGroupDev*)table.p, (int)h.size());
   count_launch();
   CQ_CHECK_CUDA(cudaGetLastError());
 }
@@ -1258,8 +1303,12 @@ void tc_row_max_grouped(std::vector<TcRowMaxGroup> groups, DevBuf<unsigned char>
 
 void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, const float2* Bt,
                        bool conj_b, int64_t N, const uint32_t* row_max, float2* C,
-                       uint32_t* out_max, int half, int64_t batch, cudaStream_t s) {
+                       uint32_t* out_max, int half, int64_t batch, cudaStream_t s, bool b_has_ks,
+                       bool ks_c) {
+  CQ_REQUIRE(!ks_c || N == f.K, COQUI_B200_EINVAL, "tc_packed_product: scales of C");
   FacParams p;
+  p.kB = b_has_ks ? nullptr : f.ks;
+  p.nC = ks_c ? f.ks : nullptr;
   p.A = f.packed;
   p.sA = f.stride;
   p.invA = f.inv;
@@ -1287,18 +1336,23 @@ void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, 
     // one stage and two CTAs per SM while a tile has few K blocks: M products of 30 q at N_mu 203
     // 0.504 against 0.516 ms, of 32 at 256 0.563 against 0.591; at 384 1.14 against 1.11 and at
     // 1024 12.6 against 11.4 ms two stages are ahead
-    if (p.K <= 256)
-      k_tc_fac<1><<<dim3(tn, tm, nb), kFacThreads, fac_smem<1>(), s>>>(p);
-    else
-      k_tc_fac<2><<<dim3(tn, tm, nb), kFacThreads, fac_smem<2>(), s>>>(p);
+    const dim3 grid(tn, tm, nb);
+    if (p.K <= 256) {
+      auto fn = p.kB ? k_tc_fac<1, true> : k_tc_fac<1, false>;
+      fn<<<grid, kFacThreads, fac_smem<1>(), s>>>(p);
+    } else {
+      auto fn = p.kB ? k_tc_fac<2, true> : k_tc_fac<2, false>;
+      fn<<<grid, kFacThreads, fac_smem<2>(), s>>>(p);
+    }
     count_launch();
     CQ_CHECK_CUDA(cudaGetLastError());
   }
 }
 
-void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s) {
+void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s,
+                const float* ks, int64_t per, int64_t mod, int64_t q0) {
   CQ_REQUIRE(rows <= (int64_t)8 * 2147483647, COQUI_B200_EUNSUPPORTED, "tc_row_max: too many rows");
-  k_row_max<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(A, rm, rows, n);
+  k_row_max<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(A, ks, rm, rows, n, per, mod, q0);
   count_launch();
   CQ_CHECK_CUDA(cudaGetLastError());
 }
@@ -1422,7 +1476,7 @@ void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t 
   float2* Xc = (float2*)op.packed.p;
   to_c64(X, Xc, Np, nb, nk, false, s);                 // X   (nk, Np, nb)
   to_c64(X, Xc + nk * Np * nb, Np, nb, nk, true, s);   // X^T (nk, nb, Np)
-  if (packed_projection(Np, nb)) tc_pack_matrix(op.Xp, X, Np, nb, nk, s);
+  if (packed_projection(Np, nb)) tc_pack_matrix(op.Xp, X, Np, nb, nk, true, s);
 }
 
 void tc_project_p2a(TcOperand& op, const double2* Gk, float2* out, int64_t nk, int64_t Np,
@@ -1444,8 +1498,9 @@ void tc_project_p2a(TcOperand& op, const double2* Gk, float2* out, int64_t nk, i
     CQ_CHECK_CUDA(cudaGetLastError());
     tc_cgemm_nt(Xs, false, true, nb, Np * nb, Gt, false, false, nb, nb * nb, T, nb, Np * nb, Np, nb,
                 nb, nbatch, s, sx_a);
-    tc_row_max(T, op.rm.p, nbatch * Np, nb, s);
-    tc_packed_product(op.Xp.view(), 0, nk, 0, T, false, Np, op.rm.p, out, nullptr, 0, nbatch, s);
+    const TcFactorView x = op.Xp.view();
+    tc_row_max(T, op.rm.p, nbatch * Np, nb, s, x.ks, Np, nk);
+    tc_packed_product(x, 0, nk, 0, T, false, Np, op.rm.p, out, nullptr, 0, nbatch, s);
     return;
   }
   k_transpose_c64<<<grid_for(tg, 256), 256, 0, s>>>(Gk, Gt, nb, nb, tg);

@@ -8,23 +8,35 @@ namespace cq {
 // Matrices A (M x K) packed for tc_packed_product (split FP16 tiles, tc_fac.cuh).
 struct TcFactorView {
   const unsigned char* packed = nullptr;  // matrices `stride` bytes apart
-  const float* inv = nullptr;             // 1 / scale of each
+  const float* inv = nullptr;             // 1 / scale of each row, (nmat, M)
+  const float* ks = nullptr;              // graded columns only: their powers of two, (nmat, K)
   int64_t M = 0, K = 0, stride = 0;
 };
 struct TcFactor {
   DevBuf<unsigned char> packed;
   DevBuf<float> inv;
-  DevBuf<uint32_t> mx;  // largest element of each, kept for the next packing
+  DevBuf<float> ks;
+  DevBuf<uint32_t> mx;  // row maxima, kept for the next packing
+  DevBuf<int> flag;
+  bool graded = false;
   int64_t M = 0, K = 0, stride = 0;
-  TcFactorView view() const { return {packed.p, inv.p, M, K, stride}; }
+  TcFactorView view() const { return {packed.p, inv.p, graded ? ks.p : nullptr, M, K, stride}; }
   void release() {
     packed.release();
     inv.release();
+    ks.release();
     mx.release();
+    flag.release();
   }
 };
-// nmat row-major complex128 matrices
-void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, cudaStream_t s);
+// nmat row-major complex128 matrices; level_k: columns that differ by more than 2^6 are brought to
+// one size (asks the device, and waits for the answer), for a product whose Bt carries the inverse
+// grading along K
+void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, bool level_k,
+                    cudaStream_t s);
+// dst = the matrices idx of src
+void tc_gather_matrices(TcFactor& dst, const TcFactor& src, const std::vector<int64_t>& idx,
+                        cudaStream_t s);
 
 // C[b](m, n) = sum_k A(m, k) opB(Bt[b])(n, k) for b < batch: A the packed matrix (q0 + b) % mod,
 // upper (tri > 0: k >= m) or lower (tri < 0: k <= m) triangular or full; Bt (N x K) and C (M x N)
@@ -32,9 +44,13 @@ void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t
 // Bt (bits of the largest |re|, |im| as float, (batch, N)); those of C are raised in out_max
 // ((batch, M), may be null).  half < 0: only the 128 x 128 tiles on or below the diagonal are formed
 // and written, half > 0: on or above it.
+// Of a factor with levelled columns Bt is multiplied by ks along K; row_max is then that of the
+// multiplied Bt (tc_row_max with ks).  b_has_ks: Bt was written with it already.  ks_c: C's columns
+// (N = K of them) are written multiplied by ks, for a next product with the same factor.
 void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, const float2* Bt,
                        bool conj_b, int64_t N, const uint32_t* row_max, float2* C,
-                       uint32_t* out_max, int half, int64_t batch, cudaStream_t s);
+                       uint32_t* out_max, int half, int64_t batch, cudaStream_t s,
+                       bool b_has_ks = false, bool ks_c = false);
 
 // THC collocation X (nk, Np, nb) prepared for the projection GEMMs.
 struct TcOperand {
@@ -105,8 +121,8 @@ void tc_cgemm_nt(const void* A, bool a_split, bool conj_a, int64_t lda, int64_t 
                  const TcStructure& st = TcStructure{});
 
 // Products of square triangular factors (M = N = K) of different sizes in one launch; a group's Bt
-// and C hold `batch` matrices
-// sB and sC elements apart, all with one factor.  table: device copy of the descriptors.
+// and C hold `batch` matrices sB and sC elements apart, all with one factor.  table: device copy of
+// the descriptors.
 struct TcFactorGroup {
   TcFactorView f;
   bool upper = false, conj_b = false;
@@ -118,6 +134,7 @@ struct TcFactorGroup {
   uint32_t* out_max = nullptr;
   int half = 0;
   int64_t batch = 1;
+  bool b_has_ks = false, ks_c = false;
 };
 void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned char>& table,
                        cudaStream_t s);
@@ -126,12 +143,15 @@ struct TcRowMaxGroup {
   const float2* A;
   int64_t n, sA, batch;
   uint32_t* rm;
+  const float* ks;    // along each row; may be null
   int64_t row_begin;  // filled in by the call
 };
 void tc_row_max_grouped(std::vector<TcRowMaxGroup> groups, DevBuf<unsigned char>& table,
                         cudaStream_t s);
-// Row maxima of a (rows, n) complex64 array, as tc_packed_product reads them.
-void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s);
+// Row maxima of a (rows, n) complex64 array, as tc_packed_product reads them; ks (mod, n) along each
+// row (may be null), `per` rows to a problem and problem b with the scales (q0 + b) % mod.
+void tc_row_max(const float2* A, uint32_t* rm, int64_t rows, int64_t n, cudaStream_t s,
+                const float* ks = nullptr, int64_t per = 1, int64_t mod = 1, int64_t q0 = 0);
 
 // One group of a grouped product: a batched "NT" product as tc_cgemm_nt describes.
 struct TcGroup {
