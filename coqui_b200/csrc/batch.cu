@@ -97,6 +97,8 @@ struct coqui_b200_batch {
   DevBuf<unsigned char> gtab, ctab, ctab2, htab;
   std::vector<int64_t> chol_perm;  // factorisation list position -> (molecule, iW) problem
   DevBuf<int> info;
+  int* info_host = nullptr;        // page-locked: read back behind the factorisations
+  cudaEvent_t info_ev = nullptr;
   DevBuf<double> ld;
   DevBuf<double2> tr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -318,6 +320,9 @@ void batch_gw(Batch* b, const double* const* G_list, double* const* Sigma_list) 
   } else {
     cq::launch_chol_inv_grouped(cp, b->ctab, b->ld.p, b->tr.p, b->info.p, s, true);
   }
+  CQ_CHECK_CUDA(cudaMemcpyAsync(b->info_host, b->info.p, nprob * sizeof(int),
+                                cudaMemcpyDeviceToHost, s));
+  CQ_CHECK_CUDA(cudaEventRecord(b->info_ev, s));
   for (int64_t m = 0; m < b->nmol; ++m)
     cq::launch_chol_split(b->Ab.p + b->offD[m], b->Zb.p + b->offD[m], b->Zl.p + b->offD[m],
                           b->T1.p + b->offD[m], b->Np[m], nwh, s);
@@ -431,6 +436,13 @@ void batch_gw(Batch* b, const double* const* G_list, double* const* Sigma_list) 
     CQ_CHECK_CUDA(cudaEventRecord(b->s_out[h], s));
   }
   CQ_CHECK_CUDA(cudaEventRecord(b->ev1, s));
+  // the caller's arrays are written only when every factorisation has succeeded; all kernels are
+  // queued by now, so that the GPU works on while the host looks
+  CQ_CHECK_CUDA(cudaEventSynchronize(b->info_ev));
+  for (int64_t i = 0; i < nprob; ++i)
+    CQ_REQUIRE(b->info_host[i] == 0, COQUI_B200_ENOTHPD,
+               "I - L^H Pi L is not positive definite (problem " +
+                   std::to_string(b->chol_perm[i]) + ")");
   for (int h = 0; h < 2 && Sigma_list; ++h) {
     CQ_CHECK_CUDA(cudaStreamWaitEvent(b->st2, b->s_out[h], 0));
     for (int64_t m = from[h]; m < from[h + 1]; ++m)
@@ -439,14 +451,7 @@ void batch_gw(Batch* b, const double* const* G_list, double* const* Sigma_list) 
                                       (goff(m + 1) - goff(m)) * sizeof(double2),
                                       cudaMemcpyDeviceToHost, b->st2));
   }
-  // factorisation status
-  std::vector<int> info(nprob);
-  CQ_CHECK_CUDA(cudaMemcpyAsync(info.data(), b->info.p, nprob * sizeof(int), cudaMemcpyDeviceToHost, s));
   CQ_CHECK_CUDA(cudaStreamSynchronize(s));
-  for (int64_t i = 0; i < nprob; ++i)
-    CQ_REQUIRE(info[i] == 0, COQUI_B200_ENOTHPD,
-               "I - L^H Pi L is not positive definite (problem " +
-                   std::to_string(b->chol_perm[i]) + ")");
 }
 
 }  // namespace
@@ -475,6 +480,7 @@ int coqui_b200_batch_create(coqui_b200_batch** out, int64_t nmol, const int64_t*
       CQ_CHECK_CUDA(cudaEventCreateWithFlags(&b->g_in[h], cudaEventDisableTiming));
       CQ_CHECK_CUDA(cudaEventCreateWithFlags(&b->s_out[h], cudaEventDisableTiming));
     }
+    CQ_CHECK_CUDA(cudaEventCreateWithFlags(&b->info_ev, cudaEventDisableTiming));
     CQ_CHECK_CUDA(cudaEventCreate(&b->ev0));
     CQ_CHECK_CUDA(cudaEventCreate(&b->ev1));
     b->nmol = nmol;
@@ -522,6 +528,8 @@ int coqui_b200_batch_create(coqui_b200_batch** out, int64_t nmol, const int64_t*
     b->Ab.ensure(b->nD);
     b->rm0.ensure(b->nR);
     b->rm1.ensure(b->nR);
+    CQ_CHECK_CUDA(cudaHostAlloc((void**)&b->info_host, nmol * b->nwh * sizeof(int),
+                                cudaHostAllocDefault));
     std::vector<int64_t> offs(b->offG);
     b->dofG.ensure(nmol);
     b->dnb.ensure(nmol);
@@ -548,6 +556,8 @@ void coqui_b200_batch_destroy(coqui_b200_batch* b) {
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->join) cudaEventDestroy(b->join);
+  if (b->info_ev) cudaEventDestroy(b->info_ev);
+  if (b->info_host) cudaFreeHost(b->info_host);
   for (cudaEvent_t e : {b->g_in[0], b->g_in[1], b->s_out[0], b->s_out[1]})
     if (e) cudaEventDestroy(e);
   delete b;

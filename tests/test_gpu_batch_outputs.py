@@ -1,0 +1,50 @@
+"""What the batched iteration leaves: Sigma arrays stay as they were when a molecule's dielectric
+matrix is not positive definite."""
+import numpy as np
+import pytest
+
+from coqui_b200 import capi
+from coqui_b200.iaft import IAFT
+from coqui_b200.synthetic import make_system
+
+pytestmark = pytest.mark.gpu
+
+ENOTHPD = -5
+FT = IAFT(500.0, 20.0, "low")
+
+
+def batch(mols):
+    b = capi.Batch([m.nb for m in mols], [m.Np for m in mols], FT.nt_f, FT.nw_b)
+    b.set_ir(FT)
+    for i, m in enumerate(mols):
+        b.set_thc(i, m.X[0, 0], m.V[0])
+    return b
+
+
+def pinned(a):
+    import torch
+    h = torch.empty(a.shape, dtype=torch.complex128, pin_memory=True).numpy()
+    h[...] = a
+    return h
+
+
+@pytest.mark.parametrize("bad", [0, 1, 2])
+@pytest.mark.parametrize("page_locked", [False, True])
+def test_sigma_is_untouched_when_a_molecule_is_not_positive_definite(bad, page_locked):
+    mols = [make_system(1, nb, nb // 2, Np, beta=500.0, seed=nb, gamma_only=True)
+            for nb, Np in ((8, 48), (12, 150), (6, 36))]
+    b = batch(mols)
+    Gs = [m.G0(FT)[:, 0, 0] for m in mols]
+    wrong = [G.copy() for G in Gs]
+    wrong[bad][FT.nt_f // 2:] *= -1e4  # Pi(tau) = -2 G(tau) G(beta - tau)* changes its sign
+    out = [np.full(G.shape, 7.0 + 3.0j) for G in Gs]
+    if page_locked:
+        out = [pinned(S) for S in out]
+    with pytest.raises(capi.CoquiB200Error) as e:
+        b.gw_iteration(wrong, out)
+    assert e.value.code == ENOTHPD
+    assert all(np.all(S == 7.0 + 3.0j) for S in out)
+    ref = b.gw_iteration(Gs)
+    b.gw_iteration(Gs, out)
+    assert all(np.array_equal(S, R) for S, R in zip(out, ref))
+    b.close()
