@@ -298,7 +298,8 @@ COQUI_B200_API int coqui_b200_batch_create(coqui_b200_batch** batch, int64_t nmo
                                            int64_t nw_b, int device);
 COQUI_B200_API void coqui_b200_batch_destroy(coqui_b200_batch* batch);
 COQUI_B200_API const char* coqui_b200_batch_last_error(const coqui_b200_batch* batch);
-/* Device time (CUDA events on the batch's stream) of the last batch GW iteration, ms. */
+/* Device time (CUDA events on the batch's stream) of the last batch GW iteration, ms, without the
+   time the stream waited for host arrays to cross the bus. */
 COQUI_B200_API double coqui_b200_batch_last_ms(const coqui_b200_batch* batch);
 /* Shared bosonic IR tables as for coqui_b200_set_ir (Twt_bb (nw_b, nt_f), Ttw_bb (nt_f, nw_b),
    tau_mesh_x (nt_f)). */
