@@ -237,17 +237,24 @@ void gemm_tt(const float* A, int64_t lda, const TB* B, int64_t ldb, float* C, in
   CQ_CHECK_CUDA(cudaGetLastError());
 }
 
+// Slices that the K of an M x N weight gradient is cut into (1: not cut): at least 256 long, two
+// blocks of 128 x 128 outputs per SM.
+constexpr int64_t kSms = 148;
+int64_t gemm_slices(int64_t M, int64_t N, int64_t K) {
+  const int64_t t128 = ((M + 127) / 128) * ((N + 127) / 128);
+  return std::min((K + 255) / 256, (2 * kSms + t128 - 1) / t128);
+}
+
 // Tiles of 128 x 128 when they fill the GPU, else 64 x 64.  A weight gradient has few tiles and
-// a long K (the batch): its K is cut into slices (at least 256 long, two blocks per SM), whose
-// partial sums go through `part` and are added in slice order.
+// a long K (the batch): the partial sums of its slices go through `part` and are added in slice
+// order.
 template <typename TB, int EPI, bool AK, bool BK>
 void gemm(const float* A, int64_t lda, const TB* B, int64_t ldb, float* C, int64_t ldc, int64_t M,
           int64_t N, int64_t K, const TB* bias, const float* aux, DevBuf<float>& part,
           cudaStream_t s) {
-  const int64_t sms = 148;
   const int64_t t128 = ((M + 127) / 128) * ((N + 127) / 128);
   if constexpr (EPI == kStore) {
-    const int64_t slices = std::min((K + 255) / 256, (2 * sms + t128 - 1) / t128);
+    const int64_t slices = gemm_slices(M, N, K);
     if (slices > 1) {
       const int64_t kslice = ((K + slices - 1) / slices + TK - 1) / TK * TK;
       const int64_t nz = (K + kslice - 1) / kslice;
@@ -258,7 +265,7 @@ void gemm(const float* A, int64_t lda, const TB* B, int64_t ldb, float* C, int64
       return;
     }
   }
-  if (t128 >= sms)
+  if (t128 >= kSms)
     gemm_tt<128, TB, EPI, AK, BK>(A, lda, B, ldb, C, ldc, M, N, K, 1, K, bias, aux, s);
   else
     gemm_tt<64, TB, EPI, AK, BK>(A, lda, B, ldb, C, ldc, M, N, K, 1, K, bias, aux, s);
@@ -273,9 +280,10 @@ __global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ A, int
     part[blockIdx.x * cols + c] = sum;
   }
 }
+int64_t colsum_blocks(int64_t rows) { return std::min<int64_t>(rows, 296); }
 void colsum(const float* A, int64_t rows, int64_t cols, float* out, DevBuf<float>& part,
             cudaStream_t s) {
-  const int64_t blocks = std::min<int64_t>(rows, 296);
+  const int64_t blocks = colsum_blocks(rows);
   part.ensure(blocks * cols);
   k_colsum<<<(unsigned)blocks, 256, 0, s>>>(A, rows, cols, part.p);
   count_launch();
@@ -575,7 +583,8 @@ static void launch_out(Mlp& n, const float* t, int64_t B, float* y, unsigned blo
   count_launch();
   CQ_CHECK_CUDA(cudaGetLastError());
 }
-static unsigned out_blocks(int64_t B) { return (unsigned)std::min<int64_t>(148, (B + 15) / 16); }
+static int64_t out_blocks(int64_t B) { return std::min<int64_t>(148, (B + 15) / 16); }
+static int64_t in_blocks(int64_t B) { return std::min<int64_t>(592, (B + 15) / 16); }
 
 // h1, h2 of a batch
 static void mlp_hidden(Mlp& n, const float* x, int64_t B, cudaStream_t s) {
@@ -593,7 +602,7 @@ void mlp_forward(Mlp& n, const float* x, int64_t B, float* y, cudaStream_t s) {
   const int64_t H = n.width;
   mlp_hidden(n, x, B, s);
   if (fused_out(n))
-    launch_out<false>(n, nullptr, B, y, out_blocks(B), s);
+    launch_out<false>(n, nullptr, B, y, (unsigned)out_blocks(B), s);
   else
     gemm<__nv_bfloat16, kBias, true, true>(n.h2.p, H, W + n.oW3(), H, y, n.dout, B, n.dout, H,
                                            W + n.ob3(), nullptr, n.part, s);
@@ -614,12 +623,14 @@ float mlp_backward(Mlp& n, const float* x, const float* t, int64_t B, cudaStream
   // one workspace for every split reduction below (growing it step by step would free and
   // allocate between the kernels of a first call): the widest weight gradient's slices, the
   // output layer's and the input layer's block sums
-  const int64_t widest = std::max({H * H, H * n.din, H * D});
-  n.part.ensure(std::max({(2 * 148 + (H * H + 16383) / 16384) * widest / std::max<int64_t>(1, (H * H) / 16384),
-                          148 * (D * H + H + D + 1), 592 * (H * std::min<int64_t>(n.din, 8) + H)}));
+  auto slices = [&](int64_t M, int64_t N) { return gemm_slices(M, N, B) * M * N; };
+  n.part.ensure(std::max({slices(H, H),
+                          n.din <= 8 ? in_blocks(B) * (H * n.din + H) : slices(H, n.din),
+                          fused_out(n) ? out_blocks(B) * (D * H + H + D + 1) : slices(D, H),
+                          colsum_blocks(B) * std::max(H, D)}));
   if (fused_out(n)) {
     mlp_hidden(n, x, B, s);
-    const unsigned blocks = out_blocks(B);
+    const unsigned blocks = (unsigned)out_blocks(B);
     const int64_t np = D * H + H + D + 1;
     n.part.ensure(blocks * np);
     launch_out<true>(n, t, B, nullptr, blocks, s);
@@ -654,7 +665,7 @@ float mlp_backward(Mlp& n, const float* x, const float* t, int64_t B, cudaStream
                                               nullptr, n.h1.p, n.part, s);
   // dW1 = dz1^T x, db1 = colsum(dz1)
   if (n.din <= 8) {
-    const unsigned blocks = (unsigned)std::min<int64_t>(592, (B + 15) / 16);
+    const unsigned blocks = (unsigned)in_blocks(B);
     const int64_t np = H * n.din + H;  // W1 and b1 follow each other
     n.part.ensure(blocks * np);
     k_mlp_in_grad<<<blocks, 256, 0, s>>>(n.dh1.p, x, B, (int)H, (int)n.din, n.part.p);

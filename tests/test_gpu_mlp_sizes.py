@@ -32,3 +32,30 @@ def test_loss_gradient_and_forward(din, width, dout, batch):
         assert np.abs(g - g_ref).max() < 2e-5 * np.abs(g_ref).max()
         assert np.abs(net.forward(X) - Y_ref).max() < 1e-5 * max(1.0, np.abs(Y_ref).max())
     net.close()
+
+
+@pytest.mark.parametrize("din,width,dout", [(4096, 64, 2), (4, 64, 6000)])
+def test_workspace_follows_the_slices_in_use(din, width, dout):
+    """The widest weight gradient is cut into few slices when the batch is small: the workspace is
+    a few copies of it and not one per block the GPU could run."""
+    import torch
+    batch = 1000
+    rng = np.random.default_rng(din)
+    X = rng.standard_normal((batch, din)).astype(np.float32)
+    T = rng.standard_normal((batch, dout)).astype(np.float32)
+    warm = capi.Mlp(din, width, dout, seed=1)
+    warm.gradient(X[:10], T[:10])  # the kernels are on the device
+    warm.close()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    net = capi.Mlp(din, width, dout, seed=11)
+    loss, g = net.gradient(X, T)
+    used = free0 - torch.cuda.mem_get_info()[0]
+    loss_ref, g_ref = M.loss_and_grad(net.params(), X, T, din, width, dout)
+    assert abs(loss - loss_ref) < 1e-5 * loss_ref
+    assert np.abs(g - g_ref).max() < 2e-5 * np.abs(g_ref).max()
+    # parameters and optimiser state (about 8 copies), inputs and activations, 4 slices per gradient
+    # of 256-long K, and the 2 MB blocks of the allocator
+    need = 4 * (16 * net.nparam + 2 * batch * (din + 4 * width + 3 * dout)) + (64 << 20)
+    assert used < need, (used, need)
+    net.close()
