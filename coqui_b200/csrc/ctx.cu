@@ -259,9 +259,9 @@ template <typename F> int guarded(Ctx* c, F&& f) {
     f();
     if (c->st) CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));
     if (c->cs) CQ_CHECK_CUDA(cudaStreamSynchronize(c->cs));
-    const int flags = cq::tc_take_flags(cq::kTcNonfinite | cq::kTcTimeout);
-    if (flags & cq::kTcNonfinite) throw Error(COQUI_B200_EINVAL, "G holds NaN or Inf values");
-    if (flags & cq::kTcTimeout)
+    const int flag = cq::tc_take_flags(cq::kTcNonfinite | cq::kTcTimeout);
+    if (flag == cq::kTcNonfinite) throw Error(COQUI_B200_EINVAL, "G holds NaN or Inf values");
+    if (flag == cq::kTcTimeout)
       throw Error(COQUI_B200_ETIMEDOUT, "a tensor-core kernel gave up a bounded wait");
     c->err.clear();
     return COQUI_B200_OK;

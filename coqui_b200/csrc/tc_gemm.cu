@@ -1149,13 +1149,12 @@ int tc_take_flags(int mask) {
   int h[2] = {0, 0};
   const int z = 0, bit[2] = {kTcTimeout, kTcNonfinite};
   CQ_CHECK_CUDA(cudaMemcpyFromSymbol(h, g_flags, sizeof(h)));
-  int got = 0;
-  for (int i = 0; i < 2; ++i)
+  for (int i = 1; i >= 0; --i)
     if (h[i] && (mask & bit[i])) {
       CQ_CHECK_CUDA(cudaMemcpyToSymbol(g_flags, &z, sizeof(int), i * sizeof(int)));
-      got |= bit[i];
+      return bit[i];
     }
-  return got;
+  return 0;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -180,8 +180,9 @@ int64_t tc_tuned_shapes();
 bool tc_set_forced_cfg(int cfg);
 int tc_num_cfgs();
 
-// What tensor-core kernels reported since the last call, of the kinds in `mask`, read and cleared:
-// a bounded wait was given up; a primary -> auxiliary projection saw NaN or Inf in G.
+// What tensor-core kernels reported, of the kinds in `mask`: a bounded wait was given up; a primary ->
+// auxiliary projection saw NaN or Inf in G.  Returns and clears one kind, the input's first; the
+// other stays for the next call.
 constexpr int kTcTimeout = 1, kTcNonfinite = 2;
 int tc_take_flags(int mask);
 // Time limit of the tensor-core kernels' bounded waits on the current device (ns; <= 0: the

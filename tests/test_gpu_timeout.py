@@ -50,3 +50,31 @@ def test_wait_runs_out_and_context_recovers(case, cfg):
         capi.set_wait_limit_ns(0)
         capi.set_tile_config(-1)
         c.close()
+
+
+def test_a_wait_that_ran_out_is_reported_after_a_refused_input(case):
+    """A call that meets a non-finite input and a wait that runs out reports the input; the wait is
+    reported by the next call and not lost."""
+    s, ft, G = case
+    c = capi.Context(s.nk, s.nb, s.Np, ft.nt_f, ft.nw_b, s.kp_grid, mode=capi.MIXED)
+    try:
+        c.set_ir(ft)
+        c.set_kmesh(s.kpts, s.lattv, s.chi_bar)
+        c.set_thc(s.X, s.V)
+        capi.set_tile_config(0)
+        ref = c.primary_to_aux(G)
+        bad = G.copy()
+        bad[0, 0, 0, 1, 1] = np.nan
+        capi.set_wait_limit_ns(1)
+        with pytest.raises(capi.CoquiB200Error) as err:
+            c.primary_to_aux(bad)
+        assert err.value.code == -1
+        capi.set_wait_limit_ns(0)
+        with pytest.raises(capi.CoquiB200Error) as err:
+            c.primary_to_aux(G)
+        assert err.value.code == ETIMEDOUT
+        assert np.array_equal(c.primary_to_aux(G), ref)
+    finally:
+        capi.set_wait_limit_ns(0)
+        capi.set_tile_config(-1)
+        c.close()
