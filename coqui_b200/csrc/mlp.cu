@@ -519,6 +519,7 @@ __global__ void k_extrap_apply(const double2* __restrict__ h, int64_t nel, const
 
 void ensure_batch(Mlp& n, int64_t B) {
   if (B <= n.cap) return;
+  n.cap = 0;  // an allocation that fails leaves a buffer empty
   n.x.ensure(B * n.din);
   n.t.ensure(B * n.dout);
   n.h1.ensure(B * n.width);

@@ -59,3 +59,28 @@ def test_workspace_follows_the_slices_in_use(din, width, dout):
     need = 4 * (16 * net.nparam + 2 * batch * (din + 4 * width + 3 * dout)) + (64 << 20)
     assert used < need, (used, need)
     net.close()
+
+
+def test_a_batch_that_did_not_fit_leaves_the_network_usable():
+    """A batch whose buffers do not fit is an error code; the next, smaller one allocates again and
+    does not run on the buffers that the failed call gave up."""
+    import torch
+    batch, big = 300, 60000
+    rng = np.random.default_rng(5)
+    X = rng.standard_normal((big, 4)).astype(np.float32)
+    T = rng.standard_normal((big, 2)).astype(np.float32)
+    net = capi.Mlp(4, 256, 2, seed=11)
+    loss_ref, g_ref = net.gradient(X[:batch], T[:batch])
+    net.forward(X[:2 * batch])
+    torch.cuda.empty_cache()
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (100 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(capi.CoquiB200Error) as e:
+            net.gradient(X, T)
+        assert e.value.code == -4
+        loss, g = net.gradient(X[:batch], T[:batch])
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    assert loss == loss_ref and np.array_equal(g, g_ref)
+    net.close()
