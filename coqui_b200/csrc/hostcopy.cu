@@ -145,17 +145,26 @@ cudaError_t staged(StageSet* set, unsigned char* dst, const unsigned char* src, 
 
 }  // namespace
 
-bool host_is_pinned(const void* p) {
+namespace {
+bool memory_is(const void* p, cudaMemoryType type) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeHost;
+  return a.type == type;
 }
+// A staging set for a copy from or to host memory at p that the threads may read and write
+// themselves: ordinary memory only.  Page-locked, managed and device memory go to the driver.
+StageSet* take_for(const void* p, size_t bytes) {
+  return bytes >= kMinBytes && memory_is(p, cudaMemoryTypeUnregistered) ? take() : nullptr;
+}
+}  // namespace
+
+bool host_is_pinned(const void* p) { return memory_is(p, cudaMemoryTypeHost); }
 
 void copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  StageSet* set = bytes >= kMinBytes && !host_is_pinned(src) ? take() : nullptr;
+  StageSet* set = take_for(src, bytes);
   if (!set) {
     CQ_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
     return;
@@ -166,7 +175,7 @@ void copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
 }
 
 void copy_from_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  StageSet* set = bytes >= kMinBytes && !host_is_pinned(dst) ? take() : nullptr;
+  StageSet* set = take_for(dst, bytes);
   if (!set) {
     CQ_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
     return;

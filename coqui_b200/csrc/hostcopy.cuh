@@ -12,9 +12,9 @@ namespace cq {
 
 bool host_is_pinned(const void* p);
 
-// Stream-ordered copies.  Page-locked memory: asynchronous, as cudaMemcpyAsync.  Pageable
-// memory: to_device returns once the source has been read (it may be reused), from_device once
-// the destination is complete.
+// Stream-ordered copies.  Page-locked, managed or device memory: as cudaMemcpyAsync.  Ordinary
+// (pageable) memory: to_device returns once the source has been read (it may be reused),
+// from_device once the destination is complete.
 void copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 void copy_from_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 

@@ -1,6 +1,7 @@
 """Large ordinary (pageable) host arrays, which cross the bus through the threaded staging copies,
 give the same bytes as page-locked ones: a size that is no multiple of the staging piece, two
 contexts driven from two threads at once, and a context created after the last one was closed."""
+import ctypes
 import threading
 
 import numpy as np
@@ -52,3 +53,41 @@ def test_pageable_arrays_match_page_locked_ones(nb):
         for S in runs:
             assert np.array_equal(S, out)
     c.close()
+
+
+@pytest.mark.parametrize("managed", [False, True])
+def test_arrays_in_device_or_managed_memory_are_left_to_the_driver(managed):
+    """The threaded copies read and write host memory themselves: they take ordinary host arrays
+    only.  A pointer to device or managed memory goes to the driver's copy, which resolves it."""
+    import torch
+    ft = IAFT(1000.0, 10.0, "low")
+    s = make_system(2, 53, 26, 64, seed=5)
+    G = np.ascontiguousarray(s.G0(ft))
+    assert G.nbytes > 16 << 20
+    c = _context(s, ft)
+    ref = c.gw_iteration(G)[0]
+    if managed:
+        rt = ctypes.CDLL("libcudart.so.12")
+        addr = []
+        for _ in range(2):
+            p = ctypes.c_void_p()
+            assert rt.cudaMallocManaged(ctypes.byref(p), ctypes.c_size_t(G.nbytes), 1) == 0
+            addr.append(p.value)
+        g, out = (np.ctypeslib.as_array((ctypes.c_double * (2 * G.size)).from_address(a))
+                  for a in addr)
+        g[...] = G.reshape(-1).view(np.float64)
+        out[...] = 0
+    else:
+        g = torch.from_numpy(G).cuda()
+        out = torch.zeros_like(g)
+        addr = [g.data_ptr(), out.data_ptr()]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        rc = c.lib.coqui_b200_gw_iteration(c.h, addr[0], addr[1], None)
+        assert rc == 0, c.lib.coqui_b200_last_error(c.h)
+    got = out.view(np.complex128).reshape(G.shape) if managed else out.cpu().numpy()
+    assert np.array_equal(got, ref)
+    c.close()
+    if managed:
+        for a in addr:
+            rt.cudaFree(ctypes.c_void_p(a))
