@@ -10,18 +10,21 @@
 //  * the factor is laid out once per set_thc as the very shared-memory tiles the MMA reads (hi and
 //    lo planes, 128-byte swizzle), so a K block of A is one 32 KB bulk copy;
 //  * the words are FP16: half the bytes per value and twice the K per MMA.  hi = fp16(s x),
-//    lo = fp16(s x - hi) carry 22 bits for every value within 2^-18 of the largest of its row; s is
-//    a power of two from that maximum (of a row of Bt: from a pass over it or from the epilogue
-//    that wrote it), and the epilogue takes the powers out again.  Half as many additions into the
-//    FP32 accumulator round toward zero.
+//    lo = fp16(s x - hi) carry 22 bits for every value within 2^-18 of the largest of its row (of
+//    Bt: the maximum comes from a pass over it or from the epilogue that wrote it) or of its matrix
+//    (A), and smaller ones are off by 2^-40 of it; s is a power of two from that maximum, and the
+//    epilogue takes the powers out again.  Half as many additions into the FP32 accumulator round
+//    toward zero.
 //
 // FP16 has five exponent bits, where TF32 words have eight, so gradings have to be taken out first.
 // THC data have a free scale per point (X_P -> s_P X_P with V_PQ -> V_PQ / (s_P^2 s_Q^2)): L's rows
 // carry it and Pi its inverse, so in L^H Pi the small elements of one meet the large ones of the
-// other along K.  A factor whose columns differ by more than 2^kFacGrade is packed with them
-// brought to one size by powers of two, `ks`, which the product puts on Bt instead (X's columns in
-// the projection likewise: a free scale per orbital).  Relative error of Sigma at N_mu 300 for s_P
-// spread over 10^3 / 10^5 / 10^6, with one scale per matrix: 1.8e-5 / 3e-3 / 7e-2.
+// other along K.  Where the columns of a factor differ by more than 2^kFacGrade they are brought to
+// one size by powers of two, `ks`, which the product puts on Bt instead (X's columns in the
+// projection likewise: a free scale per orbital); where its rows do, each row gets a scale of its
+// own (GR kernels: 2 % slower, for the row's multiplication in the epilogue).  Relative error of
+// Sigma at N_mu 300 for s_P spread over 10^3 / 10^5 / 10^6: 1.8e-5 each; with one scale per matrix
+// throughout 1.8e-5 / 3e-3 / 7e-2.
 //
 // Per 32 complex K: 96 KB stored and 144 KB read against 1536 cycles of MMA, and half the
 // conversion work.  Measured (1600 problems of N_mu 512 / 675 of 1024): the M products
@@ -42,7 +45,7 @@ constexpr int kFacThreads = 320;
 // ST stages: two for long K; one for K of a few blocks, where a second CTA on the SM (96 KB each)
 // covers the first one's start and epilogue
 template <int ST> constexpr int fac_smem() {
-  return ST * kFacStage + 1024 /*align*/ + 256 /*barriers*/ + 512 + 32 /*scales, their exponents*/;
+  return ST * kFacStage + 1024 /*align*/ + 256 /*barriers*/ + 512 /*scales*/;
 }
 template <int ST> constexpr int fac_epi_cols() { return ST == 2 ? kFacN : kFacN / 2; }
 constexpr uint32_t kFacIdesc = (1u << 4) | ((uint32_t)(2 * kFacN >> 3) << 17) |
@@ -95,15 +98,15 @@ struct FacParams {
   int b_al;
 };
 
-// 32 complex K of four rows of Bt per thread: four values (32 bytes) of rows r + 32 j; KS: with the
-// scales of these K (one each without a kb)
-template <bool KS> struct FacStaging {
+// 32 complex K of four rows of Bt per thread: four values (32 bytes) of rows r + 32 j; GR: with the
+// scales of these K (1 without a kb)
+template <bool GR> struct FacStaging {
   float4 v[4][2];
   float ck[4];
   __device__ __forceinline__ void load(const FacParams& p, const float2* base, const float* kb,
                                        uint32_t ok, int64_t k0) {
     const int64_t k = k0 + 4 * (threadIdx.x & 7);
-    if constexpr (KS) {
+    if constexpr (GR) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) ck[i] = kb && k + i < p.K ? __ldg(kb + k + i) : 1.f;
     }
@@ -139,7 +142,7 @@ template <bool KS> struct FacStaging {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float4 q = v[j][i >> 1];
-        const float sk = KS ? sc[j] * ck[i] : sc[j];
+        const float sk = GR ? sc[j] * ck[i] : sc[j];
         const float x = sk * ((i & 1) ? q.z : q.x), y = sk * ((i & 1) ? q.w : q.y);
         const __half2 a = __floats2half2_rn(x, y);
         const float2 f = __half22float2(a);
@@ -162,7 +165,7 @@ template <bool KS> struct FacStaging {
   }
 };
 
-template <int ST, bool KS>
+template <int ST, bool GR>
 __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t m0, int64_t n0,
                                          unsigned char* smem_raw) {
   if (p.half < 0 && n0 > m0) return;  // tiles strictly above the diagonal
@@ -173,7 +176,6 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
   uint64_t *acc_bar = empty + ST, *done_bar = acc_bar + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
   float* scale = reinterpret_cast<float*>(smem + ST * kFacStage + 256);
-  int* scale_exp = reinterpret_cast<int*>(scale + kFacN);  // smallest and largest, per warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // a triangular factor is zero beyond its triangle
@@ -194,17 +196,14 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < kFacN) {
-    // takes the power of two of column n0 + threadIdx.x out again
+    // takes the power of two of column n0 + threadIdx.x out again, and A's if all its rows have one
+    // (then at least 2^-34: the pair is at least 2^-148, which a float holds)
     const int64_t c = n0 + threadIdx.x;
     const int e = c < p.N ? fac_exp(p.rmB[bz * p.N + c]) : 14;
-    const float f = pow2f(e - 14) * (p.nC && c < p.N ? p.nC[ia * p.N + c] : 1.f);
-    scale[threadIdx.x] = f;
-    const int ef = (int)(__float_as_uint(f) >> 23) - 127;
-    const int lo = __reduce_min_sync(0xffffffffu, ef), hi = __reduce_max_sync(0xffffffffu, ef);
-    if (lane == 0) {
-      scale_exp[2 * warp] = lo;
-      scale_exp[2 * warp + 1] = hi;
-    }
+    if constexpr (GR)
+      scale[threadIdx.x] = pow2f(e - 14) * (p.nC && c < p.N ? p.nC[ia * p.N + c] : 1.f);
+    else
+      scale[threadIdx.x] = p.invA[ia * p.M] * pow2f(e - 14);
   }
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -223,7 +222,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     bool ok = true;
     const int r = threadIdx.x >> 3;
     const float2* base = p.B + bz * p.sB + (n0 + r) * p.ldb + 4 * (threadIdx.x & 7);
-    const float* kb = KS && p.kB ? p.kB + ia * p.K : nullptr;
+    const float* kb = GR && p.kB ? p.kB + ia * p.K : nullptr;
     uint32_t rows = 0;
     float sc[4];
 #pragma unroll
@@ -232,7 +231,7 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
       if (row < p.N) rows |= 1u << j;
       sc[j] = pow2f(14 - (row < p.N ? fac_exp(p.rmB[bz * p.N + row]) : 14));
     }
-    auto step = [&](FacStaging<KS>& st, int it) -> bool {
+    auto step = [&](FacStaging<GR>& st, int it) -> bool {
       const int s = it % ST;
       if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(it / ST) & 1u) ^ 1u)) return false;
       const uint32_t hi = smem_u32(smem + s * kFacStage + kFacTile);
@@ -243,10 +242,10 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
       if (it + ST < nkb) st.load(p, base, kb, rows, (int64_t)(kb_lo + it + ST) * kFacKC);
       return true;
     };
-    FacStaging<KS> st0;
+    FacStaging<GR> st0;
     st0.load(p, base, kb, rows, (int64_t)kb_lo * kFacKC);
     if constexpr (ST == 2) {
-      FacStaging<KS> st1;
+      FacStaging<GR> st1;
       if (nkb > 1) st1.load(p, base, kb, rows, (int64_t)(kb_lo + 1) * kFacKC);
       for (int it = 0; it < nkb; it += 2) {
         if (!step(st0, it)) { ok = false; break; }
@@ -269,19 +268,10 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
     // all producers are past their last stage before it is reused
     asm volatile("bar.sync 1, %0;" ::"r"(256) : "memory");
     float mx = 0.f;
-    // The row's power of two.  It multiplies the column's first unless that pair leaves the range of
-    // normal floats, which the result need not: then the smaller one goes onto the sum, then the
-    // larger.
+    // GR: the row's power of two.  The smaller one of it and the column's goes first, so that the
+    // pair neither overflows nor underflows where the result does not.
     const int64_t row = m0 + q * 32 + lane;
-    const float ra = row < p.M ? p.invA[ia * p.M + row] : 1.f;
-    bool plain = true;
-    {
-      const int er = (int)(__float_as_uint(ra) >> 23) - 127;
-#pragma unroll
-      for (int w = 0; w < kFacN / 32; ++w)
-        plain = plain && er + scale_exp[2 * w] >= -126 && er + scale_exp[2 * w + 1] <= 127 - 42;
-      plain = __all_sync(0xffffffffu, plain);
-    }
+    const float ra = GR && row < p.M ? p.invA[ia * p.M + row] : 1.f;
 #pragma unroll 1
     for (int c0 = 0; c0 < kFacN; c0 += EC) {
       const int col = h * kFacN + c0;  // first real column of this piece
@@ -313,13 +303,11 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
           const float4 f4 = sc4[x];
           const float f[4] = {f4.x, f4.y, f4.z, f4.w};
           float o[8];
-          if (plain) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[8 * x + i]) * (f[i / 2] * ra);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              o[i] = __uint_as_float(v[8 * x + i]) * fminf(f[i / 2], ra) * fmaxf(f[i / 2], ra);
+          for (int i = 0; i < 8; ++i) {
+            o[i] = __uint_as_float(v[8 * x + i]);
+            if constexpr (GR) o[i] = o[i] * fminf(f[i / 2], ra) * fmaxf(f[i / 2], ra);
+            else o[i] *= f[i / 2];
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(o[i]));
@@ -402,10 +390,10 @@ __device__ __forceinline__ void fac_tile(const FacParams& p, int64_t bz, int64_t
   }
 }
 
-template <int ST, bool KS>
+template <int ST, bool GR>
 __global__ void __launch_bounds__(kFacThreads, 3 - ST) k_tc_fac(const __grid_constant__ FacParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  fac_tile<ST, KS>(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
+  fac_tile<ST, GR>(p, blockIdx.z, (int64_t)blockIdx.y * kBM, (int64_t)blockIdx.x * kFacN, smem_raw);
 }
 
 // Products of different sizes in one launch (a group each); the flattened tile index picks the
@@ -414,7 +402,7 @@ struct FacGroupDev {
   FacParams p;
   int64_t tiles, tile_begin;  // tiles per matrix edge
 };
-template <bool KS>
+template <bool GR>
 __global__ void __launch_bounds__(kFacThreads, 1)
     k_tc_fac_grouped(const FacGroupDev* __restrict__ groups, int ngroups) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -436,11 +424,12 @@ __global__ void __launch_bounds__(kFacThreads, 1)
     s_n0 = r % g.tiles * kFacN;
   }
   __syncthreads();
-  fac_tile<2, KS>(sp, s_bz, s_m0, s_n0, smem_raw);
+  fac_tile<2, GR>(sp, s_bz, s_m0, s_n0, smem_raw);
 }
 
 // Packing a factor: column maxima, the powers of two that level graded columns, row maxima of what
-// remains, then the tiles.  Maxima are the bits of the largest |re|, |im| as a float, rounded up.
+// remains, their common value where the rows are not graded, then the tiles.  Maxima are the bits
+// of the largest |re|, |im| as a float, rounded up.
 __device__ __forceinline__ float fac_abs(double2 v) {
   return __double2float_ru(fmax(fabs(v.x), fabs(v.y)));
 }
@@ -461,30 +450,60 @@ __global__ void __launch_bounds__(256) k_fac_colmax(const double2* __restrict__ 
     cm[q * K + k] = __float_as_uint(m);
   }
 }
-// Columns of a matrix may differ by this power of two and stay as they are: an element that small
-// in its row still has its 22 bits if it is within 2^-12 of the largest of its column.
-constexpr int kFacGrade = 6;
-// cm (bits) -> ks: a column's power of two over the largest one's, 0 for an empty column; *graded is
-// set when two columns of a matrix differ by more than 2^kFacGrade
-__global__ void __launch_bounds__(256) k_fac_kscale(uint32_t* __restrict__ cm, int64_t K,
-                                                    int* __restrict__ graded) {
-  __shared__ int lo, hi;
+// Columns, and rows, of a matrix may differ by this power of two and keep one scale: the words'
+// 2^-40 of the largest element is still 2^-30 of the largest of any column and row, and FP32 rounds
+// a sum of such terms at 2^-24.
+constexpr int kFacGrade = 10;
+constexpr int kFacExp = 20;  // a scale common to all rows lies within 2^+-20
+__device__ __forceinline__ int fac_max_exp(uint32_t bits) { return min((int)(bits >> 23) - 127, 127); }
+// smallest and largest exponent of the n nonzero maxima of a matrix (block-wide; hi < lo: none)
+__device__ __forceinline__ void fac_exp_range(const uint32_t* m, int64_t n, int* lo, int* hi) {
+  __shared__ int r[2];
   if (threadIdx.x == 0) {
-    lo = 1 << 20;
-    hi = -(1 << 20);
+    r[0] = 1 << 20;
+    r[1] = -(1 << 20);
   }
   __syncthreads();
-  uint32_t* c = cm + (int64_t)blockIdx.x * K;
-  for (int64_t k = threadIdx.x; k < K; k += blockDim.x)
-    if (c[k]) {
-      const int e = min((int)(c[k] >> 23) - 127, 127);
-      atomicMin(&lo, e);
-      atomicMax(&hi, e);
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+    if (m[i]) {
+      atomicMin(&r[0], fac_max_exp(m[i]));
+      atomicMax(&r[1], fac_max_exp(m[i]));
     }
   __syncthreads();
-  for (int64_t k = threadIdx.x; k < K; k += blockDim.x)
-    c[k] = c[k] ? __float_as_uint(pow2f(max(min((int)(c[k] >> 23) - 127, 127) - hi, -100))) : 0u;
-  if (threadIdx.x == 0 && hi - lo > kFacGrade && lo < (1 << 20)) *graded = 1;
+  *lo = r[0];
+  *hi = r[1];
+}
+// cm (bits) -> ks: of graded columns (*flag gets kFacColumns) a column's power of two over the
+// largest one's, 0 for an empty column; else 1
+__global__ void __launch_bounds__(256) k_fac_kscale(uint32_t* __restrict__ cm, int64_t K,
+                                                    int* __restrict__ flag) {
+  uint32_t* c = cm + (int64_t)blockIdx.x * K;
+  int lo, hi;
+  fac_exp_range(c, K, &lo, &hi);
+  const bool graded = hi - lo > kFacGrade;
+  for (int64_t k = threadIdx.x; k < K; k += blockDim.x) {
+    const float s = !graded ? 1.f : c[k] ? pow2f(max(fac_max_exp(c[k]) - hi, -100)) : 0.f;
+    c[k] = __float_as_uint(s);
+  }
+  if (threadIdx.x == 0 && graded) atomicOr(flag, kFacColumns);
+}
+// rm -> the matrix's maximum in every row, unless its rows are graded or it lies beyond 2^+-kFacExp
+// (*flag gets kFacRows)
+__global__ void __launch_bounds__(256) k_fac_rscale(uint32_t* __restrict__ rm, int64_t M,
+                                                    int* __restrict__ flag) {
+  uint32_t* r = rm + (int64_t)blockIdx.x * M;
+  __shared__ uint32_t most;
+  if (threadIdx.x == 0) most = 0u;
+  int lo, hi;
+  fac_exp_range(r, M, &lo, &hi);
+  const bool one = hi - lo <= kFacGrade && hi <= kFacExp && hi >= -kFacExp;
+  if (hi < lo || one) {
+    for (int64_t i = threadIdx.x; i < M; i += blockDim.x) atomicMax(&most, r[i]);
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < M; i += blockDim.x) r[i] = most;
+  } else if (threadIdx.x == 0) {
+    atomicOr(flag, kFacRows);
+  }
 }
 // one warp per row, after division by ks (may be null)
 __global__ void __launch_bounds__(256) k_fac_rowmax(const double2* __restrict__ L,

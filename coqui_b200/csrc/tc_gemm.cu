@@ -1169,28 +1169,25 @@ void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t
   f.packed.ensure((size_t)nmat * f.stride);
   f.inv.ensure((size_t)nmat * M);
   f.mx.ensure((size_t)nmat * M);
-  f.graded = false;
+  f.flag.ensure(1);
+  CQ_CHECK_CUDA(cudaMemsetAsync(f.flag.p, 0, sizeof(int), s));
   if (level_k) {
     f.ks.ensure((size_t)nmat * K);
-    f.flag.ensure(1);
-    CQ_CHECK_CUDA(cudaMemsetAsync(f.flag.p, 0, sizeof(int), s));
     uint32_t* cm = reinterpret_cast<uint32_t*>(f.ks.p);
     k_fac_colmax<<<dim3((unsigned)((K + 31) / 32), (unsigned)nmat), 256, 0, s>>>(L, cm, M, K);
     k_fac_kscale<<<(unsigned)nmat, 256, 0, s>>>(cm, K, f.flag.p);
     count_launch(2);
-    CQ_CHECK_CUDA(cudaGetLastError());
-    int flag = 0;
-    CQ_CHECK_CUDA(cudaMemcpyAsync(&flag, f.flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CQ_CHECK_CUDA(cudaStreamSynchronize(s));
-    f.graded = flag != 0;
   }
-  const float* ks = f.graded ? f.ks.p : nullptr;
+  const float* ks = level_k ? f.ks.p : nullptr;
   const unsigned g = grid_for(M * K, 256, 64);
   k_fac_rowmax<<<dim3((unsigned)((M + 7) / 8), (unsigned)nmat), 256, 0, s>>>(L, ks, f.mx.p, M, K);
+  k_fac_rscale<<<(unsigned)nmat, 256, 0, s>>>(f.mx.p, M, f.flag.p);
   k_fac_pack<<<dim3(g, (unsigned)nmat), 256, 0, s>>>(L, ks, f.mx.p, f.packed.p, f.inv.p, M, K,
                                                      f.stride);
-  count_launch(2);
+  count_launch(3);
   CQ_CHECK_CUDA(cudaGetLastError());
+  CQ_CHECK_CUDA(cudaMemcpyAsync(&f.grade, f.flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CQ_CHECK_CUDA(cudaStreamSynchronize(s));
 }
 
 void tc_gather_matrices(TcFactor& dst, const TcFactor& src, const std::vector<int64_t>& idx,
@@ -1199,16 +1196,16 @@ void tc_gather_matrices(TcFactor& dst, const TcFactor& src, const std::vector<in
   dst.M = src.M;
   dst.K = src.K;
   dst.stride = src.stride;
-  dst.graded = src.graded;
+  dst.grade = src.grade;
   dst.packed.ensure((size_t)n * src.stride);
   dst.inv.ensure((size_t)n * src.M);
-  if (src.graded) dst.ks.ensure((size_t)n * src.K);
+  if (src.grade & kFacColumns) dst.ks.ensure((size_t)n * src.K);
   for (int64_t i = 0; i < n; ++i) {
     CQ_CHECK_CUDA(cudaMemcpyAsync(dst.packed.p + i * src.stride, src.packed.p + idx[i] * src.stride,
                                   src.stride, cudaMemcpyDeviceToDevice, s));
     CQ_CHECK_CUDA(cudaMemcpyAsync(dst.inv.p + i * src.M, src.inv.p + idx[i] * src.M,
                                   src.M * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    if (src.graded)
+    if (src.grade & kFacColumns)
       CQ_CHECK_CUDA(cudaMemcpyAsync(dst.ks.p + i * src.K, src.ks.p + idx[i] * src.K,
                                     src.K * sizeof(float), cudaMemcpyDeviceToDevice, s));
   }
@@ -1242,13 +1239,13 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
                    [](const TcFactorGroup& x, const TcFactorGroup& y) { return x.f.K > y.f.K; });
   std::vector<FacGroupDev> h;
   int64_t total = 0;
-  bool scaled = false;
+  bool graded = false;
   for (const TcFactorGroup& g : order) {
     const int64_t n = g.f.K;
     FacGroupDev d;
     d.p.kB = g.b_has_ks ? nullptr : g.f.ks;
     d.p.nC = g.ks_c ? g.f.ks : nullptr;
-    scaled = scaled || d.p.kB;
+    graded = graded || g.f.ks || g.f.rows;
     d.p.A = g.f.packed;
     d.p.sA = 0;
     d.p.a_mod = 1;
@@ -1276,7 +1273,7 @@ void tc_factor_grouped(const std::vector<TcFactorGroup>& groups, DevBuf<unsigned
   table.ensure(h.size() * sizeof(FacGroupDev));
   CQ_CHECK_CUDA(cudaMemcpyAsync(table.p, h.data(), h.size() * sizeof(FacGroupDev),
                                 cudaMemcpyHostToDevice, s));
-  auto fn = scaled ? k_tc_fac_grouped<true> : k_tc_fac_grouped<false>;
+  auto fn = graded ? k_tc_fac_grouped<true> : k_tc_fac_grouped<false>;
   fn<<<(unsigned)total, kFacThreads, fac_smem<2>(), s>>>((const FacGroupDev*)table.p, (int)h.size());
   count_launch();
   CQ_CHECK_CUDA(cudaGetLastError());
@@ -1308,6 +1305,7 @@ void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, 
   FacParams p;
   p.kB = b_has_ks ? nullptr : f.ks;
   p.nC = ks_c ? f.ks : nullptr;
+  const bool graded = f.ks || f.rows;
   p.A = f.packed;
   p.sA = f.stride;
   p.invA = f.inv;
@@ -1337,10 +1335,10 @@ void tc_packed_product(const TcFactorView& f, int tri, int64_t mod, int64_t q0, 
     // 1024 12.6 against 11.4 ms two stages are ahead
     const dim3 grid(tn, tm, nb);
     if (p.K <= 256) {
-      auto fn = p.kB ? k_tc_fac<1, true> : k_tc_fac<1, false>;
+      auto fn = graded ? k_tc_fac<1, true> : k_tc_fac<1, false>;
       fn<<<grid, kFacThreads, fac_smem<1>(), s>>>(p);
     } else {
-      auto fn = p.kB ? k_tc_fac<2, true> : k_tc_fac<2, false>;
+      auto fn = graded ? k_tc_fac<2, true> : k_tc_fac<2, false>;
       fn<<<grid, kFacThreads, fac_smem<2>(), s>>>(p);
     }
     count_launch();

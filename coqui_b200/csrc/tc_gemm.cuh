@@ -5,11 +5,14 @@
 
 namespace cq {
 
+// what of a packed matrix is graded
+constexpr int kFacColumns = 1, kFacRows = 2;
 // Matrices A (M x K) packed for tc_packed_product (split FP16 tiles, tc_fac.cuh).
 struct TcFactorView {
   const unsigned char* packed = nullptr;  // matrices `stride` bytes apart
   const float* inv = nullptr;             // 1 / scale of each row, (nmat, M)
   const float* ks = nullptr;              // graded columns only: their powers of two, (nmat, K)
+  bool rows = false;                      // rows of one matrix differ in `inv`
   int64_t M = 0, K = 0, stride = 0;
 };
 struct TcFactor {
@@ -18,9 +21,11 @@ struct TcFactor {
   DevBuf<float> ks;
   DevBuf<uint32_t> mx;  // row maxima, kept for the next packing
   DevBuf<int> flag;
-  bool graded = false;
+  int grade = 0;        // kFacColumns | kFacRows
   int64_t M = 0, K = 0, stride = 0;
-  TcFactorView view() const { return {packed.p, inv.p, graded ? ks.p : nullptr, M, K, stride}; }
+  TcFactorView view() const {
+    return {packed.p, inv.p, grade & kFacColumns ? ks.p : nullptr, (grade & kFacRows) != 0, M, K, stride};
+  }
   void release() {
     packed.release();
     inv.release();
@@ -29,9 +34,8 @@ struct TcFactor {
     flag.release();
   }
 };
-// nmat row-major complex128 matrices; level_k: columns that differ by more than 2^6 are brought to
-// one size (asks the device, and waits for the answer), for a product whose Bt carries the inverse
-// grading along K
+// nmat row-major complex128 matrices; level_k: graded columns are brought to one size, for a product
+// whose Bt carries the inverse grading along K.  Waits for the stream.
 void tc_pack_matrix(TcFactor& f, const double2* L, int64_t M, int64_t K, int64_t nmat, bool level_k,
                     cudaStream_t s);
 // dst = the matrices idx of src

@@ -42,7 +42,7 @@ def dense_g(s):
 
 
 @pytest.mark.parametrize("Np", [129, 200, 290])
-@pytest.mark.parametrize("decades", [2, 5, 8])
+@pytest.mark.parametrize("decades", [2, 3, 5, 8])  # 10^3: just below the level that is graded
 def test_w_of_graded_v_and_pi(Np, decades):
     """V = D V0 D with Pi = D^-1 Pi0 D^-1: D^-1 W D^-1 does not depend on D."""
     s = make_system((2, 1, 1), 3, 1, Np, seed=Np)
