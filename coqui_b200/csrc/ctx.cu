@@ -66,8 +66,8 @@ struct SymState {
   cq::TcFactor Lpi, LHpi;
   DevBuf<double2> Gi;             // (nt, nk_ibz, nb, nb) G on the IBZ k-points
   DevBuf<unsigned char> PWi;      // (nmax, nq_ibz, Np, Np) Pi / W on the IBZ q-points
-  DevBuf<unsigned char> Sq;       // (nsym, nk_ibz, Np, Np) Sigma_PQ rows of one tau
-  DevBuf<double2> Sab, Tab, Rab;  // (nsym, nk_ibz, nb, nb)
+  DevBuf<unsigned char> Sq;       // (tau group, nsym, nk_ibz, Np, Np) Sigma_PQ rows
+  DevBuf<double2> Sab, Tab, Rab;  // (tau group, nsym, nk_ibz, nb, nb)
   // long-wavelength treatments on the IBZ: X of the IBZ k-points, chi-bar heads and prefactors
   // of the IBZ q-points, T^k of Sigma_div_correction, eps^-1 per (tau, q_ibz)
   DevBuf<double2> Xibz, chi_i, Tdiv;

@@ -275,13 +275,22 @@ void sym_sigma(Ctx* c, double* host_out) {
   const int64_t nki = S.nk_ibz, nqi = S.nq_ibz, pp = Np * Np, bb = nb * nb;
   const int64_t nrow = S.nsym * nki;
   const size_t es = c->elem(), slab = (size_t)nk * pp * es;
-  // slices per group: 256 projections fill the GPU (36 of N_mu 384 leave most of it idle), in at
-  // most 512 MB of Sigma_PQ rows
-  const int64_t group = std::max<int64_t>(
-      1, std::min<int64_t>({(256 + nrow - 1) / nrow, nth,
-                            (int64_t)(((size_t)512 << 20) / ((size_t)nrow * pp * es))}));
   c->Gp.ensure(slab);
-  S.Sq.ensure((size_t)group * nrow * pp * es);
+  // slices per group: 256 projections fill the GPU (36 of N_mu 384 leave most of it idle), in at
+  // most 512 MB of Sigma_PQ rows and, where that buffer has to grow, a quarter of the free memory
+  // (the other buffers were sized for one slice's rows)
+  const size_t row_bytes = (size_t)nrow * pp * es;
+  auto in = [&](size_t bytes) {
+    return std::max<int64_t>(
+        1, std::min<int64_t>({(256 + nrow - 1) / nrow, nth, (int64_t)(bytes / row_bytes)}));
+  };
+  int64_t group = in((size_t)512 << 20);
+  if (S.Sq.n < (size_t)group * row_bytes) {
+    size_t fr = 0, tot = 0;
+    CQ_CHECK_CUDA(cudaMemGetInfo(&fr, &tot));
+    group = std::min(group, in(std::max(S.Sq.n, (fr + S.Sq.n) / 4)));
+  }
+  S.Sq.ensure((size_t)group * row_bytes);
   S.Sab.ensure((size_t)group * nrow * bb);
   S.Tab.ensure((size_t)group * nrow * bb);
   S.Rab.ensure((size_t)group * nrow * bb);

@@ -35,3 +35,36 @@ def test_convolution_rows_match_the_term_sums(kind, grid, lam, mode, tol):
     assert np.abs(S1 - S).max() < 1e-12
     assert np.abs(ref).max() > 1e-3
     c.close()
+
+
+def test_sigma_fits_beside_other_allocations():
+    """The rows of a group of tau slices are a buffer of up to 512 MB; with less memory left on the
+    GPU the groups become smaller and the call succeeds."""
+    import torch
+    ft, pft = O.IAFT(1000.0, 10.0, "low"), ProductIAFT(1000.0, 10.0, "low")
+    d = symmetric_system("trev", (2, 2, 2), 5, 640, ft, seed=3)
+    sym = d["sym"]
+    rows = sym["nk_ibz"] * 640 ** 2 * 8
+    assert min(32, ft.nt_f // 2) * rows > 300 << 20
+    c = capi.Context(sym["nk"], 5, 640, ft.nt_f, ft.nw_b, d["grid"], mode=capi.MIXED)
+    c.set_ir(pft)
+    c.set_kmesh(d["kpts_lex"], d["lattv"], d["chi_lex"])
+    c.set_thc(d["X_lex"], d["V_lex"])
+    c.set_symmetry(sym, d["D"])
+    c.update_w(d["G_ibz"], want_w=False, want_head=False)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    ballast = torch.empty(free - (260 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        S = c.eval_sigma(d["G_ibz"])
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    c.close()
+    c = capi.Context(sym["nk"], 5, 640, ft.nt_f, ft.nw_b, d["grid"], mode=capi.MIXED)
+    c.set_ir(pft)
+    c.set_kmesh(d["kpts_lex"], d["lattv"], d["chi_lex"])
+    c.set_thc(d["X_lex"], d["V_lex"])
+    c.set_symmetry(sym, d["D"])
+    assert np.abs(c.gw_iteration(d["G_ibz"])[0] - S).max() < 1e-12
+    c.close()
