@@ -10,6 +10,7 @@
 // The self-energy and the RPA energy reuse the same stages.
 #include <algorithm>
 #include <complex>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <set>

@@ -176,8 +176,10 @@ void sym_update_w(Ctx* c) {
 // terms against convolutions), 4x4x1 with 10 irreducible k-points 0.84 / 1.05, 6x6x1 with 21 and
 // two operations 2.17 / 2.63, 5x4x3 with 31 4.5 / 1.9, 6x6x2 with 42 and two operations 7.7 / 3.4;
 // the cubic grids run DFTs of compile-time shape: 2x2x2 with 8 0.49 / 0.19, 3x3x3 with 14
-// 1.28 / 0.40, 4x4x4 with 36 5.7 / 0.80.
+// 1.28 / 0.40, 4x4x4 with 36 5.7 / 0.80.  COQUI_B200_IBZ_CONV=0 or 1 picks the form (tests).
 bool sym_conv_pays(KGrid g, int64_t nk_ibz, int64_t nsym) {
+  const char* force = std::getenv("COQUI_B200_IBZ_CONV");
+  if (force && (force[0] == '0' || force[0] == '1')) return force[0] == '1';
   const bool cubic = g.n0 == g.n1 && g.n1 == g.n2;
   return (cubic ? 8 : 12) * nsym <= nk_ibz;
 }

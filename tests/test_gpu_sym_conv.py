@@ -2,6 +2,8 @@
 k-points per operation; cubic and non-cubic grids, odd edges, one and two operations, whole and
 partial groups of tau slices) against the k-space oracle, with an odd number of tau points too.
 Tolerances as the other IBZ parity tests."""
+import os
+
 import numpy as np
 import pytest
 
@@ -35,6 +37,34 @@ def test_convolution_rows_match_the_term_sums(kind, grid, lam, mode, tol):
     assert np.abs(S1 - S).max() < 1e-12
     assert np.abs(ref).max() > 1e-3
     c.close()
+
+
+@pytest.mark.parametrize("kind,grid,Np", [("trev", (2, 2, 2), 19), ("swap", (5, 5, 2), 20),
+                                          ("trev", (3, 2, 1), 131)])
+@pytest.mark.parametrize("mode,tol", [(capi.FP64, 1e-12), (capi.MIXED, 1e-6)], ids=["fp64", "mixed"])
+def test_both_forms_of_the_rows_agree(kind, grid, Np, mode, tol):
+    """COQUI_B200_IBZ_CONV picks the form: term sums launch once per tau slice, convolutions once
+    per group of slices, and both give the same Sigma."""
+    ft, pft = O.IAFT(1000.0, 10.0, "low"), ProductIAFT(1000.0, 10.0, "low")
+    d = symmetric_system(kind, grid, 5, Np, ft, seed=4)
+    sym, S, launches = d["sym"], [], []
+    try:
+        for form in "01":
+            os.environ["COQUI_B200_IBZ_CONV"] = form
+            c = capi.Context(sym["nk"], 5, Np, ft.nt_f, ft.nw_b, d["grid"], mode=mode)
+            c.set_ir(pft)
+            c.set_kmesh(d["kpts_lex"], d["lattv"], d["chi_lex"])
+            c.set_thc(d["X_lex"], d["V_lex"])
+            c.set_symmetry(sym, d["D"])
+            c.gw_iteration(d["G_ibz"])
+            n0 = c.kernel_launches()
+            S.append(c.gw_iteration(d["G_ibz"])[0])
+            launches.append(c.kernel_launches() - n0)
+            c.close()
+    finally:
+        os.environ.pop("COQUI_B200_IBZ_CONV", None)
+    assert launches[1] < launches[0]
+    assert np.abs(S[0] - S[1]).max() < tol * max(1.0, np.abs(S[0]).max())
 
 
 def test_sigma_fits_beside_other_allocations():
