@@ -428,23 +428,27 @@ bool chol_prefer_tiled(const std::vector<int64_t>& sizes) {
   const int64_t nmax0 = sizes.empty() ? 0 : *std::max_element(sizes.begin(), sizes.end());
   if (force && (force[0] == '0' || force[0] == '1'))
     return force[0] == '1' && nmax0 >= 4 * b32::CB;
-  // Problems of one size (a chunk's remainder below a wave): the times of both forms, from a fit
-  // (within 25 %) of measurements at N_mu 192 to 1024 and 36 to 576 problems, in us.  One CTA per
-  // problem: T1 = 1e-5 n^3 + 25 a block column with one problem on an SM, half of it more for each
-  // further one (N_mu 512: 1.86, 2.53, 3.65, 4.60 ms for 1 to 4; 1024: 10.7, 15.5, 23.6, 30.6).
-  // Tiled: 57 a block column for the launches' latency and 5e-8 n^3 (1 + 200 / n) a problem
-  // (512: 1.24 ms for 36 problems, 2.31 for 144, 4.94 for 432; 1024: 4.0, 10.4, 28.4).  The tiled
-  // form is the faster one below about 60 problems of 384, 100 of 512, 150 of 1024, and never
-  // at 192.
+  // Problems of one size (a chunk's remainder below a wave, a batch of equal molecules): the times of
+  // both forms in us, from a fit (within 9 %, 13 % far from where they cross) of measurements at
+  // N_mu 384 to 1024 and 36 to 576 problems on 148 SMs.  One CTA per problem: T1 = 9e-6 n^3 + 38 a
+  // block column (N_mu 512 1.9 ms, 768 5.1, 1024 10.8) with one problem on an SM, times
+  // 0.13 + 0.63 p with p of them (512 2.5 ms for p = 2; 1024 15.5 and 23.1 for 2 and 3).  Tiled, N
+  // block columns: (45 + 0.75 N) N for the launches' latency and 3.6e-8 n^3 (1 + 530 / n) a problem
+  // (512 1.59 ms for 72, 3.38 for 252; 1024 10.5 for 144, 20.8 for 324).  One CTA's time steps with
+  // the problems on an SM, so the tiled form is chosen in windows that begin with each step: up to 65
+  // problems of 384; up to 91 and 149 to 163 of 512; 126 and 149 to 196 of 768; 147, 149 to 220,
+  // 297 to 337 and 445 to 453 of 1024.  At 52 of those sizes the rule missed the faster form once, by
+  // 1.4 %.  Below 384 one CTA was always ahead (320: 0.63 against 0.68 ms for 36, 1.49 against 2.29 for
+  // 576; 192: 0.25 / 0.40, 0.52 / 0.92).
   if (!sizes.empty() && nmax0 == *std::min_element(sizes.begin(), sizes.end())) {
     int dv = 0, nsm = 148;
     cudaGetDevice(&dv);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dv);
     const double n = (double)nmax0, n3 = n * n * n, blocks = (double)((nmax0 + b32::CB - 1) / b32::CB);
     const double per_sm = (double)(((int64_t)sizes.size() + nsm - 1) / nsm);
-    const double one = (1e-5 * n3 + 25.0 * blocks) * (0.5 + 0.5 * per_sm);
-    const double tiled = 57.0 * blocks + 5e-8 * n3 * (1.0 + 200.0 / n) * (double)sizes.size();
-    return nmax0 >= 4 * b32::CB && tiled < one;
+    const double one = (9e-6 * n3 + 38.0 * blocks) * std::max(1.0, 0.13 + 0.63 * per_sm);
+    const double tiled = (45.0 + 0.75 * blocks) * blocks + 3.6e-8 * n3 * (1.0 + 530.0 / n) * (double)sizes.size();
+    return nmax0 >= 384 && tiled < one;
   }
   // one CTA per problem: the makespan is at least the largest problem's time; spreading each
   // problem over many CTAs pays when the whole set would otherwise finish sooner than that

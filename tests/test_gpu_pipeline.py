@@ -110,10 +110,11 @@ def test_resident_iteration_graph_matches_direct_launches(case):
     c.close()
 
 
-def test_graph_capture_of_tiled_factorisation_and_tensor_core_inverse():
-    """Np = 300 with one q: a few large Dyson problems take the tiled factorisation and the
-    tensor-core inverse levels; both are captured in the resident-G graph and replay to the
-    directly launched result."""
+def test_graph_capture_of_tiled_factorisation_and_tensor_core_inverse(monkeypatch):
+    """Np = 300 with one q: a few large Dyson problems on the tiled factorisation (asked for: at
+    this size the library would take the other one) and the tensor-core inverse levels; both are
+    captured in the resident-G graph and replay to the directly launched result."""
+    monkeypatch.setenv("COQUI_B200_CHOL_TILED", "1")
     s = make_system(1, 16, 8, 300, seed=7, gamma_only=True)
     ft = O.IAFT(1000.0, 10.0, "low")
     G = s.G0(ft)
