@@ -2,10 +2,10 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
-#include <vector>
 
 #include "hostcopy.cuh"
 
@@ -27,7 +27,8 @@ struct StageSet {
 
 std::mutex g_mu;
 int g_users = 0, g_sets = 0;            // live users; sets in use or free
-std::vector<StageSet*>* g_free = nullptr;
+StageSet* g_free[kMaxStageSets];        // the first g_nfree
+int g_nfree = 0;
 
 void destroy(StageSet* s) {
   for (auto& t : s->ev)
@@ -44,24 +45,25 @@ StageSet* take() {
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_free)
-      for (size_t i = 0; i < g_free->size(); ++i)
-        if ((*g_free)[i]->dev == dev) {
-          StageSet* s = (*g_free)[i];
-          g_free->erase(g_free->begin() + i);
-          return s;
-        }
+    for (int i = 0; i < g_nfree; ++i)
+      if (g_free[i]->dev == dev) {
+        StageSet* s = g_free[i];
+        g_free[i] = g_free[--g_nfree];
+        return s;
+      }
     if (g_users == 0 || g_sets >= kMaxStageSets) return nullptr;
     ++g_sets;
   }
-  StageSet* s = new StageSet();
-  s->dev = dev;
-  bool ok = cudaHostAlloc((void**)&s->p, kMaxThreads * 2 * kPiece, cudaHostAllocDefault) == cudaSuccess;
-  for (auto& t : s->ev)
-    for (cudaEvent_t& e : t)
-      ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  StageSet* s = new (std::nothrow) StageSet();
+  bool ok = s && cudaHostAlloc((void**)&s->p, kMaxThreads * 2 * kPiece, cudaHostAllocDefault) == cudaSuccess;
+  if (ok) {
+    s->dev = dev;
+    for (auto& t : s->ev)
+      for (cudaEvent_t& e : t)
+        ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  }
   if (!ok) {
-    destroy(s);
+    if (s) destroy(s);
     std::lock_guard<std::mutex> lk(g_mu);
     --g_sets;
     return nullptr;
@@ -72,8 +74,7 @@ StageSet* take() {
 void give_back(StageSet* s) {
   std::unique_lock<std::mutex> lk(g_mu);
   if (g_users > 0) {
-    if (!g_free) g_free = new std::vector<StageSet*>();
-    g_free->push_back(s);
+    g_free[g_nfree++] = s;
     return;
   }
   --g_sets;
@@ -88,17 +89,17 @@ int thread_count(size_t bytes) {
 }
 
 // work(t) on n threads, this one included; a thread that cannot be started has its share done
-// here
+// here.  Nothing is thrown while threads run.
 template <typename F> void parallel(int n, F&& work) {
-  std::vector<std::thread> th;
+  std::thread th[kMaxThreads];
   int started = 1;
   try {
-    for (; started < n; ++started) th.emplace_back(work, started);
-  } catch (const std::system_error&) {
+    for (; started < n; ++started) th[started] = std::thread(work, started);
+  } catch (const std::exception&) {
   }
   work(0);
   for (int t = started; t < n; ++t) work(t);
-  for (auto& t : th) t.join();
+  for (int t = 1; t < started; ++t) th[t].join();
 }
 
 // Moves `bytes` through the staging set: thread t takes the pieces t, t + n, ...
@@ -191,15 +192,18 @@ StageUser::StageUser() {
 }
 
 StageUser::~StageUser() {
-  std::vector<StageSet*> gone;
+  StageSet* gone[kMaxStageSets];
+  int n = 0;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (--g_users == 0 && g_free) {
-      gone.swap(*g_free);
-      g_sets -= (int)gone.size();
+    if (--g_users == 0) {
+      n = g_nfree;
+      std::copy(g_free, g_free + n, gone);
+      g_nfree = 0;
+      g_sets -= n;
     }
   }
-  for (StageSet* s : gone) destroy(s);
+  for (int i = 0; i < n; ++i) destroy(gone[i]);
 }
 
 }  // namespace cq
