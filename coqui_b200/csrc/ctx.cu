@@ -360,9 +360,13 @@ void require_ready(Ctx* c, bool thc, bool ir, bool k) {
 // ntau consecutive G slices (ntau, nk, nb, nb) complex128 on the device -> out (ntau, nk,
 // Np, Np) in storage precision.  The tensor-core form batches all ntau * nk problems.
 // FP64: the tau slices go in batches of at least 256 (tau, k) problems (one 384 x 48 x 48
-// product of 27 k-points has 162 CTAs, one per SM), X addressed periodically in k.
+// product of 27 k-points has 162 CTAs, one per SM), X addressed periodically in k.  The intermediate
+// of a batch stays below 128 MB: larger problems fill the GPU a slice at a time, and the buffer is
+// not among those that the projected-G cache leaves room for.
 int64_t fp64_tau_batch(Ctx* c, int64_t ntau) {
-  return std::min<int64_t>(ntau, (256 + c->nk - 1) / c->nk);
+  const int64_t slice = c->nk * c->Np * c->nb * (int64_t)sizeof(double2);
+  const int64_t most = std::max<int64_t>(1, ((int64_t)128 << 20) / slice);
+  return std::min<int64_t>({ntau, (256 + c->nk - 1) / c->nk, most});
 }
 void p2a_fp64(Ctx* c, const double2* Gk, double2* out, int64_t ntau) {
   const int64_t nk = c->nk, nb = c->nb, Np = c->Np, step = fp64_tau_batch(c, ntau);

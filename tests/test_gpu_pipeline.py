@@ -202,3 +202,28 @@ def test_partial_projection_cache(case, mode, tol):
     c.set_gcache_limit(-1)
     with pytest.raises(capi.CoquiB200Error):
         c.set_gcache_limit(-2)
+
+
+def test_fp64_projection_buffer_is_bounded():
+    """The FP64 projections batch tau slices of small systems only: with the projected-G cache a
+    large system holds the cache and no more than 128 MB beyond what it holds without."""
+    import torch
+    nb, Np = 300, 1800
+    s = make_system(1, nb, nb // 2, Np, beta=100.0, seed=7, gamma_only=True)
+    ft = ProductIAFT(100.0, 10.0, "low")
+    G = s.G0(ft)
+    assert ft.nt_f * Np * nb * 16 > 250 << 20
+    used = []
+    for limit in (0, -1):
+        c = capi.Context(1, nb, Np, ft.nt_f, ft.nw_b, s.kp_grid, mode=capi.FP64)
+        c.set_ir(ft)
+        c.set_kmesh(s.kpts, s.lattv, s.chi_bar)
+        c.set_thc(s.X, s.V)
+        c.set_gcache_limit(limit)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        c.update_w(G, want_w=False, want_head=False)
+        used.append(free - torch.cuda.mem_get_info()[0])
+        c.close()
+    cache = ft.nt_f * Np ** 2 * 16
+    assert used[1] - used[0] < cache + (136 << 20), (used, cache)
