@@ -1171,7 +1171,7 @@ int coqui_b200_set_thc(coqui_b200_ctx* c, const double* X_skPa, const double* V_
     CQ_REQUIRE(info == 0, COQUI_B200_ENOTHPD, "Coulomb matrix V^q is not positive definite");
     cq::launch_zero_upper_and_adjoint(c->L.p, c->LH.p, Np, nk, c->st);
     if (c->mode == COQUI_B200_MIXED) {
-      cq::tc_pack_X(c->Xtc, c->X.p, nk, Np, nb, c->st);
+      cq::tc_pack_X(c->Xtc, c->X.p, nk, Np, nb, true, c->st);
       if (Np > cq::kInvGroup) {
         cq::tc_pack_matrix(c->Lp, c->L.p, Np, Np, nk, false, c->st);
         cq::tc_pack_matrix(c->LHp, c->LH.p, Np, Np, nk, true, c->st);

@@ -91,7 +91,7 @@ void sym_prepare_thc(Ctx* c) {
       CQ_CHECK_CUDA(cudaMemcpyAsync(S.LHci.p + i * pp, c->LHc.p + q * pp, bc, cudaMemcpyDeviceToDevice, c->st));
     }
   }
-  if (mixed) cq::tc_pack_X(S.Xtc, S.Xs.p, S.nsym * nki, Np, nb, c->st);
+  if (mixed) cq::tc_pack_X(S.Xtc, S.Xs.p, S.nsym * nki, Np, nb, false, c->st);
   CQ_CHECK_CUDA(cudaStreamSynchronize(c->st));
   S.thc_ready = true;
 }

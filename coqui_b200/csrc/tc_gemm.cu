@@ -1463,7 +1463,7 @@ void to_c64(const double2* in, float2* out, int64_t rows, int64_t cols, int64_t 
 // keeps the narrower autotuned tiles.
 static bool packed_projection(int64_t Np, int64_t nb) { return Np > 128 && nb >= 24; }
 
-void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t nb,
+void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t nb, bool p2a,
                cudaStream_t s) {
   op.X = X;
   op.nk = nk;
@@ -1473,7 +1473,7 @@ void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t 
   float2* Xc = (float2*)op.packed.p;
   to_c64(X, Xc, Np, nb, nk, false, s);                 // X   (nk, Np, nb)
   to_c64(X, Xc + nk * Np * nb, Np, nb, nk, true, s);   // X^T (nk, nb, Np)
-  if (packed_projection(Np, nb)) tc_pack_matrix(op.Xp, X, Np, nb, nk, true, s);
+  if (p2a && packed_projection(Np, nb)) tc_pack_matrix(op.Xp, X, Np, nb, nk, true, s);
 }
 
 void tc_project_p2a(TcOperand& op, const double2* Gk, float2* out, int64_t nk, int64_t Np,

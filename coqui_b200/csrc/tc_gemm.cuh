@@ -73,7 +73,8 @@ struct TcOperand {
   }
 };
 
-void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t nb,
+// p2a: for tc_project_p2a too (the IBZ route's X per self-energy row only projects back)
+void tc_pack_X(TcOperand& op, const double2* X, int64_t nk, int64_t Np, int64_t nb, bool p2a,
                cudaStream_t s);
 
 // out[b] = X^k G^b X^k^H  (Np x Np, complex64) for nbatch problems b = (tau, k), k = b % nk;
