@@ -209,22 +209,40 @@ struct coqui_b200_ctx {
   std::vector<cudaEvent_t> up_ev;
   bool g_pipelined = false;
 
-  // phase timing of the last call
-  std::vector<std::pair<std::string, cudaEvent_t>> marks;
+  // phase timing of the last call; a captured iteration's phases are events inside its graph
+  struct Mark {
+    std::string name;
+    cudaEvent_t ev;
+    bool own;  // by the list it stands in
+  };
+  std::vector<Mark> marks, gw_marks, rpa_marks;
+  std::vector<Mark>* captured_marks = nullptr;  // while capturing: where phases go, if anywhere
+  // the caller reads last_timings: only then do graphs hold phases (8 events cost the iteration of
+  // 8 k-points, N_mu 128 40 of its 900 us)
+  mutable bool timings_read = false;
   std::vector<std::pair<std::string, double>> last_ms;
 
   size_t elem() const { return mode == COQUI_B200_FP64 ? sizeof(double2) : sizeof(float2); }
 
   void mark(const char* name) {
-    if (capturing) return;  // the phases of a captured iteration are not recorded
-    cudaEvent_t e;
-    CQ_CHECK_CUDA(cudaEventCreate(&e));
-    CQ_CHECK_CUDA(cudaEventRecord(e, st));
-    marks.emplace_back(name, e);
+    if (capturing && !captured_marks) return;
+    std::vector<Mark>& to = capturing ? *captured_marks : marks;
+    to.push_back(Mark{name, nullptr, true});
+    CQ_CHECK_CUDA(cudaEventCreate(&to.back().ev));
+    CQ_CHECK_CUDA(cudaEventRecordWithFlags(to.back().ev, st,
+                                           capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
+  }
+  static void drop(std::vector<Mark>& list) {
+    for (auto& m : list)
+      if (m.own && m.ev) cudaEventDestroy(m.ev);
+    list.clear();
+  }
+  // the phases of a graph launched in this call
+  void take_marks(const std::vector<Mark>& graph) {
+    for (const Mark& m : graph) marks.push_back(Mark{m.name, m.ev, false});
   }
   void begin_timing() {
-    for (auto& m : marks) cudaEventDestroy(m.second);
-    marks.clear();
+    drop(marks);
     mark("start");
   }
   void end_timing() {
@@ -233,11 +251,10 @@ struct coqui_b200_ctx {
     last_ms.clear();
     for (size_t i = 1; i < marks.size(); ++i) {
       float ms = 0;
-      cudaEventElapsedTime(&ms, marks[i - 1].second, marks[i].second);
-      last_ms.emplace_back(marks[i].first, ms);
+      cudaEventElapsedTime(&ms, marks[i - 1].ev, marks[i].ev);
+      last_ms.emplace_back(marks[i].name, ms);
     }
-    for (auto& m : marks) cudaEventDestroy(m.second);
-    marks.clear();
+    drop(marks);
   }
 };
 
@@ -1009,7 +1026,7 @@ void coqui_b200_destroy(coqui_b200_ctx* c) {
   c->Lp.release();
   c->LHp.release();
   c->Xtc.release();
-  for (auto& m : c->marks) cudaEventDestroy(m.second);
+  for (auto* list : {&c->marks, &c->gw_marks, &c->rpa_marks}) Ctx::drop(*list);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
@@ -1024,6 +1041,7 @@ int64_t coqui_b200_kernel_launches(const coqui_b200_ctx* c) {
 
 int coqui_b200_last_timings(const coqui_b200_ctx* c, char* names, int name_len, double* ms, int n) {
   if (!c) return COQUI_B200_EINVAL;
+  c->timings_read = true;
   int k = 0;
   for (const auto& p : c->last_ms) {
     if (k >= n) break;
@@ -1710,20 +1728,23 @@ void check_dyson_status(Ctx* c, std::vector<double>* ld = nullptr,
 // G_host / S_host: page-locked host buffers copied in / out inside the graph (chunked on the
 // copy stream as in the directly launched path), or nullptr for the resident G and a Sigma
 // left on the device.  The graph is replayed by the next call with the same buffers.  `timed`:
-// the caller marks the call's phases.
+// the caller has begun the call's timing; the graph's phases are marked in it if they are read.
 void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host, bool timed = false) {
   if (!timed) c->begin_timing();
+  const bool phases = timed && c->timings_read;
   const bool replay = c->gexec && c->graph_call == c->calls - 1 && c->graph_g == G_host &&
-                      c->graph_s == S_host;
+                      c->graph_s == S_host && (!phases || !c->gw_marks.empty());
   if (!replay) {
     if (c->gexec) {
       cudaGraphExecDestroy(c->gexec);
       c->gexec = nullptr;
     }
+    Ctx::drop(c->gw_marks);
     c->g_pipelined = false;  // the resident G is complete on the device
     const int64_t l0 = cq::launches_total();
     CQ_CHECK_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
+    c->captured_marks = phases ? &c->gw_marks : nullptr;
     cudaGraph_t g = nullptr;
     try {
       if (G_host) upload_G(c, G_host);
@@ -1731,11 +1752,13 @@ void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host, bool timed
       sigma_device(c, S_host);
     } catch (...) {
       c->capturing = false;
+      c->captured_marks = nullptr;
       if (cudaStreamEndCapture(c->st, &g) == cudaSuccess && g) cudaGraphDestroy(g);
       cudaGetLastError();
       throw;
     }
     c->capturing = false;
+    c->captured_marks = nullptr;
     CQ_CHECK_CUDA(cudaStreamEndCapture(c->st, &g));
     c->graph_launches = cq::launches_total() - l0;
     const cudaError_t e = cudaGraphInstantiate(&c->gexec, g, 0);
@@ -1747,7 +1770,8 @@ void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host, bool timed
     cq::count_launch(c->graph_launches);  // the replay launches the captured kernels again
   }
   CQ_CHECK_CUDA(cudaGraphLaunch(c->gexec, c->st));
-  c->mark("GW_ITERATION_GRAPH");
+  if (phases) c->take_marks(c->gw_marks);
+  else c->mark("GW_ITERATION_GRAPH");
   c->graph_call = c->calls;
   check_dyson_status(c);  // factorisation status of every (iW, q) problem of this iteration
   if (!timed) c->end_timing();
@@ -1759,29 +1783,38 @@ void gw_iteration_graph(Ctx* c, const double* G_host, double* S_host, bool timed
 // the next call with the same G argument.
 void rpa_energy_graph(Ctx* c, const double* G_host, double* e_rpa, bool timed = false) {
   if (!timed) c->begin_timing();
-  const bool replay = c->rexec && c->rgraph_call == c->calls - 1 && c->rgraph_g == G_host;
+  const bool phases = timed && c->timings_read;
+  const bool replay = c->rexec && c->rgraph_call == c->calls - 1 && c->rgraph_g == G_host &&
+                      (!phases || !c->rpa_marks.empty());
   if (!replay) {
     if (c->rexec) {
       cudaGraphExecDestroy(c->rexec);
       c->rexec = nullptr;
     }
+    Ctx::drop(c->rpa_marks);
     c->g_pipelined = false;  // the resident G is complete on the device
     const int64_t l0 = cq::launches_total();
     CQ_CHECK_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
+    c->captured_marks = phases ? &c->rpa_marks : nullptr;
     cudaGraph_t g = nullptr;
     try {
       if (G_host) upload_G(c, G_host);
       eval_pi_device(c);
+      c->mark("EVALUATE_PI_R");
       ir_inplace(c, (int)c->nth, (int)c->nwh, c->dTwt.p);
+      c->mark("IMAG_FT_TtoW");
       dyson_all(c, false, true, nullptr, nullptr);
+      c->mark("EVALUATE_RPA");
     } catch (...) {
       c->capturing = false;
+      c->captured_marks = nullptr;
       if (cudaStreamEndCapture(c->st, &g) == cudaSuccess && g) cudaGraphDestroy(g);
       cudaGetLastError();
       throw;
     }
     c->capturing = false;
+    c->captured_marks = nullptr;
     CQ_CHECK_CUDA(cudaStreamEndCapture(c->st, &g));
     c->rgraph_launches = cq::launches_total() - l0;
     const cudaError_t e = cudaGraphInstantiate(&c->rexec, g, 0);
@@ -1792,7 +1825,8 @@ void rpa_energy_graph(Ctx* c, const double* G_host, double* e_rpa, bool timed = 
     cq::count_launch(c->rgraph_launches);
   }
   CQ_CHECK_CUDA(cudaGraphLaunch(c->rexec, c->st));
-  c->mark("RPA_GRAPH");
+  if (phases) c->take_marks(c->rpa_marks);
+  else c->mark("RPA_GRAPH");
   c->rgraph_call = c->calls;
   std::vector<double> ld;
   std::vector<double2> tr;

@@ -323,7 +323,10 @@ COQUI_B200_API int coqui_b200_tau_to_w(coqui_b200_ctx* ctx, const double* X_tqPQ
 COQUI_B200_API int coqui_b200_w_to_tau(coqui_b200_ctx* ctx, const double* X_wqPQ, double* X_tqPQ);
 COQUI_B200_API int coqui_b200_dyson_w(coqui_b200_ctx* ctx, const double* Pi_wqPQ, double* W_wqPQ);
 
-/* Device-timed breakdown of the last call: fills up to n (name, ms) pairs, returns count. */
+/* Device-timed breakdown of the last call: fills up to n (name, ms) pairs, returns count.  An
+   iteration of a resident G or of page-locked arrays that ran as one CUDA graph is one phase.
+   With ordinary arrays a graph holds the phases of the direct call once a caller of the context
+   has read this breakdown (one phase in the first reading, if calls were replayed before it). */
 COQUI_B200_API int coqui_b200_last_timings(const coqui_b200_ctx* ctx, char* names, int name_len, double* ms,
                             int n);
 

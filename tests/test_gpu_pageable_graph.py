@@ -52,3 +52,31 @@ def test_replayed_calls_match_fresh_contexts(grid, Np):
         assert np.array_equal(c.gw_iteration(Gs[i])[0], sigma[1, i])
         assert c.rpa_energy(Gs[i]) == energy[1, i]
     c.close()
+
+
+def test_replayed_calls_report_the_phases_of_the_direct_one():
+    """To a caller that reads the breakdown; another one's graphs do not pay for the events."""
+    s = make_system((2, 2, 2), 7, 3, 40, seed=1)
+    G = s.G0(FT)
+    c = context(s)
+    for call in (lambda: c.gw_iteration(G), lambda: c.rpa_energy(G)):
+        names, total = [], []
+        for _ in range(4):  # direct, captured, replayed twice
+            call()
+            t = c.timings()
+            names.append([n for n, _ in t])
+            assert all(0 < ms < 1000 for _, ms in t), t
+            total.append(sum(ms for _, ms in t))
+        assert all(n == names[0] for n in names) and "EVALUATE_PI_R" in names[0]
+        assert total[3] < 10 * total[2] and total[2] < 10 * total[3]
+    c.close()
+    c = context(s)  # nobody reads the breakdown of the first calls
+    for call, one in ((lambda: c.gw_iteration(G), "GW_ITERATION_GRAPH"), (lambda: c.rpa_energy(G), None)):
+        for _ in range(3):
+            call()
+        if one:
+            assert one in [n for n, _ in c.timings()]
+        for _ in range(2):
+            call()
+            assert "EVALUATE_PI_R" in [n for n, _ in c.timings()]
+    c.close()
