@@ -24,7 +24,8 @@
 namespace cq {
 namespace {
 
-// Gt[m][t] = G[m][t]^T as complex64 for the elements [begin, end) (whole molecules); offsets/edges from the molecule table
+// Gt[m][t] = G[m][t]^T as complex64 for the elements [begin, end) (whole molecules); offsets and
+// edges from the molecule table
 __global__ void k_transpose_grouped(const double2* __restrict__ G, float2* __restrict__ Gt,
                                     const int64_t* __restrict__ off, const int64_t* __restrict__ nb,
                                     int nmol, int64_t begin, int64_t end) {
@@ -158,10 +159,11 @@ cq::TcGroup group(const void* A, bool as, bool ca, int64_t lda, int64_t sA, cons
   return g;
 }
 
-// one GW iteration for all molecules; G in b->G, Sigma (complex128) into b->Sig
-// The host copies run on the second stream in two halves of the molecules: the second half's G
-// crosses while the first half is projected, and the first half's Sigma leaves while the second
-// half is (twelve molecules of 30 to 150 orbitals: 26.6 -> 25.4 ms with 1.85 ms of copies each way).
+// One GW iteration for all molecules: G into b->G, Sigma (complex128) in b->Sig and out.  The host
+// copies run on the second stream in two halves of the molecules (one molecule: no overlap): the
+// second half's G crosses while the first half is projected, and the first half's Sigma leaves while
+// the second half is projected back (twelve molecules of 30 to 150 orbitals: 25.4 ms, 26.6 with the
+// 1.85 ms of copies each way before and after).
 void batch_gw(Batch* b, const double* const* G_list, double* const* Sigma_list) {
   const cudaStream_t s = b->st;
   const int64_t nt = b->nt, nth = b->nth, nwh = b->nwh, cols = b->cols;

@@ -12,10 +12,9 @@
 // The block is a serial chain of 32 pivots, so what counts is the latency of one: a row's 32
 // values stay in registers of NTH / 32 neighbouring lanes, one barrier per column passes the
 // vector v and the pivot through shared memory, the chain holds one reciprocal, and the square
-// roots and logarithms are taken for all rows at once at the end.  (The earlier form updated
-// shared memory with a square root, a division and a logarithm per column inside the chain and
-// inverted the factor by forward substitution with a division per row: 246 us for 200 problems of N_mu 128, four
-// blocks each, now 127 us; 22.2 ms for 5400 of 384, now 18.0 ms.)
+// roots and logarithms are taken for all rows at once at the end.  200 problems of N_mu 128, four
+// blocks each: 127 us in all (246 with a square root, a division and a logarithm per column inside
+// the chain and the factor inverted afterwards); 5400 of 384: 18.0 ms (22.2).
 //
 // Each element's operations do not depend on NTH, so all kernels give identical results.
 template <typename F, int... C>

@@ -1942,7 +1942,8 @@ int coqui_b200_gw_iteration(coqui_b200_ctx* c, const double* G_tskij, double* Si
     // buffers and replayed by the following ones
     // page-locked host buffers: the copies join the graph
     if (!eps_inv_head && c->mode == COQUI_B200_MIXED && !c->prof.on && !div_active(c) &&
-        (G_tskij ? cq::host_is_pinned(G_tskij) : c->g_resident) && (!Sigma_tskij || cq::host_is_pinned(Sigma_tskij))) {
+        (G_tskij ? cq::host_is_pinned(G_tskij) : c->g_resident) &&
+        (!Sigma_tskij || cq::host_is_pinned(Sigma_tskij))) {
       gw_iteration_graph(c, G_tskij, Sigma_tskij);
       return;
     }

@@ -103,11 +103,11 @@ void launch_zero_upper_and_adjoint(double2* L, double2* LH, int64_t Np, int64_t 
   CQ_CHECK_CUDA(cudaGetLastError());
 }
 
-// The factorisation keeps each 32 x 32 diagonal block of its factor in shared memory only
-// (global memory gets the panel blocks below it and, in the upper triangle, the block's
-// inverse adjoint).  This kernel forms the diagonal blocks again the way the factorisation
-// does: C_jj = chol(A_jj - sum_{kb < j} L_j,kb L_j,kb^H) from I - M = A and the stored panel
-// blocks, and writes them into A's lower triangle.  One CTA per (block j, problem).
+// The factorisation never forms the 32 x 32 diagonal blocks of its factor: the panels need their
+// inverses only (chol_diag.cuh), which go into the upper triangle as adjoints, with the panel blocks
+// below.  This kernel forms the diagonal blocks separately, C_jj = chol(A_jj - sum_{kb < j} L_j,kb
+// L_j,kb^H) from I - M = A and the stored panel blocks (equal to the factor behind them to rounding),
+// and writes them into A's lower triangle.  One CTA per (block j, problem).
 constexpr int kDiagB = 32;
 __global__ void __launch_bounds__(256) k_chol_diag_blocks(const double2* __restrict__ Mall,
                                                           double2* __restrict__ Aall, int64_t n,

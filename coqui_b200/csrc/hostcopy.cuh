@@ -18,8 +18,9 @@ bool host_is_pinned(const void* p);
 void copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 void copy_from_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
-// The page-locked buffers are kept between calls while at least one user (a context, a batch)
-// lives, at most kMaxStageSets sets per process, and freed with the last user.
+// The page-locked buffers are kept between calls while at least one user (a context; the molecule
+// batch and the network copy through the driver) lives, at most kMaxStageSets sets per process, and
+// freed with the last user.
 struct StageUser {
   StageUser();
   ~StageUser();

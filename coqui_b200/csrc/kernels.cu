@@ -112,9 +112,9 @@ __device__ __forceinline__ void dft_line(C (&x)[N], int sign) {
   } else {
     // N = 5, 7: with t_m = x_m + x_{N-m} and d_m = x_m - x_{N-m},
     //   y_k, y_{N-k} = x_0 + sum_m cos(2 pi k m / N) t_m +- sign i sum_m sin(2 pi k m / N) d_m:
-    // real multipliers that are literals of the storage type.  (The plain sum with a table of
-    // double2 converted every twiddle in the loop: Pi and Sigma of a 5 x 3 x 2 grid at N_mu 203
-    // took 0.89 and 1.17 ms, now 0.47 and 1.18.)
+    // real multipliers that are literals of the storage type (a table of double2 in the plain sum
+    // has every twiddle converted in the loop: Pi of a 5 x 3 x 2 grid at N_mu 203 0.89 ms, so 0.47;
+    // Sigma, bound by its registers then, stayed at 1.17).
     static_assert(N == 5 || N == 7, "DFT length");
     using R = decltype(x[0].x);
     constexpr int H = (N - 1) / 2;
@@ -615,11 +615,10 @@ template <typename R, int N0> constexpr int fused_blocks() {
 // memory sweeps per tile (load + innermost DFT, middle DFT, outermost DFT + product + inverse,
 // middle inverse, innermost inverse + store).
 template <typename R, int TILE, int NC, int N0>
-__global__ void __launch_bounds__(256, (fused_blocks<R, N0>())) k_pi_fused(const cplx_t<R>* __restrict__ Gp,
-                                                  const cplx_t<R>* __restrict__ Gn,
-                                                  cplx_t<R>* __restrict__ Pi, int64_t ncol,
-                                                  int rn0, int rn1, int rn2, R scale,
-                                                  TauSlices ts) {
+__global__ void __launch_bounds__(256, (fused_blocks<R, N0>()))
+    k_pi_fused(const cplx_t<R>* __restrict__ Gp, const cplx_t<R>* __restrict__ Gn,
+               cplx_t<R>* __restrict__ Pi, int64_t ncol, int rn0, int rn1, int rn2, R scale,
+               TauSlices ts) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n0 = NC ? NC : rn0, n1 = NC ? NC : rn1, n2 = NC ? NC : rn2;
@@ -658,11 +657,10 @@ __global__ void __launch_bounds__(256, (fused_blocks<R, N0>())) k_pi_fused(const
 // Sigma(t) columns (both halves): S = f_kR[ -(f_Rk G) o W_R ] (scale = -1/nk), W_R read from
 // global memory inside the outermost-dimension sweep.  In place (S may alias G).
 template <typename R, int TILE, int NC, int N0>
-__global__ void __launch_bounds__(256, (fused_blocks<R, N0>())) k_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm,
-                                                     const cplx_t<R>* __restrict__ WR,
-                                                     cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol,
-                                                     int rn0, int rn1, int rn2, R scale,
-                                                     TauSlices ts) {
+__global__ void __launch_bounds__(256, (fused_blocks<R, N0>()))
+    k_sigma_fused(const cplx_t<R>* Gp, const cplx_t<R>* Gm, const cplx_t<R>* __restrict__ WR,
+                  cplx_t<R>* Sp, cplx_t<R>* Sm, int64_t ncol, int rn0, int rn1, int rn2, R scale,
+                  TauSlices ts) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n0 = NC ? NC : rn0, n1 = NC ? NC : rn1, n2 = NC ? NC : rn2;

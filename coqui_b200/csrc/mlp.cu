@@ -609,12 +609,10 @@ void mlp_forward(Mlp& n, const float* x, int64_t B, float* y, cudaStream_t s) {
                                            W + n.ob3(), nullptr, n.part, s);
 }
 
-// Forward and backward of a 65536-sample batch of the 4 -> 256 -> 256 -> 2 network took 42.0 ms
-// (40.7 ms of it in the three weight gradients, whose few output tiles each walked the whole
-// batch in one block); with their K cut into slices, packed 8 x 8 register tiles, the output
-// layer in one kernel and the input layer's gradients in another it takes 0.99 ms, 0.87 ms on the
-// device (the three 65536 x 256 x 256 products at 36-42 TFLOP/s FP32), and the shorter sums bring
-// the gradient from 2.3e-6 to 6e-8 of its FP64 value.
+// Forward and backward of a 65536-sample batch of the 4 -> 256 -> 256 -> 2 network: 0.99 ms, 0.87 ms
+// on the device, bound by the FP32 pipe in the three 65536 x 256 x 256 products (36-42 TFLOP/s).
+// The weight gradients have few output tiles and are cut along the batch: uncut they take 40.7 ms,
+// and their long sums leave the gradient 2.3e-6 from FP64 where the sliced ones leave 6e-8.
 float mlp_backward(Mlp& n, const float* x, const float* t, int64_t B, cudaStream_t s) {
   ensure_batch(n, B);
   const int64_t H = n.width, D = n.dout, nout = B * D;
@@ -622,8 +620,8 @@ float mlp_backward(Mlp& n, const float* x, const float* t, int64_t B, cudaStream
   const __nv_bfloat16* W = n.wb.p;
   std::vector<float> part;
   // one workspace for every split reduction below (growing it step by step would free and
-  // allocate between the kernels of a first call): the widest weight gradient's slices, the
-  // output layer's and the input layer's block sums
+  // allocate between the kernels of a first call): the slices of the weight gradients, the block
+  // sums of the output layer, the input layer and the biases
   auto slices = [&](int64_t M, int64_t N) { return gemm_slices(M, N, B) * M * N; };
   n.part.ensure(std::max({slices(H, H),
                           n.din <= 8 ? in_blocks(B) * (H * n.din + H) : slices(H, n.din),

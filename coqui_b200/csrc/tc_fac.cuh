@@ -27,9 +27,11 @@
 // throughout 1.8e-5 / 3e-3 / 7e-2.
 //
 // Per 32 complex K: 96 KB stored and 144 KB read against 1536 cycles of MMA, and half the
-// conversion work.  Measured (1600 problems of N_mu 512 / 675 of 1024): the M products
-// 6.87 -> 4.24 ms / 17.1 -> 9.9 ms, T and W 8.7 -> 4.3 / 18.6 -> 9.9; W of random Hermitian Pi is
-// 3.8e-6 / 5.7e-6 (N_mu 512 / 768) from FP64 in the 2-norm where split TF32 gave 7.0e-6 / 1.05e-5.
+// conversion work.  Measured (1600 problems of N_mu 512 / 675 of 1024; split TF32 -> this form): the
+// M products with their row-maximum pass 6.87 -> 4.9 ms / 17.1 -> 11.3, the W group (T and W, and
+// with them the D^H D product, E and its row maxima, which are as they were) 11.4 -> 9.8 /
+// 25.2 -> 20.7; W of random Hermitian Pi is 3.8e-6 / 5.7e-6 (N_mu 512 / 768) from FP64 in the 2-norm
+// where split TF32 gave 7.0e-6 / 1.05e-5.
 //
 // CTA: 128 rows x 128 complex columns (UMMA M = 128, N = 256 with the realified rows of
 // tc_gemm.cu), K blocks of 32 complex = one 128-byte row, two stages of 96 KB.  Warps 0-7 stage B

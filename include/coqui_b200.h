@@ -309,7 +309,8 @@ COQUI_B200_API int coqui_b200_batch_set_ir(coqui_b200_batch* batch, const double
 COQUI_B200_API int coqui_b200_batch_set_thc(coqui_b200_batch* batch, int64_t m, const double* X_Pa,
                                             const double* V_PQ);
 /* One GW iteration (update_w + evaluate) of every molecule: G_list[m] (nt_f, nb_m, nb_m) in,
-   Sigma_list[m] (nt_f, nb_m, nb_m) out (the list or entries may be NULL). */
+   Sigma_list[m] (nt_f, nb_m, nb_m) out (the list or entries may be NULL; written only when every
+   molecule's factorisations succeeded). */
 COQUI_B200_API int coqui_b200_batch_gw_iteration(coqui_b200_batch* batch,
                                                  const double* const* G_list,
                                                  double* const* Sigma_list);
