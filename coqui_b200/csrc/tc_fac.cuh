@@ -452,10 +452,11 @@ __global__ void __launch_bounds__(256) k_fac_colmax(const double2* __restrict__ 
     cm[q * K + k] = __float_as_uint(m);
   }
 }
-// Columns, and rows, of a matrix may differ by this power of two and keep one scale: the words'
-// 2^-40 of the largest element is still 2^-30 of the largest of any column and row, and FP32 rounds
-// a sum of such terms at 2^-24.
-constexpr int kFacGrade = 10;
+// Columns, and rows, of a matrix may differ by this power of two and keep one scale.  The words are
+// off by 2^-40 of the largest element; in a row that is 2^-8 of it the terms of a sum with a graded
+// Bt weigh 2^-8, and a column 2^-8 of the largest meets a Bt of 2^8: 2^(-40 + 8 + 8) of the sum,
+// where FP32 rounds it.
+constexpr int kFacGrade = 8;
 constexpr int kFacExp = 20;  // a scale common to all rows lies within 2^+-20
 __device__ __forceinline__ int fac_max_exp(uint32_t bits) { return min((int)(bits >> 23) - 127, 127); }
 // smallest and largest exponent of the n nonzero maxima of a matrix (block-wide; hi < lo: none)

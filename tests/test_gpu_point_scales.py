@@ -42,14 +42,14 @@ def dense_g(s):
 
 
 @pytest.mark.parametrize("Np", [129, 200, 290])
-@pytest.mark.parametrize("decades", [2, 3, 5, 8])  # 10^3: just below the level that is graded
+@pytest.mark.parametrize("decades", [2, 2.4, 3, 5, 8])  # 10^2.4: the largest that counts as ungraded
 def test_w_of_graded_v_and_pi(Np, decades):
     """V = D V0 D with Pi = D^-1 Pi0 D^-1: D^-1 W D^-1 does not depend on D."""
     s = make_system((2, 1, 1), 3, 1, Np, seed=Np)
     rng = np.random.default_rng(Np)
     B = rng.standard_normal((FT.nw_half, s.nk, Np, Np)) + 1j * rng.standard_normal((FT.nw_half, s.nk, Np, Np))
     Pi = -(B @ np.conj(np.swapaxes(B, -1, -2))) * (0.5 / Np)
-    d = 1.0 / scales(Np, decades, Np + decades)
+    d = 1.0 / scales(Np, decades, Np + int(decades))
     dd = d[:, None] * d[None, :]
     c = context(s, capi.FP64)
     ref = c.dyson_w(Pi)
